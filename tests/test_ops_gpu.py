@@ -46,6 +46,42 @@ def test_layernorm_fwd_bwd():
     close(y1, y0); close(dx1, dx0); close(dw1, dw0); close(db1, db0)
 
 
+@pytest.mark.parametrize("layernorm", [False, True])
+@pytest.mark.parametrize("T,H", [(1, 8), (9, 264), (4801, 512), (2500, 1024), (13, 1032), (700, 2048), (5, 2056), (301, 4104), (40, 8192)])
+def test_norm_edges(T, H, layernorm):
+    """Rows by warps and by blocks at the edges of their ranges, more rows than one pass of the grid takes; with and without what is
+    added.  Sums of T values against a pairwise sum: relative error well below 1e-5 sqrt(T); outputs one bf16 rounding (2^-8)."""
+    x, r, dy = (torch.randn(T, H, dtype=BF).cuda() for _ in range(3))
+    w, b = ((1 + 0.1 * torch.randn(H)).to(BF).cuda() for _ in range(2))
+    for res in (None, r):
+        if layernorm:
+            y, h, rstd, mean = F.layernorm_fwd(x, w, b, 1e-5, res)
+        else:
+            (y, h, rstd), mean = F.rmsnorm_fwd(x, w, 1e-5, res), None
+        hd = (x.double() + (0 if res is None else r.double())).to(BF).double()
+        m = hd.mean(1, keepdim=True) if layernorm else torch.zeros_like(hd[:, :1])
+        s = torch.rsqrt((hd - m).square().mean(1, keepdim=True) + 1e-5)
+        xh = (hd - m) * s
+        assert torch.equal(h.double(), hd)
+        assert ((y.double() - (xh * w.double() + (b.double() if layernorm else 0))).abs() <= 2 ** -8 * (xh * w.double()).abs() + (2 ** -7 if layernorm else 1e-5)).all()
+        dw, db = torch.zeros(H, device="cuda"), torch.zeros(H, device="cuda")
+        dx = F.layernorm_bwd(dy, h, w, rstd, mean, dw, db, res) if layernorm else F.rmsnorm_bwd(dy, h, w, rstd, dw, res)
+        g = dy.double() * w.double()
+        want = s * (g - xh * (g * xh).mean(1, keepdim=True) - (g.mean(1, keepdim=True) if layernorm else 0)) + (0 if res is None else r.double())
+        assert ((dx.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-4 * (1 + s)).all()
+        assert ((dw.double() - (dy.double() * xh).sum(0)).abs() <= 1e-5 * (dy.double() * xh).abs().sum(0) + 1e-6).all()
+        if layernorm:
+            assert ((db.double() - dy.double().sum(0)).abs() <= 1e-5 * dy.double().abs().sum(0) + 1e-6).all()
+
+
+@pytest.mark.parametrize("T,N", [(1, 8), (31, 264), (33, 768), (4662, 3072), (130, 50304)])
+def test_col_sum(T, N):
+    x = torch.randn(T, N + 8, dtype=BF).cuda()[:, :N]
+    out = torch.ones(N, device="cuda")
+    F.col_sum_(x, out)
+    assert ((out.double() - 1 - x.double().sum(0)).abs() <= 1e-5 * (1 + x.double().abs().sum(0))).all()
+
+
 def test_rope_roundtrip_and_ref():
     T, S, nh, D = 256, 128, 10, 64
     ld = 12 * D

@@ -1,9 +1,11 @@
 // RMSNorm / LayerNorm forward and backward, fused with the residual add.
 //
-// One warp per row, 128-bit loads, the row held in registers between the statistics pass and
-// the scale pass (one read of the activations per kernel).  The backward accumulates the weight
-// gradient in registers over all rows a warp visits and flushes it once with fp32 atomics into
-// the fp32 gradient buffer.
+// All of these are bound by HBM: every activation is read once and written once, 128 bits at a time, and the row stays in
+// registers between the statistics pass and the scale pass.  Rows of up to 1024 entries belong to a warp each (no barrier, and
+// the loads of the warp's next row are in flight while it finishes this one), wider rows to a block of 256 threads: a warp that
+// holds 4096 entries needs 166 registers a lane, which leaves 12 % of the warps resident and the loads unhidden (5000 x 4096
+// forward: 58 us by warps, 18 us by blocks, 13 us of HBM time).  The backward accumulates the weight gradient in registers
+// over all rows that a thread visits and flushes it once with fp32 atomics into the fp32 gradient buffer.
 //
 // Replaces the reference's one-thread-per-row kernels (src/backend/gpu_compute_cuda.cpp:219
 // rmsnorm_kernel, :617 layernorm_kernel) and its CPU fused residual+norm
@@ -38,7 +40,18 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(p) = u;
 }
 
+__device__ __forceinline__ void cvt8(const uint4& u, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = unpack_bf16(w[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+
 // y = norm(x + res) * w (+ b);  h_out = x + res (optional);  stats: rstd (and mean for LayerNorm).
+// One warp per row (H <= 256 NCHUNK).
 template <int NCHUNK, bool LAYERNORM>
 __global__ void __launch_bounds__(256) norm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                        const __nv_bfloat16* __restrict__ res,
@@ -112,21 +125,14 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const __nv_bfloat16* __re
   }
 }
 
-// dx = rstd * (g - xhat * mean(g * xhat) [- mean(g)])  with g = dy * w, xhat = (h - mean) * rstd,
-// plus the incoming residual-stream gradient `dres`.  With FUSE_DW the warp also accumulates
-// dw += sum_rows dy * xhat (db += sum_rows dy) in registers and flushes once per block; for wide
-// rows the weight gradient is a separate column reduction (norm_dw_kernel) to bound registers.
-__device__ __forceinline__ void cvt8(const uint4& u, float (&f)[8]) {
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = unpack_bf16(w[i]);
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
-}
-
-template <int NCHUNK, bool LAYERNORM, bool FUSE_DW>
+// dx = rstd * (g - xhat * mean(g * xhat) [- mean(g)])  with g = dy * w, xhat = (h - mean) * rstd, plus the incoming
+// residual-stream gradient `dres`;  dw += sum_rows dy * xhat (db += sum_rows dy).
+// WIDE = false: a warp per row, eight rows at a time in a block (H <= 256 NCHUNK).  WIDE = true: the block's 256 threads share a row
+// (H <= 2048 NCHUNK); the row's two sums meet in shared memory, in one of two slots so that a row costs one barrier.
+// The loads of the next row are issued before the sums of this one are reduced.  The weight gradient of the block's rows
+// meets in shared memory (plain stores, one slice per warp: fp32 atomics on shared memory are a compare-and-swap loop, and
+// with them layer norm of 4662 x 768 took 33 us, 13 us without) and leaves with one atomic per column.
+template <int NCHUNK, bool LAYERNORM, bool WIDE>
 __global__ void __launch_bounds__(256) norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                        const __nv_bfloat16* __restrict__ h,
                                                        const __nv_bfloat16* __restrict__ w,
@@ -136,55 +142,98 @@ __global__ void __launch_bounds__(256) norm_bwd_kernel(const __nv_bfloat16* __re
                                                        __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
                                                        float* __restrict__ db, int rows, int H) {
   tfb::pdl_sync();
-  const int lane = threadIdx.x & 31;
-  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  constexpr int NACC = FUSE_DW ? NCHUNK : 1;
-  float dw_acc[NACC][8], db_acc[NACC][8];
+  extern __shared__ float red[];                      // gradient slices: [8][H], WIDE: [H]
+  __shared__ float sums[2][2][8];
+  constexpr int TPR = WIDE ? 256 : 32;                // threads per row
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t = WIDE ? int(threadIdx.x) : lane;       // place in the row
+  const int first = WIDE ? int(blockIdx.x) : int(blockIdx.x) * 8 + warp;
+  const int step = WIDE ? int(gridDim.x) : int(gridDim.x) * 8;
+  float dw_acc[NCHUNK][8], db_acc[LAYERNORM ? NCHUNK : 1][8];
 #pragma unroll
-  for (int c = 0; c < NACC; ++c)
+  for (int c = 0; c < NCHUNK; ++c)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) dw_acc[c][i] = 0.f, db_acc[c][i] = 0.f;
-
-  for (int row = warp_global; row < rows; row += nwarps) {
+    for (int i = 0; i < 8; ++i) {
+      dw_acc[c][i] = 0.f;
+      if (LAYERNORM) db_acc[c][i] = 0.f;
+    }
+  uint4 wr[NCHUNK];
+#pragma unroll
+  for (int c = 0; c < NCHUNK; ++c) {
+    const int col = (c * TPR + t) * 8;
+    if (col < H) wr[c] = *reinterpret_cast<const uint4*>(w + col);
+  }
+  uint4 dyn[NCHUNK], hn[NCHUNK], rn[NCHUNK];
+  float rstd_n = 0.f, mean_n = 0.f;
+  auto fetch = [&](int row) {
     const long long off = (long long)row * H;
-    const float rstd = rstd_in[row];
-    const float mean = LAYERNORM ? mean_in[row] : 0.f;
-    uint4 dyr[NCHUNK], hr[NCHUNK];
+    rstd_n = rstd_in[row];
+    if (LAYERNORM) mean_n = mean_in[row];
+#pragma unroll
+    for (int c = 0; c < NCHUNK; ++c) {
+      const int col = (c * TPR + t) * 8;
+      if (col < H) {
+        dyn[c] = *reinterpret_cast<const uint4*>(dy + off + col);
+        hn[c] = *reinterpret_cast<const uint4*>(h + off + col);
+        if (dres) rn[c] = *reinterpret_cast<const uint4*>(dres + off + col);
+      }
+    }
+  };
+  if (first < rows) fetch(first);
+  int slot = 0;
+  for (int row = first; row < rows; row += step, slot ^= 1) {
+    const long long off = (long long)row * H;
+    const float rstd = rstd_n, mean = mean_n;
+    uint4 dyr[NCHUNK], hr[NCHUNK], rr[NCHUNK];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int c = 0; c < NCHUNK; ++c) {
-      const int col = (c * 32 + lane) * 8;
+      const int col = (c * TPR + t) * 8;
       if (col < H) {
-        dyr[c] = *reinterpret_cast<const uint4*>(dy + off + col);
-        hr[c] = *reinterpret_cast<const uint4*>(h + off + col);
+        dyr[c] = dyn[c];
+        hr[c] = hn[c];
+        rr[c] = rn[c];
         float d[8], xh[8], wv[8];
         cvt8(dyr[c], d);
         cvt8(hr[c], xh);
-        load8(w + col, wv);
+        cvt8(wr[c], wv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           xh[i] = (xh[i] - mean) * rstd;
-          if (FUSE_DW) {
-            dw_acc[c % NACC][i] += d[i] * xh[i];
-            if (LAYERNORM) db_acc[c % NACC][i] += d[i];
-          }
+          dw_acc[c][i] += d[i] * xh[i];
+          if (LAYERNORM) db_acc[c][i] += d[i];
           const float g = d[i] * wv[i];
           s1 += g * xh[i];
           s2 += g;
         }
       }
     }
-    s1 = warp_sum(s1) / H;
-    s2 = LAYERNORM ? warp_sum(s2) / H : 0.f;
+    if (row + step < rows) fetch(row + step);
+    s1 = warp_sum(s1);
+    if (LAYERNORM) s2 = warp_sum(s2);
+    if (WIDE) {
+      if (lane == 0) {
+        sums[slot][0][warp] = s1;
+        sums[slot][1][warp] = s2;
+      }
+      __syncthreads();
+      s1 = s2 = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        s1 += sums[slot][0][i];
+        s2 += sums[slot][1][i];
+      }
+    }
+    s1 /= H;
+    s2 = LAYERNORM ? s2 / H : 0.f;
 #pragma unroll
     for (int c = 0; c < NCHUNK; ++c) {
-      const int col = (c * 32 + lane) * 8;
+      const int col = (c * TPR + t) * 8;
       if (col < H) {
         float d[8], xh[8], wv[8], o[8];
         cvt8(dyr[c], d);
         cvt8(hr[c], xh);
-        load8(w + col, wv);
+        cvt8(wr[c], wv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float xn = (xh[i] - mean) * rstd;
@@ -192,7 +241,7 @@ __global__ void __launch_bounds__(256) norm_bwd_kernel(const __nv_bfloat16* __re
         }
         if (dres) {
           float r[8];
-          load8(dres + off + col, r);
+          cvt8(rr[c], r);
 #pragma unroll
           for (int i = 0; i < 8; ++i) o[i] += r[i];
         }
@@ -200,70 +249,69 @@ __global__ void __launch_bounds__(256) norm_bwd_kernel(const __nv_bfloat16* __re
       }
     }
   }
-  if (FUSE_DW) {
-    // block-level reduction of the weight gradient through shared memory, then one atomic per column
-    extern __shared__ float red[];  // [H]
-    for (int pass = 0; pass < (LAYERNORM && db ? 2 : 1); ++pass) {
-      for (int i = threadIdx.x; i < H; i += blockDim.x) red[i] = 0.f;
-      __syncthreads();
+  for (int pass = 0; pass < (LAYERNORM && db ? 2 : 1); ++pass) {
+    float* dst = pass == 0 ? dw : db;
 #pragma unroll
-      for (int c = 0; c < NACC; ++c) {
-        const int col = (c * 32 + lane) * 8;
-        if (col < H) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) atomicAdd(&red[col + i], pass == 0 ? dw_acc[c][i] : db_acc[c][i]);
-        }
+    for (int c = 0; c < NCHUNK; ++c) {
+      const int col = (c * TPR + t) * 8;
+      if (col < H) {
+        const float(&a)[8] = pass == 0 ? dw_acc[c] : db_acc[LAYERNORM ? c : 0];
+        float4* r = reinterpret_cast<float4*>(red + (WIDE ? 0 : warp * H) + col);
+        r[0] = make_float4(a[0], a[1], a[2], a[3]);
+        r[1] = make_float4(a[4], a[5], a[6], a[7]);
       }
-      __syncthreads();
-      float* dst = pass == 0 ? dw : db;
-      for (int i = threadIdx.x; i < H; i += blockDim.x) atomicAdd(dst + i, red[i]);
-      __syncthreads();
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < H; i += 256) {
+      float v = red[i];                               // WIDE: every column has one thread in the block
+      if (!WIDE) {
+#pragma unroll
+        for (int k = 1; k < 8; ++k) v += red[k * H + i];
+      }
+      atomicAdd(dst + i, v);
+    }
+    __syncthreads();
   }
 }
 
-// Column reduction for wide rows: block (x) owns 256 columns, blocks along y split the rows.
-template <bool LAYERNORM>
-__global__ void __launch_bounds__(256) norm_dw_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                      const __nv_bfloat16* __restrict__ h,
-                                                      const float* __restrict__ rstd_in,
-                                                      const float* __restrict__ mean_in, float* __restrict__ dw,
-                                                      float* __restrict__ db, int rows, int H) {
+// out[n] += sum over rows of x[m, n]: the gradient of a bias.  Bound by reading x once: a warp covers 256 columns of a row with
+// 16-byte loads, four rows in flight, the block's eight warps and the blocks along y share the rows.
+__global__ void __launch_bounds__(256) col_sum_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, float* __restrict__ out, int rows, int N) {
   tfb::pdl_sync();
+  __shared__ float red[8][256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = (blockIdx.x * 32 + lane) * 8;
-  float aw[8] = {0, 0, 0, 0, 0, 0, 0, 0}, ab[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (col < H) {
-    for (int row = blockIdx.y * 8 + warp; row < rows; row += gridDim.y * 8) {
-      float d[8], xh[8];
-      load8(dy + (long long)row * H + col, d);
-      load8(h + (long long)row * H + col, xh);
-      const float rstd = rstd_in[row], mean = LAYERNORM ? mean_in[row] : 0.f;
+  const int step = gridDim.y * 8;
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (col < N) {
+    for (int row = blockIdx.y * 8 + warp; row < rows; row += 4 * step) {
+      uint4 v[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        aw[i] += d[i] * (xh[i] - mean) * rstd;
-        if (LAYERNORM) ab[i] += d[i];
+      for (int u = 0; u < 4; ++u)
+        if (row + u * step < rows) v[u] = *reinterpret_cast<const uint4*>(x + (long long)(row + u * step) * ldx + col);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (row + u * step >= rows) break;
+        float f[8];
+        cvt8(v[u], f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] += f[i];
       }
     }
   }
-  __shared__ float red[2][256];
-  for (int i = threadIdx.x; i < 512; i += 256) (&red[0][0])[i] = 0.f;
-  __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    atomicAdd(&red[0][lane * 8 + i], aw[i]);
-    if (LAYERNORM) atomicAdd(&red[1][lane * 8 + i], ab[i]);
-  }
+  for (int i = 0; i < 8; ++i) red[warp][lane * 8 + i] = acc[i];
   __syncthreads();
   const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c < H) {
-    atomicAdd(dw + c, red[0][threadIdx.x]);
-    if (LAYERNORM && db) atomicAdd(db + c, red[1][threadIdx.x]);
+  if (c < N) {
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v += red[k][threadIdx.x];
+    atomicAdd(out + c, v);
   }
 }
 
-// Few rows (decode batches): one CTA per row, so that a 4096-wide row is two 16-byte loads per thread instead of sixteen
-// dependent round trips in one warp; the warp-per-row kernel above relies on many resident rows to hide that latency.
+// Wide rows (more than 1024 entries): one CTA per row, so that a 4096-wide row is two 16-byte loads per thread.
 template <int NCH, bool LAYERNORM>
 __global__ void __launch_bounds__(256) norm_fwd_rowblock_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                                                                 const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
@@ -358,24 +406,19 @@ template <bool LN>
 static int launch_fwd(const void* x, const void* res, const void* w, const void* b, void* y, void* h_out, float* rstd,
                       float* mean, int rows, int H, float eps, cudaStream_t st) {
   if (H % 8 || H > 8192) return TFB_ERR_ARG;
-  const int blocks = min((rows + 7) / 8, sm_count() * 8);
   auto X = static_cast<const __nv_bfloat16*>(x);
   auto R = static_cast<const __nv_bfloat16*>(res);
   auto W = static_cast<const __nv_bfloat16*>(w);
   auto B = static_cast<const __nv_bfloat16*>(b);
   auto Y = static_cast<__nv_bfloat16*>(y);
   auto Ho = static_cast<__nv_bfloat16*>(h_out);
-  if (H >= 2048 && rows <= 4 * sm_count()) {
-    if (H <= 4096) tfb::launch_k(norm_fwd_rowblock_kernel<2, LN>, rows, 256, 0, st, X, R, W, B, Y, Ho, rstd, mean, rows, H, eps);
-    else tfb::launch_k(norm_fwd_rowblock_kernel<4, LN>, rows, 256, 0, st, X, R, W, B, Y, Ho, rstd, mean, rows, H, eps);
-    return int(cudaGetLastError());
-  }
-#define TFB_GO(NC) tfb::launch_k(norm_fwd_kernel<NC, LN>, blocks, 256, 0, st, X, R, W, B, Y, Ho, rstd, mean, rows, H, eps)
-  if (H <= 512) TFB_GO(2);
-  else if (H <= 1024) TFB_GO(4);
-  else if (H <= 2048) TFB_GO(8);
-  else if (H <= 4096) TFB_GO(16);
-  else TFB_GO(32);
+#define TFB_GO(KERN, blocks) tfb::launch_k(KERN, blocks, 256, 0, st, X, R, W, B, Y, Ho, rstd, mean, rows, H, eps)
+  const int warps8 = (rows + 7) / 8;
+  if (H <= 512) TFB_GO((norm_fwd_kernel<2, LN>), warps8);
+  else if (H <= 1024) TFB_GO((norm_fwd_kernel<4, LN>), warps8);
+  else if (H <= 2048) TFB_GO((norm_fwd_rowblock_kernel<1, LN>), rows);
+  else if (H <= 4096) TFB_GO((norm_fwd_rowblock_kernel<2, LN>), rows);
+  else TFB_GO((norm_fwd_rowblock_kernel<4, LN>), rows);
 #undef TFB_GO
   return int(cudaGetLastError());
 }
@@ -389,21 +432,16 @@ static int launch_bwd(const void* dy, const void* h, const void* w, const float*
   auto W = static_cast<const __nv_bfloat16*>(w);
   auto DR = static_cast<const __nv_bfloat16*>(dres);
   auto DX = static_cast<__nv_bfloat16*>(dx);
-  const size_t sm = size_t(H) * 4;
-  if (H <= 1024) {
-    // 64 registers per thread: four resident blocks per SM; fewer leaves the loads of a row unhidden (94 -> 70 us at
-    // 65536 x 512), more only adds atomics on dw
-    const int blocks = min((rows + 7) / 8, sm_count() * 4);
-    if (H <= 512) tfb::launch_k(norm_bwd_kernel<2, LN, true>, blocks, 256, sm, st, DY, Hh, W, rstd, mean, DR, DX, dw, db, rows, H);
-    else tfb::launch_k(norm_bwd_kernel<4, LN, true>, blocks, 256, sm, st, DY, Hh, W, rstd, mean, DR, DX, dw, db, rows, H);
-  } else {
-    const int blocks = min((rows + 7) / 8, sm_count() * 8);
-    if (H <= 2048) tfb::launch_k(norm_bwd_kernel<8, LN, false>, blocks, 256, 0, st, DY, Hh, W, rstd, mean, DR, DX, dw, db, rows, H);
-    else if (H <= 4096) tfb::launch_k(norm_bwd_kernel<16, LN, false>, blocks, 256, 0, st, DY, Hh, W, rstd, mean, DR, DX, dw, db, rows, H);
-    else tfb::launch_k(norm_bwd_kernel<32, LN, false>, blocks, 256, 0, st, DY, Hh, W, rstd, mean, DR, DX, dw, db, rows, H);
-    dim3 g((H + 255) / 256, min(64, (rows + 7) / 8));
-    tfb::launch_k(norm_dw_kernel<LN>, g, 256, 0, st, DY, Hh, rstd, mean, dw, db, rows, H);
-  }
+#define TFB_GO(NC, WIDE, blocks) \
+  tfb::launch_k(norm_bwd_kernel<NC, LN, WIDE>, blocks, 256, size_t(H) * (WIDE ? 4 : 32), st, DY, Hh, W, rstd, mean, DR, DX, dw, db, rows, H)
+  // blocks that stay for many rows: each adds one atomic per column of dw at its end
+  const int warps8 = min((rows + 7) / 8, sm_count() * 4);
+  if (H <= 512) TFB_GO(2, false, warps8);
+  else if (H <= 1024) TFB_GO(4, false, warps8);
+  else if (H <= 2048) TFB_GO(1, true, min(rows, sm_count() * 4));
+  else if (H <= 4096) TFB_GO(2, true, min(rows, sm_count() * 2));
+  else TFB_GO(4, true, min(rows, sm_count()));
+#undef TFB_GO
   return int(cudaGetLastError());
 }
 
@@ -428,4 +466,13 @@ TFB_API int tfb_layernorm_fwd(const void* x, const void* res, const void* w, con
 TFB_API int tfb_layernorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const float* mean,
                               const void* dres, void* dx, float* dw, float* db, int rows, int H, void* stream) {
   return tfb::launch_bwd<true>(dy, h, w, rstd, mean, dres, dx, dw, db, rows, H, static_cast<cudaStream_t>(stream));
+}
+// out [N] fp32 += column sums of x [rows, N] bf16 (row pitch ldx); N and ldx multiples of 8, x aligned to 16 bytes.
+TFB_API int tfb_col_sum(const void* x, long long ldx, float* out, int rows, int N, void* stream) {
+  using namespace tfb;
+  if (rows <= 0 || N <= 0 || N % 8 || ldx % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) return TFB_ERR_ARG;
+  const int gx = (N + 255) / 256;
+  const dim3 g(gx, max(1, min((rows + 31) / 32, sm_count() * 4 / gx)));
+  tfb::launch_k(col_sum_kernel, g, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x), ldx, out, rows, N);
+  return int(cudaGetLastError());
 }

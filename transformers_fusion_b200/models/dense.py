@@ -139,7 +139,7 @@ def _norm_bwd(cfg, dy, h, w, b, stats, dres):
 
 def _bias_grad(bias, dy):
     if bias is not None:
-        bias.main_grad.add_(dy.float().sum(0))
+        F.col_sum_(dy, bias.main_grad)
 
 
 class BlockCtx:

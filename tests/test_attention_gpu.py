@@ -47,6 +47,30 @@ def test_attn_fwd_longer_keys(B, S, Skv, Hq, Hkv, D, causal):
     assert (lse - rlse).abs().max().item() < 2e-2
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("lens,causal", [([1], True), ([128, 256], True), ([5, 1, 700, 127, 129, 255, 257, 33], True), ([300, 1, 512, 513], False),
+                                         ([1500, 40], True)])
+def test_attn_fwd_packed(lens, causal, D):
+    """Sequences one after the other, each against itself; a sequence whose keys and values are infinite or NaN leaves no trace in
+    the ones before and behind it."""
+    Hq, Hkv = 4, 2
+    kc, vc = Hq * D, (Hq + Hkv) * D
+    pack = F.PackedRows(lens, "cuda")
+    qkv = _qkv(1, pack.rows, Hq, Hkv, D)
+    for poisoned in [None] + list(range(len(lens))):
+        x = qkv.clone()
+        if poisoned is not None:
+            r, n = pack.starts[poisoned], lens[poisoned]
+            x[r:r + n, kc:vc], x[r:r + n, vc:] = float("nan"), float("inf")
+        o = F.attn_fwd_packed(x, x, x, pack, Hq, Hkv, D, causal=causal, k_col0=kc, v_col0=vc)
+        torch.cuda.synchronize()
+        _lib.check_status()
+        for i, (r, n) in enumerate(zip(pack.starts, lens)):
+            if i != poisoned:
+                ro, _, _ = F.attn_ref(qkv[r:r + n], qkv[r:r + n], qkv[r:r + n], 1, n, Hq, Hkv, D, 1 / math.sqrt(D), causal, 0, kc, vc)
+                assert (o[r:r + n].float() - ro).abs().max().item() < 3e-2
+
+
 @pytest.mark.parametrize("B,S,Hq,Hkv,D,causal", [
     (1, 128, 1, 1, 64, True), (2, 256, 4, 2, 64, True), (1, 1024, 8, 8, 64, True), (2, 200, 4, 1, 64, True),
     (1, 300, 2, 1, 64, False), (1, 512, 4, 2, 128, True), (2, 130, 2, 2, 128, False),

@@ -4,7 +4,7 @@ variant repeats the parity check with the kernels."""
 import pytest
 import torch
 
-from transformers_fusion_b200.inference.engine import EngineConfig, InferenceEngine
+from transformers_fusion_b200.inference.engine import EngineConfig, InferenceEngine, Request
 from transformers_fusion_b200.inference.sampler import SamplerConfig
 from transformers_fusion_b200.models.config import TransformerConfig
 from transformers_fusion_b200.models.dense import DenseModel
@@ -236,6 +236,25 @@ def test_batched_prefill_matches_one_by_one():
         outs = eng.generate_batch(prompts, max_tokens=6, sampling=GREEDY)
         res.append((outs, eng.cache.allocator.num_free, eng.stats.prompt_tokens))
     assert res[0] == res[1]
+
+
+def test_feed_prompts_together_match_one_by_one():
+    """Prompts that start in one call of ``feed`` run as packed rows under the token budget: the logits of one call per prompt."""
+    m = _model()
+    g = torch.Generator().manual_seed(4)
+    prompts = [torch.randint(3, 200, (n,), generator=g).tolist() for n in (5, 33, 1, 64, 7, 120)]
+    want = [[4], [0, -1, 7], [], [63], [2, 2], [-120, 119]]
+    cfg = EngineConfig(max_batch=8, num_pages=64, max_prefill_tokens=80, enable_prefix_cache=False)
+    a, b = InferenceEngine(m, None, cfg), InferenceEngine(m, None, cfg)
+    ra, rb = [Request([]) for _ in prompts], [Request([]) for _ in prompts]
+    got = a.feed([(r, p, w) for r, p, w in zip(ra, prompts, want)])
+    for x, r, p, w in zip(got, rb, prompts, want):
+        y = b.feed([(r, p, w)])[0]
+        assert (x is None and y is None and not w) or (x.shape == (len(w), m.cfg.vocab_size) and torch.allclose(x, y, atol=1e-4))
+    x, y = a.feed([(r, [9], [0]) for r in ra]), b.feed([(r, [9], [0]) for r in rb])
+    assert all(torch.allclose(i, j, atol=1e-4) for i, j in zip(x, y))
+    with pytest.raises(IndexError):
+        a.feed([(Request([]), [4, 5], [2]), (Request([]), [4, 5], [0])])
 
 
 def _moe_model(device="cpu", dtype=torch.float32):

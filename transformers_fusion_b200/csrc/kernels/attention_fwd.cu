@@ -36,6 +36,7 @@ struct AttnFwdParams {
   __nv_bfloat16* O;
   long long ldo;
   float* lse;  // [B, Hq, S]
+  const int4* work;  // packed form: (first row, length, pair of query tiles, unused) of every work item, longest first
   int* status;
 };
 
@@ -117,7 +118,10 @@ __device__ __forceinline__ float row_probs(uint32_t tS, float sl2, float mb, int
   return (rs0 + rs1) + (rs2 + rs3);
 }
 
-template <int D>
+// PACKED: sequences of any lengths stand one after the other in the rows (prompts that are run together); a work item names its
+// sequence.  A tile of keys may then reach into the rows of the next sequence: its scores are masked as at the end of a
+// tensor, and its V rows, whose probabilities are zero, are cleared in shared memory (zero times infinity is not zero).
+template <int D, bool PACKED>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                 const __grid_constant__ CUtensorMap tv, const AttnFwdParams p) {
@@ -135,27 +139,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   const uint32_t bar_s_full = bar_kv_empty + ST * 8;
   const uint32_t bar_p_ready = bar_s_full + 16;
   const uint32_t bar_o_full = bar_p_ready + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * ST + 6);
+  const uint32_t bar_tail = bar_o_full + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * ST + 7);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int npair = (p.S + 2 * ATT_BM - 1) / (2 * ATT_BM);
-  const int nkb = (p.Skv + ATT_BN - 1) / ATT_BN;
-  const int bh = p.B * p.Hq;
-  const int pair = npair - 1 - int(blockIdx.x) / bh;  // longest (latest) query blocks are scheduled first
-  const int rem = int(blockIdx.x) % bh;
-  const int b = rem / p.Hq, h = rem % p.Hq;
-  const int hk = h / (p.Hq / p.Hkv);
-  // number of key blocks each tile visits (0: the tile lies past the end of the sequence)
-  int n_t[2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int qb = pair * 2 + t;
-    const int q_last = min(qb * ATT_BM + ATT_BM - 1, p.S - 1);   // last query row of the tile
-    n_t[t] = qb * ATT_BM >= p.S ? 0 : (p.causal ? min((q_last + p.q_off) / ATT_BN + 1, nkb) : nkb);
-  }
-  const int n_kv = max(n_t[0], n_t[1]);
-
   if (threadIdx.x == 0) {
     mbar_init(bar_q, 1);
     for (int s = 0; s < ST; ++s) {
@@ -167,6 +155,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       mbar_init(bar_p_ready + i * 8, 128);
       mbar_init(bar_o_full + i * 8, 1);
     }
+    mbar_init(bar_tail, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tq);
@@ -182,6 +171,34 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   tfb::pdl_sync();   // set-up above touches no global memory; operands written by the previous kernel are read below
+  int S = p.S, Skv = p.Skv, row0 = 0, b, h, pair;
+  if constexpr (PACKED) {
+    const int4 w = p.work[int(blockIdx.x) / p.Hq];
+    row0 = w.x;
+    S = Skv = w.y;
+    pair = w.z;
+    b = 0;
+    h = int(blockIdx.x) % p.Hq;
+  } else {
+    const int npair = (S + 2 * ATT_BM - 1) / (2 * ATT_BM);
+    const int bh = p.B * p.Hq;
+    pair = npair - 1 - int(blockIdx.x) / bh;  // longest (latest) query blocks are scheduled first
+    const int rem = int(blockIdx.x) % bh;
+    b = rem / p.Hq;
+    h = rem % p.Hq;
+  }
+  const int nkb = (Skv + ATT_BN - 1) / ATT_BN;
+  const int hk = h / (p.Hq / p.Hkv);
+  // number of key blocks each tile visits (0: the tile lies past the end of the sequence)
+  int n_t[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int qb = pair * 2 + t;
+    const int q_last = min(qb * ATT_BM + ATT_BM - 1, S - 1);   // last query row of the tile
+    n_t[t] = qb * ATT_BM >= S ? 0 : (p.causal ? min((q_last + p.q_off) / ATT_BN + 1, nkb) : nkb);
+  }
+  const int n_kv = max(n_t[0], n_t[1]);
+  const bool tail = PACKED && n_kv * ATT_BN > Skv;             // the last key tile ends inside the next sequence's rows
   const uint32_t tS0 = tmem_base, tO0 = tmem_base + 256;
 
   if (warp == 0) {
@@ -191,7 +208,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int i = 0; i < NB; ++i)
-          tma_load_3d(sQ + t * L::TILE + i * BOX_BYTES, &tq, bar_q, p.q_col0 + h * D + i * 64, (pair * 2 + t) * ATT_BM, b);
+          tma_load_3d(sQ + t * L::TILE + i * BOX_BYTES, &tq, bar_q, p.q_col0 + h * D + i * 64, row0 + (pair * 2 + t) * ATT_BM, b);
       for (int j = 0; j < n_kv; ++j) {
         const int st = j % ST;
         if (!mbar_wait(bar_kv_empty + st * 8, ((j / ST) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
@@ -200,13 +217,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         const uint32_t sK = sbase + L::KV_OFF + st * 2 * L::TILE, sV = sK + L::TILE;
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
-          tma_load_3d(sK + i * BOX_BYTES, &tk, fb, p.k_col0 + hk * D + i * 64, j * ATT_BN, b);
-          tma_load_3d(sV + i * BOX_BYTES, &tv, fb, p.v_col0 + hk * D + i * 64, j * ATT_BN, b);
+          tma_load_3d(sK + i * BOX_BYTES, &tk, fb, p.k_col0 + hk * D + i * 64, row0 + j * ATT_BN, b);
+          tma_load_3d(sV + i * BOX_BYTES, &tv, fb, p.v_col0 + hk * D + i * 64, row0 + j * ATT_BN, b);
         }
       }
       if (*abort_flag) {  // unwinding: bounded wait for copies already issued
         const uint64_t t0 = globaltimer_ns();
         while (globaltimer_ns() - t0 < 200000ull) {}
+      }
+    }
+    if (PACKED && tail) {
+      __syncwarp();
+      const int j = n_kv - 1, st = j % ST;
+      if (mbar_wait_warp(bar_kv_full + st * 8, (j / ST) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) {
+        const uint32_t sV = sbase + L::KV_OFF + st * 2 * L::TILE + L::TILE;
+        const int live = (Skv - j * ATT_BN) * 128, all = ATT_BN * 128;                 // bytes of a 64-column box
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+          for (int o = live + lane * 16; o < all; o += 512) st_shared_v4(sV + i * BOX_BYTES + o, 0u, 0u, 0u, 0u);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_tail);
       }
     }
   } else if (warp == 1) {
@@ -240,6 +271,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         }
         const int st = j % ST;
         const uint32_t sV = sbase + L::KV_OFF + st * 2 * L::TILE + L::TILE;
+        if (PACKED && tail && j == n_kv - 1) {
+          if (!mbar_wait(bar_tail, 0, abort_flag, p.status, ST_TIMEOUT_FULL)) break;
+          tc_fence_after();
+        }
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (!ok || j >= n_t[t]) continue;
@@ -284,8 +319,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       }
       tc_fence_after();
       const int k0 = j * ATT_BN;
-      const bool need_mask = (p.causal && k0 + ATT_BN - 1 > qb * ATT_BM + p.q_off) || (k0 + ATT_BN > p.Skv);
-      const int k_lim = p.causal ? min(q_idx + p.q_off, p.Skv - 1) : (p.Skv - 1);  // last visible key index for this row
+      const bool need_mask = (p.causal && k0 + ATT_BN - 1 > qb * ATT_BM + p.q_off) || (k0 + ATT_BN > Skv);
+      const int k_lim = p.causal ? min(q_idx + p.q_off, Skv - 1) : (Skv - 1);  // last visible key index for this row
       const float mx = need_mask ? row_max<true>(tS, m, k0, k_lim) : row_max<false>(tS, m, k0, k_lim);
       if (j > 0) {  // O_t(j-1) is complete: the commit behind S_t(j) was issued after it
 #pragma unroll
@@ -319,9 +354,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[c * 32 + i] = fmaf(o[c * 32 + i], alpha_prev, __uint_as_float(v[i]));
         }
-        if (q_idx < p.S) {
+        if (q_idx < S) {
           const float inv = l > 0.f ? 1.f / l : 0.f;
-          __nv_bfloat16* op = p.O + ((long long)b * p.S + q_idx) * p.ldo + h * D;
+          __nv_bfloat16* op = p.O + ((long long)b * S + row0 + q_idx) * p.ldo + h * D;
 #pragma unroll
           for (int c = 0; c < D / 8; ++c) {
             uint4 u;
@@ -331,7 +366,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
             u.w = pack_bf16(o[c * 8 + 6] * inv, o[c * 8 + 7] * inv);
             *reinterpret_cast<uint4*>(op + c * 8) = u;
           }
-          if (p.lse) p.lse[((long long)b * p.Hq + h) * p.S + q_idx] = m * p.scale + logf(l);
+          if (!PACKED && p.lse) p.lse[((long long)b * p.Hq + h) * S + q_idx] = m * p.scale + logf(l);
         }
       }
     }
@@ -345,15 +380,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   }
 }
 
-template <int D>
+template <int D, bool PACKED>
 static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnFwdParams& p,
-                           cudaStream_t st) {
+                           int items, cudaStream_t st) {
   using L = AttnSmem<D>;
   static DeviceOnce once;
-  auto kern = attn_fwd_kernel<D>;
+  auto kern = attn_fwd_kernel<D, PACKED>;
   if (int e = ensure_dyn_smem(once, kern, L::TOTAL)) return e;
-  const int npair = (p.S + 2 * ATT_BM - 1) / (2 * ATT_BM);
-  tfb::launch_k(kern, npair * p.B * p.Hq, ATT_THREADS, L::TOTAL, st, tq, tk, tv, p);
+  tfb::launch_k(kern, items * p.Hq, ATT_THREADS, L::TOTAL, st, tq, tk, tv, p);
   return int(cudaGetLastError());
 }
 
@@ -394,7 +428,34 @@ TFB_API int tfb_attn_fwd_kv(const void* q, long long ldq, int q_col0, const void
   p.Skv = Skv; p.q_off = Skv - S;
   p.scale = scale; p.causal = causal;
   p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
-  p.O = static_cast<__nv_bfloat16*>(o); p.ldo = ldo; p.lse = lse; p.status = status;
+  p.O = static_cast<__nv_bfloat16*>(o); p.ldo = ldo; p.lse = lse; p.work = nullptr; p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return D == 64 ? launch_attn_fwd<64>(tq, tk, tv, p, st) : launch_attn_fwd<128>(tq, tk, tv, p, st);
+  const int items = (S + 2 * ATT_BM - 1) / (2 * ATT_BM) * B;
+  return D == 64 ? launch_attn_fwd<64, false>(tq, tk, tv, p, items, st) : launch_attn_fwd<128, false>(tq, tk, tv, p, items, st);
+}
+
+// Sequences of any lengths packed one after the other: q, k, v, o rows 0 .. rows - 1, every sequence attends to itself.  `work`
+// (device, [items] of four ints): first row, length and pair of 128-query tiles of every work item; a sequence of n rows has
+// ceil(n / 256) of them.  One launch over all prompts of a batch instead of one per prompt: what a short prompt cannot
+// fill (a prompt of 160 tokens has 32 blocks at 32 heads) its neighbours do.
+TFB_API int tfb_attn_fwd_packed(const void* q, long long ldq, int q_col0, const void* k, long long ldk, int k_col0,
+                                const void* v, long long ldv, int v_col0, void* o, long long ldo, const void* work, int items,
+                                long long rows, int Hq, int Hkv, int D, float scale, int causal, int* status, void* stream) {
+  using namespace tfb;
+  if ((D != 64 && D != 128) || Hkv <= 0 || Hq <= 0 || Hq % Hkv || rows <= 0 || rows > 0x7fffff00ll || items <= 0 || !work) return TFB_ERR_ARG;
+  if ((q_col0 | k_col0 | v_col0) & 7 || (ldo & 7) || (reinterpret_cast<uintptr_t>(o) & 15) || (reinterpret_cast<uintptr_t>(work) & 15) ||
+      (long long)items * Hq > 0x7fffffffll)
+    return TFB_ERR_ARG;
+  CUtensorMap tq, tk, tv;
+  int rc;
+  if ((rc = make_tmap_3d(&tq, q, 2, ldq, rows, 1, ldq * 2, ldq * 2 * rows, 64, 128, 1))) return rc;
+  if ((rc = make_tmap_3d(&tk, k, 2, ldk, rows, 1, ldk * 2, ldk * 2 * rows, 64, 128, 1))) return rc;
+  if ((rc = make_tmap_3d(&tv, v, 2, ldv, rows, 1, ldv * 2, ldv * 2 * rows, 64, 128, 1))) return rc;
+  AttnFwdParams p;
+  p.B = 1; p.S = p.Skv = 0; p.q_off = 0; p.Hq = Hq; p.Hkv = Hkv;
+  p.scale = scale; p.causal = causal;
+  p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
+  p.O = static_cast<__nv_bfloat16*>(o); p.ldo = ldo; p.lse = nullptr; p.work = static_cast<const int4*>(work); p.status = status;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return D == 64 ? launch_attn_fwd<64, true>(tq, tk, tv, p, items, st) : launch_attn_fwd<128, true>(tq, tk, tv, p, items, st);
 }

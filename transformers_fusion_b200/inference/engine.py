@@ -226,6 +226,7 @@ class InferenceEngine:
         self.device = model.tok_embeddings.device
         self.max_len = cfg.max_seq_len or mc.max_seq_len
         self.stack = hasattr(model, "run")     # the model brings its own pass over the layers and its own kind of cache
+        self._routed = not self.stack and any(hasattr(w, "router") for w in model.layers)
         if self.stack:
             if cfg.kv_mode != "bf16":
                 raise ValueError(f"{type(model).__name__} keeps keys and values in its own dtype; kv_mode '{cfg.kv_mode}' is not available")
@@ -400,37 +401,39 @@ class InferenceEngine:
         y = self._wq.gemm_wq(x.contiguous(), pw, bias)
         return y if act is None else self.model.activation(y, act)
 
-    def _layers_prefill_batch(self, reqs: List[Request]):
-        """Whole prompts of several sequences in one pass: rows are [B, S_max] with the shorter prompts padded on the right
-        (causal attention keeps padding from reaching real tokens; padded rows carry slot -1 and are not cached).
-        Returns the hidden state of every sequence's last prompt token, [B, H]."""
+    def _layers_prefill_batch(self, reqs: List[Request], all_positions: bool = False):
+        """Whole prompts of several sequences in one pass, their rows one after the other.  Returns the hidden state of every
+        sequence's last prompt token, [B, H], or with ``all_positions`` of every token, [sum of lengths, H].  Layers that route
+        tokens to experts see the prompts padded to one length (what an expert takes depends on how many rows there are);
+        padded rows carry slot -1 and are not cached, and causal attention keeps them from reaching real tokens."""
         if self.stack:
             return self._stack_prefill(reqs, [r.tokens for r in reqs])
         m, mc = self.model, self.model.cfg
         dev = self.device
         Hq, Hkv, D = mc.num_heads, mc.num_kv_heads, mc.head_dim
-        B, S = len(reqs), max(len(r.tokens) for r in reqs)
-        ids = torch.zeros((B, S), dtype=torch.int64)
-        slots = torch.full((B, S), -1, dtype=torch.int64)
-        for b, r in enumerate(reqs):
-            n = len(r.tokens)
-            ids[b, :n] = torch.tensor(r.tokens, dtype=torch.int64)
+        lens = [len(r.tokens) for r in reqs]
+        pack = F.PackedRows([max(lens)] * len(reqs) if self._routed else lens, dev)
+        ids = torch.zeros(pack.rows, dtype=torch.int64)
+        slots = torch.full((pack.rows,), -1, dtype=torch.int64)
+        positions = torch.cat([torch.arange(n) for n in pack.lens])
+        for r, at, n in zip(reqs, pack.starts, lens):
+            ids[at:at + n] = torch.tensor(r.tokens, dtype=torch.int64)
             pg = torch.tensor(r.pages, dtype=torch.int64)
-            pos = torch.arange(n)
-            slots[b, :n] = pg[pos // PAGE] * PAGE + pos % PAGE
-        ids, slots = ids.to(dev).reshape(-1), slots.to(dev).reshape(-1)
+            pos = positions[at:at + n]
+            slots[at:at + n] = pg[pos // PAGE] * PAGE + pos % PAGE
+        ids, slots, positions = torch.stack([ids, slots, positions]).to(dev)
         h = F.embedding_fwd(ids, m.tok_embeddings.data, None, 0)
         if m.pos_embeddings is not None:
-            h = h + m.pos_embeddings.data[:S].repeat(B, 1)
+            h = h + m.pos_embeddings.data[positions]
         rope = m.rope(dev)
-        positions = torch.arange(S, dtype=torch.int32, device=dev).repeat(B)
+        positions = positions.to(torch.int32)
         for li, w in enumerate(m.layers):
             a, _ = _norm_fwd(mc, h, w.attention_norm, getattr(w, "attention_norm_bias", None))
             qkv = self._lin(a, li, "qkv", w.qkv, getattr(w, "qkv_bias", None))
             if rope is not None:
-                F.rope_(qkv, rope[0], rope[1], Hq + Hkv, D, S, positions=positions)
+                F.rope_(qkv, rope[0], rope[1], Hq + Hkv, D, pack.rows, positions=positions)
             self.cache.append(li, qkv, Hq * D, (Hq + Hkv) * D, slots)
-            o, _ = F.attn_fwd(qkv, qkv, qkv, B, S, Hq, Hkv, D, k_col0=Hq * D, v_col0=(Hq + Hkv) * D)
+            o = F.attn_fwd_packed(qkv, qkv, qkv, pack, Hq, Hkv, D, k_col0=Hq * D, v_col0=(Hq + Hkv) * D)
             if mc.use_parallel_residual:
                 attn = self._lin(o, li, "o", w.o, getattr(w, "o_bias", None))
                 f, _ = _norm_fwd(mc, h, w.ffn_norm, getattr(w, "ffn_norm_bias", None))
@@ -441,8 +444,9 @@ class InferenceEngine:
             h = self._ffn(li, w, f, base)
             if mc.use_parallel_residual:
                 h = h + attn
-        last = torch.tensor([b * S + len(r.tokens) - 1 for b, r in enumerate(reqs)], dtype=torch.int64, device=dev)
-        return h[last]
+        if all_positions:
+            return h
+        return h[torch.tensor([at + n - 1 for at, n in zip(pack.starts, lens)], dtype=torch.int64, device=dev)]
 
     def _prefill_fresh(self, fresh: List[Request], finished: list):
         """Groups the newly admitted prompts (sorted by length, so padding stays small) under the padded-token budget and
@@ -689,10 +693,31 @@ class InferenceEngine:
             for i, x in zip(fresh, lg):
                 out[i] = x
         elif fresh:
+            # prompts together up to the budget of a prefill batch (a longer one alone); layers that route see one at a time
+            groups, rows = [], 0
             for i in fresh:
-                r, t, w = entries[i]
-                h = self._layers_prefill(r.tokens, 0, r, all_positions=True)
-                out[i] = self._logits(h[torch.tensor(w, dtype=torch.int64, device=self.device)]) if w else None
+                n = len(entries[i][1])
+                if not groups or self._routed or rows + n > self.cfg.max_prefill_tokens:
+                    groups.append([])
+                    rows = 0
+                groups[-1].append(i)
+                rows += n
+            for grp in groups:
+                if len(grp) > 1:
+                    h = self._layers_prefill_batch([entries[i][0] for i in grp], all_positions=True)
+                else:
+                    h = self._layers_prefill(entries[grp[0]][0].tokens, 0, entries[grp[0]][0], all_positions=True)
+                at, want = 0, []
+                for i in grp:
+                    n = len(entries[i][1])
+                    if any(not -n <= w < n for w in entries[i][2]):
+                        raise IndexError(f"a place outside the {n} tokens of its entry")
+                    want.append([at + w % n for w in entries[i][2]])
+                    at += n
+                if any(want):
+                    lg = self._logits(h[torch.tensor(sum(want, []), dtype=torch.int64, device=self.device)]).split([len(w) for w in want])
+                    for i, w, x in zip(grp, want, lg):
+                        out[i] = x if w else None
         for i in fresh:
             entries[i][0].pos = len(entries[i][1])
         going = [i for i in range(len(entries)) if i not in set(fresh)]

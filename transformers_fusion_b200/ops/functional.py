@@ -459,6 +459,42 @@ def attn_fwd(q, k, v, B, S, Hq, Hkv, D, scale=None, causal=True, q_col0=0, k_col
     return o, lse
 
 
+_lib.register("tfb_attn_fwd_packed", [_lib.c_p, _lib.c_ll, _lib.c_i, _lib.c_p, _lib.c_ll, _lib.c_i, _lib.c_p, _lib.c_ll,
+                                      _lib.c_i, _lib.c_p, _lib.c_ll, _lib.c_p, _lib.c_i, _lib.c_ll, _lib.c_i, _lib.c_i, _lib.c_i,
+                                      _lib.c_f, _lib.c_i, _lib.c_p, _lib.c_p])
+
+
+class PackedRows:
+    """Sequences of the given lengths one after the other in the rows of a buffer, and the attention kernel's list of work items
+    for them (pairs of 128-query tiles, longest first)."""
+
+    def __init__(self, lens, device):
+        assert lens and min(lens) > 0, "sequences of one row or more"
+        self.lens = [int(n) for n in lens]
+        self.starts = [0]
+        for n in self.lens:
+            self.starts.append(self.starts[-1] + n)
+        self.rows = self.starts.pop()
+        items = sorted(((r, n, pair, 0) for r, n in zip(self.starts, self.lens) for pair in range((n + 255) // 256)), key=lambda w: -w[2])
+        self.items = len(items)
+        self.work = torch.tensor(items, dtype=torch.int32).to(device) if torch.device(device).type == "cuda" else None
+
+
+def attn_fwd_packed(q, k, v, pack: PackedRows, Hq, Hkv, D, scale=None, causal=True, q_col0=0, k_col0=0, v_col0=0):
+    """Attention of every packed sequence to itself; q / k / v: [pack.rows, ld] (may be one fused projection output).  Returns
+    o [pack.rows, Hq * D]."""
+    scale = scale if scale is not None else 1.0 / math.sqrt(D)
+    assert q.shape[0] == k.shape[0] == v.shape[0] == pack.rows
+    if not q.is_cuda:
+        return torch.cat([attn_ref(q[r:r + n], k[r:r + n], v[r:r + n], 1, n, Hq, Hkv, D, scale, causal, q_col0, k_col0, v_col0)[0].to(q.dtype)
+                          for r, n in zip(pack.starts, pack.lens)])
+    o = torch.empty((pack.rows, Hq * D), dtype=q.dtype, device=q.device)
+    check(_lib.lib().tfb_attn_fwd_packed(q.data_ptr(), q.stride(0), q_col0, k.data_ptr(), k.stride(0), k_col0, v.data_ptr(), v.stride(0), v_col0,
+                                         o.data_ptr(), o.stride(0), pack.work.data_ptr(), pack.items, pack.rows, Hq, Hkv, D, float(scale),
+                                         int(causal), _lib.status_word(q.device).data_ptr(), stream()), "attn_fwd_packed")
+    return o
+
+
 _lib.register("tfb_attn_bwd", [_lib.c_p, _lib.c_ll, _lib.c_i, _lib.c_p, _lib.c_ll, _lib.c_i, _lib.c_p, _lib.c_ll,
                                _lib.c_i, _lib.c_p, _lib.c_ll, _lib.c_p, _lib.c_ll, _lib.c_p, _lib.c_p,
                                _lib.c_p, _lib.c_ll, _lib.c_i, _lib.c_p, _lib.c_ll, _lib.c_i, _lib.c_p, _lib.c_ll,

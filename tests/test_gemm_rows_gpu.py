@@ -1,0 +1,78 @@
+"""Products of few rows (gemm_rows.cu, skinny_linear.cu) against float64: every padding of the batch, ragged widths and depths, tiles shared
+by several blocks, one block over several tiles, packed weights, the epilogue, and the same bits from run to run."""
+import pytest
+import torch
+
+from transformers_fusion_b200.ops import _lib, functional as F
+from transformers_fusion_b200.quant import wq
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return ((a.double() - b).norm() / b.norm()).item()
+
+
+def _rows(x, w, out, bias=None, residual=None, alpha=1.0, act=0):
+    _lib.check(_lib.lib().tfb_gemm_rows(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), x.shape[0], w.shape[0],
+                                        x.shape[1], _lib.ptr(bias), _lib.ptr(residual), residual.stride(0) if residual is not None else 0, alpha, act,
+                                        int(out.dtype == torch.float32), 0, _lib.status_word().data_ptr(), _lib.stream()), "gemm_rows")
+
+
+# 128 x 64: one unit; 40 x 8: less than a tile and a k-block; 4096 x 14336: five blocks share a tile; 20000 x 200: a block holds several tiles
+@pytest.mark.parametrize("N,K", [(128, 64), (40, 8), (1536, 512), (1000, 776), (6144, 4096), (4096, 14336), (20000, 200)])
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64, 65, 128])
+def test_gemm_rows(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N)
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    ref = x.double() @ w.double().t()
+    outs = []
+    for _ in range(3):          # counters and partial sums are left ready for the next product
+        out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float32)
+        _rows(x, w, out)
+        outs.append(out)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    # fp32 sums of K products of bf16 values: rounding errors of about sqrt(K) 2^-24
+    assert _rel(outs[0], ref) < 2e-6 + 1e-7 * K ** 0.5
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 1000, 4096), (16, 512, 512), (40, 6144, 4096), (64, 1408, 512), (100, 17000, 768)])
+def test_few_rows_epilogue(M, N, K):
+    """Through the public products: bias, residual with a row pitch of its own, alpha, activation, bf16 and fp32 results, weights fetched ahead."""
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
+    bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N + 24, device="cuda").bfloat16()[:, 8:8 + N]
+    prod = x.double() @ w.double().t()
+    want = 0.5 * prod + bias.double()
+    assert _rel(F.gemm(x, w, bias=bias, residual=res, alpha=0.5), want + res.double()) < 3e-3          # bf16 results: 2^-9
+    assert _rel(F.gemm(x, w, bias=bias, alpha=0.5, act="silu"), torch.nn.functional.silu(want)) < 3e-3
+    assert _rel(F.gemm(x, w, out_dtype=torch.float32), prod) < 1e-5
+    assert _rel(F.linear(x, w, bias, res), prod + bias.double() + res.double()) < 3e-3
+    y = torch.empty(M, N + 1, device="cuda", dtype=torch.bfloat16)[:, 1:]                              # rows on odd addresses
+    assert _rel(F.gemm(x, w, out=y), prod) < 3e-3
+    torch.cuda.synchronize()
+    _lib.check_status()
+
+
+def test_rows_under_capture_and_on_streams():
+    """Captured products share one workspace, eager ones have one per stream; more streams than workspaces take the general path."""
+    x, w = torch.randn(8, 4096, device="cuda").bfloat16(), (torch.randn(6144, 4096, device="cuda") / 64).bfloat16()
+    ref = F.gemm(x, w)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = F.linear(F.linear(x, w)[:, :4096].contiguous(), w)
+    for _ in range(3):
+        graph.replay()
+    z = F.linear(ref[:, :4096].contiguous(), w)
+    assert torch.equal(y, z)
+    outs = []
+    torch.cuda.synchronize()
+    for _ in range(9):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            outs.append(F.gemm(x, w))
+    torch.cuda.synchronize()
+    for o in outs:
+        assert _rel(o, ref.double()) < 3e-3

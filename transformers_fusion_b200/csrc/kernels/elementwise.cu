@@ -258,14 +258,14 @@ TFB_API int tfb_rope(void* x, const float* cos_t, const float* sin_t, const int*
                      int pos_offset, int n_heads, int D, long long ld, int backward, void* stream) {
   if (D % 16 || ld % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) return TFB_ERR_ARG;
   const long long work = (long long)T * n_heads * (D / 16);
-  tfb::launch_k(rope_kernel, grid_for(work), 256, 0, static_cast<cudaStream_t>(stream), 
+  tfb::launch_k_rows(T, rope_kernel, grid_for(work), 256, 0, static_cast<cudaStream_t>(stream), 
       static_cast<__nv_bfloat16*>(x), cos_t, sin_t, positions, T, S, pos_offset, n_heads, D, ld, backward ? -1.f : 1.f);
   return int(cudaGetLastError());
 }
 
 TFB_API int tfb_glu_fwd_rows(const void* in, void* out, long long M, int F, int act, const int* rows_dev, void* stream) {
   if (F % 8) return TFB_ERR_ARG;
-  tfb::launch_k(glu_fwd_kernel, grid_for(M * (F / 8)), 256, 0, static_cast<cudaStream_t>(stream), 
+  tfb::launch_k_rows(M, glu_fwd_kernel, grid_for(M * (F / 8)), 256, 0, static_cast<cudaStream_t>(stream), 
       static_cast<const __nv_bfloat16*>(in), static_cast<__nv_bfloat16*>(out), M, F, act, rows_dev);
   return int(cudaGetLastError());
 }
@@ -299,7 +299,7 @@ TFB_API int tfb_act_bwd(const void* x, const void* dy, void* dx, long long n, in
 TFB_API int tfb_embedding_fwd(const long long* ids, const void* W, const void* P, void* out, int T, int S, int H, int V,
                               void* stream) {
   if (H % 8) return TFB_ERR_ARG;
-  tfb::launch_k(embedding_fwd_kernel, grid_for((long long)T * (H / 8)), 256, 0, static_cast<cudaStream_t>(stream), 
+  tfb::launch_k_rows(T, embedding_fwd_kernel, grid_for((long long)T * (H / 8)), 256, 0, static_cast<cudaStream_t>(stream), 
       ids, static_cast<const __nv_bfloat16*>(W), static_cast<const __nv_bfloat16*>(P), static_cast<__nv_bfloat16*>(out),
       T, S, H, V);
   return int(cudaGetLastError());

@@ -276,16 +276,6 @@ struct SmemLayout {
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;  // + barriers + alignment slack
 };
 
-__device__ __forceinline__ float apply_act(float v, int act) {
-  switch (act) {
-    case 1: return fmaxf(v, 0.f);
-    case 2: return gelu_tanh(v);
-    case 3: return silu(v);
-    case 4: v = fmaxf(v, 0.f); return v * v;
-    default: return v;
-  }
-}
-
 template <bool A_MN, bool B_MN, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -815,10 +805,22 @@ __global__ void __launch_bounds__(256) splitk_finalize_kernel(float* __restrict_
 static int gemm_impl(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* C,
                      long long ldc, int M, int N, int K, const void* bias, const void* residual, long long ldr,
                      float alpha, int act, int out_mode, int max_ctas, const TfbGemmGroup* grp, int* status,
-                     void* stream, const TfbGemmTp* tp = nullptr, int force_splits = 0) {
+                     void* stream, const TfbGemmTp* tp = nullptr, int force_splits = 0, int w_static = 0) {
   using namespace tfb;
   if (M <= 0 || N <= 0 || K <= 0) return TFB_ERR_ARG;
   if (out_mode != 0 && (bias || residual || act)) return TFB_ERR_ARG;
+  if (!grp && !tp && !a_mn && !b_mn && out_mode != 2 && max_ctas <= 0 && M <= 128) {
+    // Few rows: the weights are streamed once.  Above 64 rows only where the tiles of 128 weight rows alone nearly fill the machine
+    // (us, streaming form against this kernel's split form with its finalize: 28672 x 4096 at 128 rows 53.8 against 86.5, 64 rows 46.9
+    // against 62.9, 1 row 44.7 against 43.9; 4096 x 4096 at 128 rows 20.4 against 18.9, 64 rows 15.6 against 15.4, 1 row 12.4
+    // against 13.0; 4096 x 14336 at 128 rows 34.8 against 31.5, 64 rows 29.0 against 28.2, 1 row 26.5 against 24.9).  With the weights
+    // fetched ahead (w_static) the streaming form gains another 1 - 3 us.
+    int rc0 = gemm_skinny(A, lda, B, ldb, C, ldc, M, N, K, bias, residual, ldr, alpha, act, out_mode == 1, stream);
+    if (rc0 == TFB_NOT_TAKEN && (M <= 64 || N >= 16384))
+      rc0 = gemm_rows(A, lda, B, ldb, nullptr, nullptr, -1, 0, C, ldc, M, N, K, K, bias, residual, ldr, alpha, act, out_mode == 1, w_static, status,
+                      stream);
+    if (rc0 != TFB_NOT_TAKEN) return rc0;
+  }
   const int gmode = grp ? grp->mode : 0;
   const int E = (gmode != 0) ? grp->num_experts : 1;
   if (gmode == 2 && out_mode == 0) return TFB_ERR_ARG;
@@ -1016,6 +1018,13 @@ TFB_API int tfb_gemm_bf16(const void* A, long long lda, int a_mn, const void* B,
                           float alpha, int act, int out_mode, int max_ctas, int* status, void* stream) {
   return gemm_impl(A, lda, a_mn, B, ldb, b_mn, C, ldc, M, N, K, bias, residual, ldr, alpha, act, out_mode, max_ctas,
                    nullptr, status, stream);
+}
+
+// The same for weights of a model that serves: the caller promises that the kernel launched just before this one on the stream does not
+// write B, so that a product of few rows may begin to fetch it before that kernel has ended.
+TFB_API int tfb_gemm_bf16_static(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
+                                 const void* bias, const void* residual, long long ldr, int out_mode, int* status, void* stream) {
+  return gemm_impl(A, lda, 0, B, ldb, 0, C, ldc, M, N, K, bias, residual, ldr, 1.f, 0, out_mode, 0, nullptr, status, stream, nullptr, 0, 1);
 }
 
 // Grouped (mixture-of-experts) form; see TfbGemmGroup.  Mode 1: M counts the padded rows of all experts, B is

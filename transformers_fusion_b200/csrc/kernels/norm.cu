@@ -412,7 +412,7 @@ static int launch_fwd(const void* x, const void* res, const void* w, const void*
   auto B = static_cast<const __nv_bfloat16*>(b);
   auto Y = static_cast<__nv_bfloat16*>(y);
   auto Ho = static_cast<__nv_bfloat16*>(h_out);
-#define TFB_GO(KERN, blocks) tfb::launch_k(KERN, blocks, 256, 0, st, X, R, W, B, Y, Ho, rstd, mean, rows, H, eps)
+#define TFB_GO(KERN, blocks) tfb::launch_k_rows(rows, KERN, blocks, 256, 0, st, X, R, W, B, Y, Ho, rstd, mean, rows, H, eps)
   const int warps8 = (rows + 7) / 8;
   if (H <= 512) TFB_GO((norm_fwd_kernel<2, LN>), warps8);
   else if (H <= 1024) TFB_GO((norm_fwd_kernel<4, LN>), warps8);

@@ -746,7 +746,7 @@ static int launch_decode_mma(dim3 grid, cudaStream_t st, const __nv_bfloat16* q,
   static DeviceOnce once;
   auto kern = paged_decode_mma_kernel<MODE, D>;
   if (int e = ensure_dyn_smem(once, kern, SMEM)) return e;
-  tfb::launch_k(kern, grid, TC_THREADS, SMEM, st, q, ldq, k, v, bt, max_pages, lens, acc, ml, Hq, Hkv, G, splits, scale, status);
+  tfb::launch_k_pdl(kern, grid, TC_THREADS, SMEM, st, q, ldq, k, v, bt, max_pages, lens, acc, ml, Hq, Hkv, G, splits, scale, status);
   return int(cudaGetLastError());
 }
 
@@ -756,7 +756,7 @@ static int launch_decode_g(int G, dim3 grid, cudaStream_t st, const __nv_bfloat1
                            int splits, float scale) {
 #define TFB_CASE(GG)                                                                                              \
   case GG:                                                                                                        \
-    tfb::launch_k(paged_decode_kernel<MODE, D, GG>, grid, DEC_THREADS, 0, st, q, ldq, k, v, bt, max_pages, lens, acc, ml, Hq, \
+    tfb::launch_k_pdl(paged_decode_kernel<MODE, D, GG>, grid, DEC_THREADS, 0, st, q, ldq, k, v, bt, max_pages, lens, acc, ml, Hq, \
                                                                    Hkv, splits, scale);                           \
     break;
   switch (G) {
@@ -881,9 +881,9 @@ TFB_API int tfb_kv_append(const void* src, long long ld, int k_col0, int v_col0,
   const unsigned blocks = unsigned((warps * 32 + 255) / 256);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto s = static_cast<const __nv_bfloat16*>(src);
-  if (mode == KV_BF16) tfb::launch_k(kv_append_kernel<KV_BF16>, blocks, 256, 0, st, s, ld, k_col0, v_col0, slot_mapping, kp, vp, T, Hkv, D);
-  else if (mode == KV_FP8) tfb::launch_k(kv_append_kernel<KV_FP8>, blocks, 256, 0, st, s, ld, k_col0, v_col0, slot_mapping, kp, vp, T, Hkv, D);
-  else if (mode == KV_Q4) tfb::launch_k(kv_append_kernel<KV_Q4>, blocks, 256, 0, st, s, ld, k_col0, v_col0, slot_mapping, kp, vp, T, Hkv, D);
+  if (mode == KV_BF16) tfb::launch_k_rows(T, kv_append_kernel<KV_BF16>, blocks, 256, 0, st, s, ld, k_col0, v_col0, slot_mapping, kp, vp, T, Hkv, D);
+  else if (mode == KV_FP8) tfb::launch_k_rows(T, kv_append_kernel<KV_FP8>, blocks, 256, 0, st, s, ld, k_col0, v_col0, slot_mapping, kp, vp, T, Hkv, D);
+  else if (mode == KV_Q4) tfb::launch_k_rows(T, kv_append_kernel<KV_Q4>, blocks, 256, 0, st, s, ld, k_col0, v_col0, slot_mapping, kp, vp, T, Hkv, D);
   else return TFB_ERR_ARG;
   return int(cudaGetLastError());
 }
@@ -920,6 +920,6 @@ TFB_API int tfb_paged_decode(const void* q, long long ldq, void* k_data, void* k
   else return TFB_ERR_ARG;
 #undef TFB_GO
   if (rc) return rc;
-  tfb::launch_k(paged_combine_kernel, dim3(B, Hq), 128, 0, st, acc_ws, ml_ws, static_cast<__nv_bfloat16*>(o), ldo, Hq, D, splits);
+  tfb::launch_k_pdl(paged_combine_kernel, dim3(B, Hq), 128, 0, st, acc_ws, ml_ws, static_cast<__nv_bfloat16*>(o), ldo, Hq, D, splits);
   return int(cudaGetLastError());
 }

@@ -22,6 +22,9 @@ struct SkinnyArgs {
   const __nv_bfloat16* gate;        // [M, ldg] or null: head h is multiplied by sigmoid(gate[:, h])
   long long ldg;
   const __nv_bfloat16* bias;        // [N] or null
+  const __nv_bfloat16* residual;    // [M, ldr] or null, added last
+  long long ldr;
+  float alpha;
 };
 
 struct Row16 { uint32_t u[8]; };      // 16 consecutive entries of a row
@@ -78,12 +81,14 @@ __global__ void __launch_bounds__(SK_WARPS * 32) skinny_linear_kernel(const Skin
     float v = 0.f;
 #pragma unroll
     for (int w = 0; w < SK_WARPS; ++w) v += red[w][m][n];
+    v *= p.alpha;
     if (p.bias) v += __bfloat162float(p.bias[n0 + n]);
     if (p.act == 4) {
       v = fmaxf(v, 0.f);
       v *= v;
     }
     if (p.gate) v *= 1.f / (1.f + expf(-__bfloat162float(p.gate[(m0 + m) * p.ldg + h])));
+    if (p.residual) v += __bfloat162float(p.residual[(m0 + m) * p.ldr + n0 + n]);
     const long long at = (m0 + m) * p.ldo + (long long)h * p.out_head + n0 + n;
     if (p.out_f32) static_cast<float*>(p.out)[at] = v;
     else static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16(v);
@@ -105,11 +110,24 @@ static int launch_skinny(const tfb::SkinnyArgs& p, int heads, int rows, void* st
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows == 0) rows = p.M <= 16 || tfb_skinny_work(p.M, p.N * heads, p.K) <= 1500000 ? 16 : 32;
   const dim3 grid((p.N + SK_N - 1) / SK_N, heads, (p.M + rows - 1) / rows);
-  if (rows == 16) launch_k(skinny_linear_kernel<1>, grid, SK_WARPS * 32, 0, st, p);
-  else if (rows == 32) launch_k(skinny_linear_kernel<2>, grid, SK_WARPS * 32, 0, st, p);
-  else if (rows == 64) launch_k(skinny_linear_kernel<4>, grid, SK_WARPS * 32, 0, st, p);
+  if (rows == 16) launch_k_pdl(skinny_linear_kernel<1>, grid, SK_WARPS * 32, 0, st, p);
+  else if (rows == 32) launch_k_pdl(skinny_linear_kernel<2>, grid, SK_WARPS * 32, 0, st, p);
+  else if (rows == 64) launch_k_pdl(skinny_linear_kernel<4>, grid, SK_WARPS * 32, 0, st, p);
   else return TFB_ERR_ARG;
   return int(cudaGetLastError());
+}
+
+// The dense decoder's products: taken while the weights are small (a set-up and drain of a few microseconds is then most of the tcgen05
+// forms' time) and the operands are read few times over.  Measured, us, against the streaming form of gemm_rows.cu: 1536 x 512
+// at 1 / 16 / 64 rows 2.1 / 2.3 / 3.4 against 6.2 / 6.0 / 7.4; 512 x 1408 2.9 / 3.2 / 3.3 against 6.9 / 7.2 / 9.9; 4096 x 4096 12.5 /
+// 12.8 / 21.6 against 12.4 / 12.6 / 15.6; 28672 x 4096 at 1 row 54.5 against 44.7.
+int tfb::gemm_skinny(const void* x, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int N, int K, const void* bias,
+                     const void* residual, long long ldr, float alpha, int act, int out_f32, void* stream) {
+  if (M > 64 || (act != 0 && act != 4) || tfb_skinny_work(M, N, K) > 700000) return TFB_NOT_TAKEN;
+  if (M <= 0 || N <= 0 || K <= 0 || K % 8 || ldx % 8 || ldw % 8 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(W) & 15))
+    return TFB_NOT_TAKEN;
+  return launch_skinny(SkinnyArgs{static_cast<const bf16*>(x), static_cast<const bf16*>(W), ldx, ldw, C, ldc, M, N, K, act, out_f32, 0, 0, nullptr, 0,
+                                  static_cast<const bf16*>(bias), static_cast<const bf16*>(residual), ldr, alpha}, 1, 0, stream);
 }
 
 // 1 where the few-row form is the one to take.  Measured against the tcgen05 form (with its split-K finalize): it wins while a warp's share
@@ -123,7 +141,7 @@ TFB_API int tfb_skinny_linear(const void* x, long long ldx, const void* w, long 
                               int out_f32, int rows, const void* bias, void* stream) {
   if (M > 64 || (act != 0 && act != 4)) return TFB_ERR_ARG;
   return launch_skinny(tfb::SkinnyArgs{static_cast<const bf16*>(x), static_cast<const bf16*>(w), ldx, ldw, out, ldo, M, N, K, act, out_f32, 0, 0,
-                                       nullptr, 0, static_cast<const bf16*>(bias)}, 1, rows, stream);
+                                       nullptr, 0, static_cast<const bf16*>(bias), nullptr, 0, 1.f}, 1, rows, stream);
 }
 
 // One product per head: x [M, ldx] (x_head entries between heads), w: heads blocks [N, K] stacked on the rows, out [M, ldo] (N entries per
@@ -131,5 +149,5 @@ TFB_API int tfb_skinny_linear(const void* x, long long ldx, const void* w, long 
 TFB_API int tfb_skinny_linear_heads(const void* x, long long ldx, int x_head, const void* w, long long ldw, void* out, long long ldo, const void* gate,
                                     long long ldg, int M, int heads, int N, int K, int rows, void* stream) {
   return launch_skinny(tfb::SkinnyArgs{static_cast<const bf16*>(x), static_cast<const bf16*>(w), ldx, ldw, out, ldo, M, N, K, 0, 0, x_head, N,
-                                       static_cast<const bf16*>(gate), ldg, nullptr}, heads, rows, stream);
+                                       static_cast<const bf16*>(gate), ldg, nullptr, nullptr, 0, 1.f}, heads, rows, stream);
 }

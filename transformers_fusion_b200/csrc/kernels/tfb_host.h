@@ -41,12 +41,21 @@ int sm_count();
 // CTAs of the next kernel take shared memory and registers from the tail of the running one.
 int pdl_enabled();
 
+// gemm_rows.cu, skinny_linear.cu: products of few rows.  x [M, K], W [N, K] (or codes and scales of a packed weight, fmt >= 0).
+// Both return 0, a CUDA error, or TFB_NOT_TAKEN where the general path is to run.
+constexpr int TFB_NOT_TAKEN = -100;
+int gemm_rows(const void* x, long long ldx, const void* W, long long ldw, const void* codes, const void* scales, int fmt, int group, void* C,
+              long long ldc, int M, int N, int K, int Kw, const void* bias, const void* residual, long long ldr, float alpha, int act, int out_f32,
+              int w_static, int* status, void* stream);
+int gemm_skinny(const void* x, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int N, int K, const void* bias,
+                const void* residual, long long ldr, float alpha, int act, int out_f32, void* stream);
+
 // Launch of a kernel of this library: same meaning as kernel<<<grid, block, smem, stream>>>(args...), plus the launch
 // attribute that lets the kernel's CTAs be placed while the previous kernel of the stream drains (each kernel starts with
 // pdl_sync(), or with its own set-up followed by pdl_sync(), so nothing is read early).  Errors surface through
 // cudaGetLastError() as with the <<<>>> form.
 template <class... KArgs, class... Args>
-inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline void launch_attr(int pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -54,10 +63,30 @@ inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled();
+  attr[0].val.programmaticStreamSerializationAllowed = pdl;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   (void)cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+template <class... KArgs, class... Args>
+inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  launch_attr(pdl_enabled(), kern, grid, block, smem, stream, std::forward<Args>(args)...);
+}
+// The same with programmatic launch always allowed: kernels of a decode step, a few microseconds each, where the gap between
+// two launches and the set-up of the next are a large part of the time.
+template <class... KArgs, class... Args>
+inline void launch_k_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  launch_attr(1, kern, grid, block, smem, stream, std::forward<Args>(args)...);
+}
+
+// For kernels that serve decode steps as well as whole batches: programmatic launch up to 256 rows (a decode batch, a short prompt).
+// A decode step of 8 layers of the 8b widths at one sequence spends about 110 launches on 1 ms of work; on launches of
+// whole training batches early-placed blocks only take room from the running kernel's tail (31.1 -> 32.0 ms a step).
+constexpr long long PDL_ROWS = 256;
+template <class... KArgs, class... Args>
+inline void launch_k_rows(long long rows, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  launch_attr(rows <= PDL_ROWS ? 1 : pdl_enabled(), kern, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 // One-time set-up per device.  Kernel attributes (cudaFuncSetAttribute) belong to the device that is current when

@@ -88,7 +88,11 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // Bounded wait. `abort_flag` is a shared-memory word any role sets when it gives up.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+  // the instruction itself waits for a while; the clock is read only when that has not helped (a read takes about as long as a
+  // k-block of a product)
+#pragma unroll 1
+  for (int i = 0; i < 64; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   uint32_t it = 0;
   while (true) {
@@ -364,5 +368,14 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   return 0.5f * x * (1.f + tanhf(k * (x + 0.044715f * x * x * x)));
 }
 __device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
+__device__ __forceinline__ float apply_act(float v, int act) {
+  switch (act) {
+    case 1: return fmaxf(v, 0.f);
+    case 2: return gelu_tanh(v);
+    case 3: return silu(v);
+    case 4: v = fmaxf(v, 0.f); return v * v;
+    default: return v;
+  }
+}
 
 }  // namespace tfb

@@ -266,7 +266,7 @@ class InferenceEngine:
         """x @ W^T (+ bias) (+ residual) with W either the bf16 parameter or its packed low-bit form."""
         pw = self.packed.get(f"layers.{li}.{name}")
         if pw is None:
-            return F.gemm(x, w.data, bias=bias, residual=residual)
+            return F.linear(x, w.data, bias, residual)
         y = self._wq.gemm_wq(x, pw, bias)
         return y if residual is None else y + residual
 
@@ -516,7 +516,7 @@ class InferenceEngine:
         if self.stack:
             return m.head(h)
         f, _ = _norm_fwd(m.cfg, h, m.norm, m.norm_bias)
-        return F.gemm(f, m.lm_head.data)
+        return F.linear(f, m.lm_head.data)
 
     def _sample_dev(self, logits, reqs):
         """Sampled token ids as a device tensor [len(reqs)] (no host synchronisation)."""

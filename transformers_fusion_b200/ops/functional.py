@@ -80,6 +80,20 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, bias=None, r
     return out
 
 
+def linear(x, w, bias=None, residual=None):
+    """x [M, K] @ w [N, K]^T + bias + residual for the weights of a model that serves: they must not be written by the kernel that is
+    launched just before (products of few rows fetch them ahead of its end)."""
+    if not x.is_cuda:
+        return gemm(x, w, bias=bias, residual=residual)
+    (M, K), N = x.shape, w.shape[0]
+    assert w.shape[1] == K and x.dtype == w.dtype == torch.bfloat16 and x.stride(-1) == 1 and w.stride(-1) == 1
+    out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    check(_lib.lib().tfb_gemm_bf16_static(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), N, M, N, K, ptr(bias), ptr(residual),
+                                          residual.stride(0) if residual is not None else 0, 0, _lib.status_word(x.device).data_ptr(), stream()),
+          "linear")
+    return out
+
+
 # ---------------------------------------------------------------------------------------------
 # normalisation
 # ---------------------------------------------------------------------------------------------

@@ -17,9 +17,9 @@ from . import _lib
 from . import functional as F
 from ._lib import c_f, c_i, c_ll, c_p, check, ptr, stream
 
-UNITS = ("tfb_host", "gemm_bf16", "skinny_linear", "stack_ops", "diff_attention", "delta_rule")    # translation units these operators need
-UNITS_LATENT = ("tfb_host", "gemm_bf16", "skinny_linear", "stack_ops", "head_attention", "latent_attention", "moe_serve")
-UNITS_GATED = ("tfb_host", "gemm_bf16", "skinny_linear", "stack_ops", "head_attention", "gated_linear", "moe_serve")
+UNITS = ("tfb_host", "gemm_bf16", "gemm_rows", "skinny_linear", "stack_ops", "diff_attention", "delta_rule")    # translation units these operators need
+UNITS_LATENT = ("tfb_host", "gemm_bf16", "gemm_rows", "skinny_linear", "stack_ops", "head_attention", "latent_attention", "moe_serve")
+UNITS_GATED = ("tfb_host", "gemm_bf16", "gemm_rows", "skinny_linear", "stack_ops", "head_attention", "gated_linear", "moe_serve")
 UNITS_STREAMS = UNITS_GATED + ("streams",)
 PAGE = 16
 ACT = {None: 0, "relu2": 4}      # codes of the product epilogues (gemm_bf16.cu: apply_act)

@@ -178,12 +178,10 @@ class _DecodeGraph:
     def __init__(self, eng, bucket: int):
         dev = eng.device
         self.bucket = bucket
-        self.tokens = torch.zeros(bucket, dtype=torch.int64, device=dev)
-        self.positions = torch.zeros(bucket, dtype=torch.int32, device=dev)
-        self.bt = torch.zeros((bucket, eng.max_pages), dtype=torch.int32, device=dev)
-        self.slots = torch.full((bucket,), -1, dtype=torch.int64, device=dev)
-        self.state_slots = torch.full((bucket,), -1, dtype=torch.int32, device=dev)
-        run = lambda: eng._logits(eng._layers_decode(self.tokens, self.positions, self.bt, self.slots, self.state_slots))
+        self.inp = torch.zeros((4, bucket), dtype=torch.int64, device=dev)       # tokens, positions, slots, state slots
+        self.inp[2:].fill_(-1)
+        bt = eng._table()[:bucket]                                               # the scheduler's own table: always current
+        run = lambda: eng._logits(eng._layers_decode(self.inp[0], self.inp[1].to(torch.int32), bt, self.inp[2], self.inp[3].to(torch.int32)))
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):                  # warm-up outside capture: workspaces, status words, lazy tables
@@ -192,7 +190,6 @@ class _DecodeGraph:
         torch.cuda.current_stream(dev).wait_stream(side)
         torch.cuda.synchronize(dev)
         self.graph = torch.cuda.CUDAGraph()
-        self._last_n = -1
         self.eng = eng
         self.token = eng._graph_capture_begin()
         # "relaxed": API calls that a capture in the default (global) mode forbids process-wide - an event query or a free by
@@ -202,18 +199,12 @@ class _DecodeGraph:
             self.logits = run()
             eng._graph_capture_end(self.token)
 
-    def replay(self, tokens, positions, bt, slots, state_slots):
-        n = tokens.shape[0]
-        self.tokens[:n].copy_(tokens, non_blocking=True)
-        self.positions[:n].copy_(positions, non_blocking=True)
-        self.bt[:n].copy_(bt, non_blocking=True)
-        self.slots[:n].copy_(slots, non_blocking=True)
-        self.state_slots[:n].copy_(state_slots, non_blocking=True)
-        if n < self.bucket and n != self._last_n:      # rows past the live batch: reset once per batch size
-            self.positions[n:].zero_()
-            self.slots[n:].fill_(-1)
-            self.state_slots[n:].fill_(-1)
-        self._last_n = n
+    def replay(self, rows, n, pending=None, prev_tokens=None):
+        """``rows``: four lists of the bucket's length for ``inp``; ``pending``: see ``_decode_logits``."""
+        self.eng._upload(sum(rows, []), self.inp.view(-1))
+        if pending is not None:
+            src, tokens = self.eng._upload(pending), self.inp[0, :n]
+            tokens.copy_(torch.where(src >= 0, prev_tokens[src.clamp(min=0)], tokens))
         self.eng._graph_before_replay(self.token)
         self.graph.replay()
         return self.logits[:n]
@@ -240,7 +231,8 @@ class InferenceEngine:
         self._step = 0
         self._graphs = {}
         self._sample_cache = None
-        self._bt_cache = None
+        self._bt_dev, self._bt_rows = None, []      # block table on the device; (request id, pages) of what its rows hold
+        self._uploads = None                        # ring of pinned slots: (memory, slot size, events, next slot)
         self._inflight = None          # (requests, device tokens, pinned host tokens, event) of the decode step in flight
         self._tok_host = None
         self.stats = InferenceStats()
@@ -649,23 +641,23 @@ class InferenceEngine:
         for r in reqs:
             if r.pos // PAGE >= len(r.pages):
                 r.pages.append(alloc.alloc())
-        # host tokens, positions, slots, state slots and pending rows travel in one small upload; the block table only
-        # re-sends what changed
-        packed = torch.tensor([host_tokens, [r.pos for r in reqs], [self._slot(r, r.pos) for r in reqs],
-                               [r.state_slot for r in reqs], pending or [-1] * len(reqs)], dtype=torch.int64).to(dev)
-        tokens, positions, slots, state_slots = packed[0], packed[1].to(torch.int32), packed[2], packed[3].to(torch.int32)
-        if pending is not None:
-            src = packed[4]
-            tokens = torch.where(src >= 0, prev_tokens[src.clamp(min=0)], tokens)
+        # host tokens, positions, slots and state slots travel in one small upload; the block table only re-sends what changed
+        n, rows = len(reqs), [list(host_tokens), [r.pos for r in reqs], [self._slot(r, r.pos) for r in reqs], [r.state_slot for r in reqs]]
         bt = self._block_table(reqs)
         if self.cfg.cuda_graph and dev.type == "cuda":
-            bucket = self._bucket(len(reqs))
+            bucket = self._bucket(n)
             g = self._graphs.get(bucket)
             if g is None:
                 g = self._graphs[bucket] = _DecodeGraph(self, bucket)
-            logits = g.replay(tokens, positions, bt, slots, state_slots)
+            # rows past the live batch: no cache write, one token of whatever page their table row names, logits ignored
+            logits = g.replay([x + [fill] * (bucket - n) for x, fill in zip(rows, (0, 0, -1, -1))], n, pending, prev_tokens)
         else:
-            logits = self._logits(self._layers_decode(tokens, positions, bt, slots, state_slots))
+            packed = self._upload(sum(rows, [])).view(4, n)
+            tokens = packed[0]
+            if pending is not None:
+                src = self._upload(pending)
+                tokens = torch.where(src >= 0, prev_tokens[src.clamp(min=0)], tokens)
+            logits = self._logits(self._layers_decode(tokens, packed[1].to(torch.int32), bt, packed[2], packed[3].to(torch.int32)))
         for r in reqs:
             r.pos += 1
             self._drop_old_pages(r)
@@ -782,15 +774,42 @@ class InferenceEngine:
                 self._emit(r, tok, finished)
         self.running = [r for r in self.running if not r.finished]
 
+    def _table(self):
+        if self._bt_dev is None:
+            self._bt_dev = torch.zeros((self._bucket(self.cfg.max_batch), self.max_pages), dtype=torch.int32, device=self.device)
+        return self._bt_dev
+
+    def _upload(self, values, out=None):
+        """Whole numbers of the host as an int64 device tensor (``out``: where), through a ring of pinned slots: the host goes on
+        while earlier steps run, and waits only for the copy that last used a slot.  A copy from pageable memory would
+        hold the host until the device has caught up, and the device would then wait for the host at every step."""
+        dev, k = self.device, len(values)
+        if dev.type == "cuda" and self._uploads is None:
+            size = max(5 * self._bucket(self.cfg.max_batch), 512)
+            self._uploads = [_pinned_token_buffers(dev, 8 * size), size, [None] * 8, 0]
+        if dev.type != "cuda" or k > self._uploads[1]:
+            t = torch.tensor(values, dtype=torch.int64).to(dev)
+            return t if out is None else out.copy_(t)
+        memory, size, events, i = self._uploads
+        if events[i] is None:
+            events[i] = torch.cuda.Event()
+        else:
+            events[i].synchronize()
+        slot = memory[0][i * size:i * size + k]
+        slot.copy_(torch.tensor(values, dtype=torch.int64))
+        out = torch.empty(k, dtype=torch.int64, device=dev) if out is None else out
+        out.copy_(slot, non_blocking=True)
+        events[i].record()
+        self._uploads[3] = (i + 1) % 8
+        return out
+
     def _block_table(self, reqs):
         """Device block table [len(reqs), max_pages] for the running sequences.  The table lives on the device; a step
         uploads only what changed since the last one - the page a sequence has just started, or the whole row when a
         different request now sits in that row - as one (index, value) list.  Entries past a sequence's last page may be
         stale: the kernels read pages below ceil(length / 16) only."""
-        dev, mp = self.device, self.max_pages
-        if self._bt_cache is None:
-            self._bt_cache = (torch.zeros((self.cfg.max_batch, mp), dtype=torch.int32, device=dev), [])
-        table, rows = self._bt_cache
+        mp = self.max_pages
+        table, rows = self._table(), self._bt_rows
         idx, val = [], []
         for i, r in enumerate(reqs):
             n = len(r.pages)
@@ -809,7 +828,7 @@ class InferenceEngine:
                 rows.append((r.id, n))
         del rows[len(reqs):]
         if idx:
-            u = torch.tensor([idx, val], dtype=torch.int64).to(dev)
+            u = self._upload(idx + val).view(2, -1)
             table.view(-1).index_copy_(0, u[0], u[1].to(torch.int32))
         return table[:len(reqs)]
 

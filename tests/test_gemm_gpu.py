@@ -113,3 +113,21 @@ def test_gemm_tile_edge_sweep(a_mn, b_mn):
     torch.cuda.synchronize()
     _lib.check_status()
     assert worst > 0.0
+
+
+@pytest.mark.parametrize("am,bm", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(136, 2816, 512), (256, 256, 64), (304, 1000, 776), (512, 264, 200), (1000, 1536, 1408), (2048, 4096, 4096)])
+def test_gemm_on_cta_pairs(M, N, K, am, bm):
+    """256 x 256 tiles of CTA pairs: a second half past the last row, ragged columns and depth, split sums, every epilogue."""
+    a = torch.randn((K, M) if am else (M, K), device="cuda").bfloat16()
+    b = (torch.randn((K, N) if bm else (N, K), device="cuda") * K ** -0.5).bfloat16()
+    ref = (a.t() if am else a).double() @ (b if bm else b.t()).double()
+    rel = lambda x, r: ((x.double() - r).norm() / r.norm()).item()
+    res, bias = torch.randn(M, N, device="cuda").bfloat16(), torch.randn(N, device="cuda").bfloat16()
+    assert rel(F.gemm(a, b, a_mn=am, b_mn=bm, bias=bias, residual=res), ref + bias.double() + res.double()) < 3e-3     # bf16 results: 2^-9
+    assert rel(F.gemm(a, b, a_mn=am, b_mn=bm, bias=bias, act="gelu"), torch.nn.functional.gelu(ref + bias.double(), approximate="tanh")) < 3e-3
+    assert rel(F.gemm(a, b, a_mn=am, b_mn=bm, out_dtype=torch.float32), ref) < 2e-5
+    c = torch.ones(M, N, device="cuda")
+    assert rel(F.gemm(a, b, a_mn=am, b_mn=bm, out=c, accumulate=True), ref + 1) < 2e-5
+    torch.cuda.synchronize()
+    _lib.check_status()

@@ -276,6 +276,115 @@ struct SmemLayout {
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;  // + barriers + alignment slack
 };
 
+// One 32-row strip of a tile, the columns of half `half`: tensor memory -> registers (alpha, bias, activation, residual) -> swizzled
+// shared-memory slab of 32 rows x 128 bytes -> TMA store or fp32 reduce-add.  Executed by a whole warp.
+template <int BN, int STG_BUFS>
+__device__ __forceinline__ void staged_epilogue(const GemmParams& p, const CUtensorMap& tma_c, const PeerMaps& tma_peers, uint32_t taddr0, int n0,
+                                                int slab_row0, int half, int lane, uint32_t stg_u32, int& sbuf, int cz) {
+  const bool vec_ok_res = p.residual && ((p.ldr & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.residual) & 15) == 0);
+  // ---- staged epilogue: registers -> swizzled shared-memory slab -> TMA store / reduce-add ----
+  const int row = slab_row0 + lane;
+  const bool slab_live = slab_row0 < p.M;            // warp-uniform
+  const uint32_t xr = uint32_t(lane & 7);
+  if (p.out_mode == 0) {
+#pragma unroll 1
+    for (int c = half * (BN / 128); c < (half + 1) * (BN / 128); ++c) {
+      const int col0 = n0 + c * 64;
+      if (col0 >= p.N) break;
+      uint32_t r0[32], r1[32];
+      tmem_ld_32x32(taddr0 + c * 64, r0);
+      tmem_ld_32x32(taddr0 + c * 64 + 32, r1);
+      tmem_ld_wait();
+      if (!slab_live) continue;
+      float v[64];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        v[j] = __uint_as_float(r0[j]) * p.alpha;
+        v[32 + j] = __uint_as_float(r1[j]) * p.alpha;
+      }
+      if (p.bias) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j)
+          if (col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
+      }
+      if (p.act) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) v[j] = apply_act(v[j], p.act);
+      }
+      if (p.residual && row < p.M) {
+        const __nv_bfloat16* rp = p.residual + (long long)row * p.ldr + col0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          if (vec_ok_res && col0 + q * 8 + 8 <= p.N) {
+            const uint4 u = *reinterpret_cast<const uint4*>(rp + q * 8);
+            const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              const float2 f = unpack_bf16(uu[h]);
+              v[q * 8 + h * 2] += f.x;
+              v[q * 8 + h * 2 + 1] += f.y;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (col0 + q * 8 + j < p.N) v[q * 8 + j] += __bfloat162float(rp[q * 8 + j]);
+          }
+        }
+      }
+      if (lane == 0) tma_store_wait_read<STG_BUFS - 1>();   // the slab about to be rewritten has been read by its copy
+      __syncwarp();
+      const uint32_t slab = stg_u32 + sbuf * 4096 + lane * 128;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        st_shared_v4(slab + ((uint32_t(q) ^ xr) << 4), pack_bf16(v[q * 8 + 0], v[q * 8 + 1]), pack_bf16(v[q * 8 + 2], v[q * 8 + 3]),
+                     pack_bf16(v[q * 8 + 4], v[q * 8 + 5]), pack_bf16(v[q * 8 + 6], v[q * 8 + 7]));
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (p.tp_mode & TP_RS) {
+          // rows of shard d go to rank d's staging buffer, slot `rank`: one 32-row x 128-byte slab per copy, so the
+          // bytes cross NVLink in whole lines (tile rows never straddle two shards: shards are multiples of 128 rows)
+          const int d = slab_row0 / p.rs_rows_per_shard;
+          tma_store_3d(&tma_peers.m[d], stg_u32 + sbuf * 4096, col0,
+                       p.rs_rank * p.rs_rows_per_shard + (slab_row0 - d * p.rs_rows_per_shard), 0);
+        } else {
+          tma_store_3d(&tma_c, stg_u32 + sbuf * 4096, col0, slab_row0, 0);
+        }
+        tma_store_commit();
+      }
+      sbuf ^= (STG_BUFS - 1);
+    }
+  } else {
+#pragma unroll 1
+    for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
+      const int col0 = n0 + c * 32;
+      if (col0 >= p.N) break;
+      uint32_t r[32];
+      tmem_ld_32x32(taddr0 + c * 32, r);
+      tmem_ld_wait();
+      if (!slab_live) continue;
+      if (lane == 0) tma_store_wait_read<STG_BUFS - 1>();
+      __syncwarp();
+      const uint32_t slab = stg_u32 + sbuf * 4096 + lane * 128;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        st_shared_v4(slab + ((uint32_t(q) ^ xr) << 4), __float_as_uint(__uint_as_float(r[q * 4]) * p.alpha),
+                     __float_as_uint(__uint_as_float(r[q * 4 + 1]) * p.alpha), __float_as_uint(__uint_as_float(r[q * 4 + 2]) * p.alpha),
+                     __float_as_uint(__uint_as_float(r[q * 4 + 3]) * p.alpha));
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (p.out_mode == 2) tma_reduce_add_3d(&tma_c, stg_u32 + sbuf * 4096, col0, slab_row0, cz);
+        else tma_store_3d(&tma_c, stg_u32 + sbuf * 4096, col0, slab_row0, cz);
+        tma_store_commit();
+      }
+      sbuf ^= (STG_BUFS - 1);
+    }
+  }
+}
+
 template <bool A_MN, bool B_MN, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -418,34 +527,36 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     // ------------------------------ MMA issuer ------------------------------
     if (lane == 0) {
       constexpr uint32_t idesc = umma_idesc(FMT_BF16, FMT_BF16, A_MN, B_MN, BM, BN);
+      // One thread feeds the tensor core an instruction per 64 - 128 cycles: descriptors are a base plus the stage's offset (their
+      // addresses count 16 bytes), and a plain product (every item the whole of K) decodes nothing.
+      const uint32_t adesc0 = umma_desc_lo(smem_base, A_MN ? 8192 : 16), bdesc0 = umma_desc_lo(smem_base + L::A_BYTES, B_MN ? 8192 : 16);
+      constexpr uint32_t ASTEP = A_MN ? 2048 >> 4 : 32 >> 4, BSTEP = B_MN ? 2048 >> 4 : 32 >> 4;
+      const bool plain = p.group_mode == 0 && p.splits == 1;
       int stage = 0;
       uint32_t phase = 0;
       int abuf = 0;
       uint32_t aphase = 0;
       bool ok = true;
       for (int w = cta; w < num_work && ok; w += nctas) {
-        WorkItem it;
-        if (!decode_work(p, w, total_kb, it)) continue;
-        const int kb0 = it.kb0, kb1 = it.kb1;
+        int n_kb = total_kb;
+        if (!plain) {
+          WorkItem it;
+          if (!decode_work(p, w, total_kb, it)) continue;
+          n_kb = it.kb1 - it.kb0;
+        }
         if (!mbar_wait(bar_tempty + abuf * 8, aphase ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + abuf * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < n_kb; ++kb) {
           if (!mbar_wait(bar_full + stage * 8, phase, abort_flag, p.status, ST_TIMEOUT_FULL)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_base + stage * L::STAGE_BYTES;
-          const uint32_t sb = sa + L::A_BYTES;
+          const uint32_t at = uint32_t(stage) * (L::STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = A_MN ? umma_smem_desc(sa + k * 2048, 8192, 1024)
-                                        : umma_smem_desc(sa + k * 32, 16, 1024);
-            const uint64_t bdesc = B_MN ? umma_smem_desc(sb + k * 2048, 8192, 1024)
-                                        : umma_smem_desc(sb + k * 32, 16, 1024);
-            umma_f16_ss(tmem_d, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / 16; ++k)
+            umma_f16_ss_lo(tmem_d, adesc0 + at + k * ASTEP, bdesc0 + at + k * BSTEP, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           umma_commit(bar_empty + stage * 8);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -478,108 +589,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       const int row = m0 + quad * 32 + lane;
       const uint32_t taddr0 = tmem_base + abuf * BN + (uint32_t(quad * 32) << 16);
       if (p.c_tma) {
-        // ---- staged epilogue: registers -> swizzled shared-memory slab -> TMA store / reduce-add ----
-        const int slab_row0 = m0 + quad * 32;
-        const bool slab_live = slab_row0 < p.M;            // warp-uniform
-        const uint32_t xr = uint32_t(lane & 7);
-        if (p.out_mode == 0) {
-#pragma unroll 1
-          for (int c = half * (BN / 128); c < (half + 1) * (BN / 128); ++c) {
-            const int col0 = n0 + c * 64;
-            if (col0 >= p.N) break;
-            uint32_t r0[32], r1[32];
-            tmem_ld_32x32(taddr0 + c * 64, r0);
-            tmem_ld_32x32(taddr0 + c * 64 + 32, r1);
-            tmem_ld_wait();
-            if (!slab_live) continue;
-            float v[64];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              v[j] = __uint_as_float(r0[j]) * p.alpha;
-              v[32 + j] = __uint_as_float(r1[j]) * p.alpha;
-            }
-            if (p.bias) {
-#pragma unroll
-              for (int j = 0; j < 64; ++j)
-                if (col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
-            }
-            if (p.act) {
-#pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] = apply_act(v[j], p.act);
-            }
-            if (p.residual && row < p.M) {
-              const __nv_bfloat16* rp = p.residual + (long long)row * p.ldr + col0;
-#pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                if (vec_ok_res && col0 + q * 8 + 8 <= p.N) {
-                  const uint4 u = *reinterpret_cast<const uint4*>(rp + q * 8);
-                  const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                  for (int h = 0; h < 4; ++h) {
-                    const float2 f = unpack_bf16(uu[h]);
-                    v[q * 8 + h * 2] += f.x;
-                    v[q * 8 + h * 2 + 1] += f.y;
-                  }
-                } else {
-#pragma unroll
-                  for (int j = 0; j < 8; ++j)
-                    if (col0 + q * 8 + j < p.N) v[q * 8 + j] += __bfloat162float(rp[q * 8 + j]);
-                }
-              }
-            }
-            if (lane == 0) tma_store_wait_read<L::STG_BUFS - 1>();   // the slab about to be rewritten has been read by its copy
-            __syncwarp();
-            const uint32_t slab = stg_u32 + sbuf * 4096 + lane * 128;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              st_shared_v4(slab + ((uint32_t(q) ^ xr) << 4), pack_bf16(v[q * 8 + 0], v[q * 8 + 1]), pack_bf16(v[q * 8 + 2], v[q * 8 + 3]),
-                           pack_bf16(v[q * 8 + 4], v[q * 8 + 5]), pack_bf16(v[q * 8 + 6], v[q * 8 + 7]));
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              if (p.tp_mode & TP_RS) {
-                // rows of shard d go to rank d's staging buffer, slot `rank`: one 32-row x 128-byte slab per copy, so the
-                // bytes cross NVLink in whole lines (tile rows never straddle two shards: shards are multiples of 128 rows)
-                const int d = slab_row0 / p.rs_rows_per_shard;
-                tma_store_3d(&tma_peers.m[d], stg_u32 + sbuf * 4096, col0,
-                             p.rs_rank * p.rs_rows_per_shard + (slab_row0 - d * p.rs_rows_per_shard), 0);
-              } else {
-                tma_store_3d(&tma_c, stg_u32 + sbuf * 4096, col0, slab_row0, 0);
-              }
-              tma_store_commit();
-            }
-            sbuf ^= (L::STG_BUFS - 1);
-          }
-        } else {
-          const int cz = p.group_mode == 2 ? it.expert : 0;
-#pragma unroll 1
-          for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
-            const int col0 = n0 + c * 32;
-            if (col0 >= p.N) break;
-            uint32_t r[32];
-            tmem_ld_32x32(taddr0 + c * 32, r);
-            tmem_ld_wait();
-            if (!slab_live) continue;
-            if (lane == 0) tma_store_wait_read<L::STG_BUFS - 1>();
-            __syncwarp();
-            const uint32_t slab = stg_u32 + sbuf * 4096 + lane * 128;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              st_shared_v4(slab + ((uint32_t(q) ^ xr) << 4), __float_as_uint(__uint_as_float(r[q * 4]) * p.alpha),
-                           __float_as_uint(__uint_as_float(r[q * 4 + 1]) * p.alpha), __float_as_uint(__uint_as_float(r[q * 4 + 2]) * p.alpha),
-                           __float_as_uint(__uint_as_float(r[q * 4 + 3]) * p.alpha));
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              if (p.out_mode == 2) tma_reduce_add_3d(&tma_c, stg_u32 + sbuf * 4096, col0, slab_row0, cz);
-              else tma_store_3d(&tma_c, stg_u32 + sbuf * 4096, col0, slab_row0, cz);
-              tma_store_commit();
-            }
-            sbuf ^= (L::STG_BUFS - 1);
-          }
-        }
+        staged_epilogue<BN, L::STG_BUFS>(p, tma_c, tma_peers, taddr0, n0, m0 + quad * 32, half, lane, stg_u32, sbuf,
+                                         p.group_mode == 2 ? it.expert : 0);
         tc_fence_before();
         mbar_arrive(bar_tempty + abuf * 8);
         abuf ^= 1;
@@ -696,6 +707,181 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
 }
 
+// The same product on CTA pairs: a cluster of two CTAs owns a 256 x 256 tile, each holds 128 rows of A, 128 of the 256 columns of B and its
+// 128 rows of the accumulator, and one thread of the first CTA issues tcgen05.mma.cta_group::2 over both.  A k-block brings 32 KB
+// into each SM instead of the 48 KB of a 128 x 256 tile, so that six of them fit in flight where four did: with short K (tiles of
+// eight k-blocks) the single-CTA form waits for its loads behind the stores of the tile before.  (Measured there: without its
+// stores 65536 x 2816 x 512 took 129 us instead of 166, with three stages and two staging slabs per warp 186.)
+//   us, single-CTA -> pair: 65536 x 2816 x 512 nt 169 -> 152, 65536 x 512 x 1408 82 -> 72, 9472 x 32000 x 512 279 -> 250, 65536 x 512 x 2816 nn
+//   143 -> 125, weight gradients 2816 x 512 x 65536 152 -> 129, 32000 x 512 x 9472 270 -> 227, 28672 x 4096 x 4096 893 -> 716, 5000 x 28672 x
+//   4096 nt 876 -> 798 (1472 TFLOP/s).  Five stages with two slabs per warp are 2 - 5 % slower than six with one.
+struct PairSmem {
+  static constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = 2 * A_BYTES;
+  static constexpr int STG_BUFS = 1, STG_BYTES = EPI_WARPS * STG_BUFS * 4096;
+  static constexpr int STAGES = 6;
+  static constexpr int STG_OFF = STAGES * STAGE_BYTES, BAR_OFF = STG_OFF + STG_BYTES;
+  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+};
+
+template <bool A_MN, bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const __grid_constant__ CUtensorMap tma_c,
+                 const __grid_constant__ PeerMaps tma_peers, const GemmParams p) {
+  using L = PairSmem;
+  constexpr int BN = 256, ST = L::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t smem_base = smem_u32(smem);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
+  const uint32_t bar_full = smem_u32(bars);          // first CTA's: both CTAs' tiles of a k-block have landed
+  const uint32_t bar_empty = bar_full + ST * 8;      // each CTA's: the instruction has read them
+  const uint32_t bar_tfull = bar_empty + ST * 8;     // each CTA's: accumulator ready
+  const uint32_t bar_tempty = bar_tfull + 2 * 8;     // first CTA's: drained by the epilogue warps of both
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * ST + 4);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int npairs = int(gridDim.x) >> 1, pair = int(blockIdx.x) >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(bar_full + s * 8, 1);
+      mbar_init(bar_empty + s * 8, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(bar_tfull + b * 8, 1);
+      mbar_init(bar_tempty + b * 8, 2 * EPI_WARPS);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tma_a);
+    tma_prefetch_desc(&tma_b);
+    tma_prefetch_desc(&tma_c);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(smem_u32(tmem_slot), 2 * BN);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();      // the other CTA's barriers are set up
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  tfb::pdl_sync();
+
+  const int total_kb = (p.K + BK - 1) / BK;
+  const int num_work = p.tiles_m * p.tiles_n * p.splits;
+  // work item -> tile (grouped raster, see decode_work) and k-blocks
+  auto decode = [&](int w, int& m0, int& n0, int& kb0, int& kb1) {
+    const int tile = w / p.splits, split = w - tile * p.splits;
+    const int per_group = p.raster_gn * p.tiles_m;
+    const int grp = tile / per_group, within = tile - grp * per_group;
+    const int gn = min(p.raster_gn, p.tiles_n - grp * p.raster_gn);
+    const int mi = within / gn;
+    m0 = mi * (2 * BM) + int(rank) * BM;
+    n0 = (grp * p.raster_gn + (within - mi * gn)) * BN;
+    kb0 = split * p.kb_per_split;
+    kb1 = min(total_kb, kb0 + p.kb_per_split);
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const uint32_t full0 = map_cta(bar_full, 0);
+      int stage = 0;
+      uint32_t phase = 1;
+      bool ok = true;
+      for (int w = pair; w < num_work && ok; w += npairs) {
+        int m0, n0, kb0, kb1;
+        decode(w, m0, n0, kb0, kb1);
+        const int nb = n0 + int(rank) * BM;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait(bar_empty + stage * 8, phase, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(bar_full + stage * 8, 2 * L::STAGE_BYTES);
+          const uint32_t fb = full0 + stage * 8, sa = smem_base + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES;
+          const int k0 = kb * BK;
+          if constexpr (!A_MN) {
+            tma_load_2d_pair(sa, &tma_a, fb, k0, m0);
+          } else {
+            tma_load_2d_pair(sa, &tma_a, fb, m0, k0);
+            tma_load_2d_pair(sa + 8192, &tma_a, fb, m0 + 64, k0);
+          }
+          if constexpr (!B_MN) {
+            tma_load_2d_pair(sb, &tma_b, fb, k0, nb);
+          } else {
+            tma_load_2d_pair(sb, &tma_b, fb, nb, k0);
+            tma_load_2d_pair(sb + 8192, &tma_b, fb, nb + 64, k0);
+          }
+          if (++stage == ST) { stage = 0; phase ^= 1; }
+        }
+      }
+      if (!ok) {   // copies in flight land before shared memory goes away
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) {}
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = umma_idesc(FMT_BF16, FMT_BF16, A_MN, B_MN, 2 * BM, BN);
+      const uint32_t adesc0 = umma_desc_lo(smem_base, A_MN ? 8192 : 16), bdesc0 = umma_desc_lo(smem_base + L::A_BYTES, B_MN ? 8192 : 16);
+      constexpr uint32_t ASTEP = A_MN ? 2048 >> 4 : 32 >> 4, BSTEP = B_MN ? 2048 >> 4 : 32 >> 4;
+      int stage = 0, abuf = 0;
+      uint32_t phase = 0, aphase = 1;
+      bool ok = true;
+      for (int w = pair; w < num_work && ok; w += npairs) {
+        int n_kb = total_kb;
+        if (p.splits > 1) {
+          int m0, n0, kb0, kb1;
+          decode(w, m0, n0, kb0, kb1);
+          n_kb = kb1 - kb0;
+        }
+        if (!mbar_wait(bar_tempty + abuf * 8, aphase, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
+        tc_fence_after();
+        const uint32_t tmem_d = tmem_base + abuf * BN;
+        for (int kb = 0; kb < n_kb; ++kb) {
+          if (!mbar_wait(bar_full + stage * 8, phase, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t at = uint32_t(stage) * (L::STAGE_BYTES >> 4);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_f16_ss_pair(tmem_d, adesc0 + at + k * ASTEP, bdesc0 + at + k * BSTEP, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(bar_empty + stage * 8);
+          if (++stage == ST) { stage = 0; phase ^= 1; }
+        }
+        if (!ok) break;
+        umma_commit_pair(bar_tfull + abuf * 8);
+        abuf ^= 1;
+        if (abuf == 0) aphase ^= 1;
+      }
+    }
+  } else {
+    const int quad = warp & 3, ew = warp - 2, half = ew >> 2;
+    const uint32_t stg_u32 = smem_base + L::STG_OFF + ew * (L::STG_BUFS * 4096), tempty0 = map_cta(bar_tempty, 0);
+    int sbuf = 0, abuf = 0;
+    uint32_t aphase = 0;
+    for (int w = pair; w < num_work; w += npairs) {
+      int m0, n0, kb0, kb1;
+      decode(w, m0, n0, kb0, kb1);
+      if (!mbar_wait_warp(bar_tfull + abuf * 8, aphase, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) break;
+      tc_fence_after();
+      staged_epilogue<BN, L::STG_BUFS>(p, tma_c, tma_peers, tmem_base + abuf * BN + (uint32_t(quad * 32) << 16), n0, m0 + quad * 32, half, lane,
+                                       stg_u32, sbuf, 0);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(tempty0 + abuf * 8);
+      abuf ^= 1;
+      if (abuf == 0) aphase ^= 1;
+    }
+    if (lane == 0) tma_store_wait<0>();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();      // neither CTA leaves while the other may read its shared memory or arrive on its barriers
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 2 * BN);
+  }
+}
+
 // -------------------------------------------------------------------------------------------------
 // host launcher
 // -------------------------------------------------------------------------------------------------
@@ -707,6 +893,17 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   auto kern = gemm_bf16_kernel<A_MN, B_MN, BN>;
   if (int e = ensure_dyn_smem(once, kern, L::TOTAL)) return e;
   tfb::launch_k(kern, grid, GEMM_THREADS, L::TOTAL, st, ta, tb, tc, tpeers, p);
+  return int(cudaGetLastError());
+}
+
+template <bool A_MN, bool B_MN>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int pairs, cudaStream_t st) {
+  using L = PairSmem;
+  static DeviceOnce once;
+  static const PeerMaps none = {};
+  auto kern = gemm_pair_kernel<A_MN, B_MN>;
+  if (int e = ensure_dyn_smem(once, kern, L::TOTAL)) return e;
+  tfb::launch_k(kern, 2 * pairs, GEMM_THREADS, L::TOTAL, st, ta, tb, tc, none, p);
   return int(cudaGetLastError());
 }
 
@@ -867,11 +1064,52 @@ static int gemm_impl(const void* A, long long lda, int a_mn, const void* B, long
     static const int narrow_env = [] { const char* e = getenv("TFB_GEMM_NARROW"); return e ? atoi(e) : 1; }();
     if (narrow_env && BN == 256 && gmode != 2 && out_mode != 2 && t256 < sms && t128 > t256 && t128 <= sms) BN = 128;
   }
+  static const int raster_env = [] { const char* e = getenv("TFB_GEMM_RASTER"); return e ? atoi(e) : -1; }();
+  // Tiles of 256 columns of a plain product with more than one tile row run on CTA pairs.
+  const bool want_pair = BN == 256 && gmode == 0 && !tp && M > BM && sms >= 2;
   CUtensorMap ta, tb;
   int rc;
   if (!a_mn) rc = make_tmap_2d(&ta, A, 2, K, M, lda * 2, BK, BM);
   else rc = make_tmap_2d(&ta, A, 2, M, K, lda * 2, 64, BK);
   if (rc) return rc;
+  if (want_pair) {
+    CUtensorMap tb2, tc2;
+    const int esz = out_mode == 0 ? 2 : 4;
+    rc = !b_mn ? make_tmap_2d(&tb2, B, 2, K, N, ldb * 2, BK, BM) : make_tmap_2d(&tb2, B, 2, N, K, ldb * 2, 64, BK);
+    if (rc) return rc;
+    if ((reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc * esz) % 16 == 0 &&
+        make_tmap_3d(&tc2, C, esz, N, M, 1, ldc * esz, (unsigned long long)ldc * esz * M, 128 / esz, 32, 1) == 0) {
+      GemmParams p = {};
+      p.M = M; p.N = N; p.K = K;
+      p.C = C; p.ldc = ldc;
+      p.bias = static_cast<const __nv_bfloat16*>(bias);
+      p.residual = static_cast<const __nv_bfloat16*>(residual);
+      p.ldr = ldr;
+      p.alpha = alpha; p.act = act; p.out_mode = out_mode;
+      p.tiles_m = (M + 2 * BM - 1) / (2 * BM);
+      p.tiles_n = (N + BN - 1) / BN;
+      p.num_experts = 1;
+      p.rs_world = 1;
+      p.c_tma = 1;
+      p.status = status;
+      // tile order as below, in groups of eight tile columns where B is wide
+      p.raster_gn = raster_env != 0 && p.tiles_n > 12 && p.tiles_m >= 2 ? (raster_env > 0 ? raster_env : 8) : p.tiles_n;
+      const int total_kb = (K + BK - 1) / BK, tiles = p.tiles_m * p.tiles_n, pairs = sms / 2;
+      int splits = 1;
+      if (force_splits > 0 && out_mode == 2) splits = force_splits;
+      else if (out_mode == 2 && tiles < pairs) splits = max(1, min(pairs / tiles, (total_kb + 7) / 8));   // one wave, at least 8 k-blocks per split
+      p.kb_per_split = (total_kb + splits - 1) / splits;
+      p.splits = (total_kb + p.kb_per_split - 1) / p.kb_per_split;
+      const int grid = int(min((long long)tiles * p.splits, (long long)pairs));
+      cudaStream_t st = static_cast<cudaStream_t>(stream);
+      switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
+        case 0: return launch_pair<false, false>(ta, tb2, tc2, p, grid, st);
+        case 1: return launch_pair<false, true>(ta, tb2, tc2, p, grid, st);
+        case 2: return launch_pair<true, false>(ta, tb2, tc2, p, grid, st);
+        default: return launch_pair<true, true>(ta, tb2, tc2, p, grid, st);
+      }
+    }
+  }
   const int EB = gmode == 1 ? E : 1;
   const unsigned long long bes = gmode == 1 ? (unsigned long long)grp->b_expert_stride * 2 : (unsigned long long)ldb * 2 * (b_mn ? K : N);
   if (!b_mn) rc = make_tmap_3d(&tb, B, 2, K, N, EB, ldb * 2, bes, BK, BN, 1);
@@ -965,7 +1203,6 @@ static int gemm_impl(const void* A, long long lda, int a_mn, const void* B, long
   {
     // tile order (see decode_work): row-major unless B is wide; the activation gather / reduce-scatter orders follow the
     // row blocks and stay row-major; a gathered K-major weight is always walked in column groups
-    static const int raster_env = [] { const char* e = getenv("TFB_GEMM_RASTER"); return e ? atoi(e) : -1; }();
     const int wide = (BN == 256) ? 8 : 16;
     p.raster_gn = p.tiles_n;
     if (gmode != 2 && !(p.tp_mode & (TP_AG | TP_RS))) {

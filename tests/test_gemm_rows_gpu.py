@@ -56,6 +56,23 @@ def test_few_rows_epilogue(M, N, K):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("fmt,group", [("int8", 32), ("int8", 64), ("mxfp8", 32), ("int4", 32), ("fp4", 32), ("ternary", 64)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (5, 1000, 776), (16, 4096, 4096), (17, 1536, 512), (32, 512, 14336)])
+def test_packed_rows(M, N, K, fmt, group):
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
+    bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+    pw = wq.pack_weight(w, fmt, group)
+    # the oracle multiplies unrounded code * scale; the kernel's weights are that in bf16, 2^-9 each
+    want = x.double() @ wq.dequant(pw).double().t() + bias.double() + res.double()
+    a = wq.gemm_wq(x, pw, bias, residual=res)
+    b = wq.gemm_wq(x, pw, bias, residual=res, w_static=True)
+    out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    c = wq.gemm_wq(x, pw, bias, residual=res, out=out)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert _rel(a, want) < 6e-3 and torch.equal(a, b) and torch.equal(a, c) and c is out
+
+
 def test_rows_under_capture_and_on_streams():
     """Captured products share one workspace, eager ones have one per stream; more streams than workspaces take the general path."""
     x, w = torch.randn(8, 4096, device="cuda").bfloat16(), (torch.randn(6144, 4096, device="cuda") / 64).bfloat16()

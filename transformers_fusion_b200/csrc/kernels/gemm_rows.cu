@@ -1,5 +1,5 @@
-// Products of few rows: out[M, N] = act(alpha * x[M, K] . W[N, K]^T + bias) + residual for M <= 128, W in bf16 or in the packed formats of
-// wq_decode.cuh.  Such a product streams the weights once; everything here serves that stream.
+// Products of few rows: out[M, N] = act(alpha * x[M, K] . W[N, K]^T + bias) + residual for M <= 128 with W in bf16, M <= 32 with W in the packed
+// formats of wq_decode.cuh.  Such a product streams the weights once; everything here serves that stream.
 //
 //   - Operands swapped: the 128 weight rows of a tile are the M side of tcgen05.mma and the batch (padded to 16, 32, 64 or 128) its
 //     N side, so shared memory and tensor time go to weights and not to padding, and the ring holds 110 - 190 KB of weights per SM.
@@ -32,8 +32,8 @@ struct RowsPlan {
   static constexpr int X_BYTES = MP * RW_BK * 2;
   static constexpr int STAGE = X_BYTES + (QUANT ? 0 : RW_W_BYTES);
   // tensor memory: two accumulators of MP columns, then 32 columns of converted weights per stage
-  static constexpr int STAGES = QUANT ? (MP == 128 ? 8 : 12) : (MP == 16 ? 12 : MP == 32 ? 11 : MP == 64 ? 9 : 6);
-  static constexpr int RAW_STAGES = QUANT ? (MP == 128 ? 10 : 12) : 0;
+  static constexpr int STAGES = QUANT ? 12 : (MP == 16 ? 12 : MP == 32 ? 11 : MP == 64 ? 9 : 6);
+  static constexpr int RAW_STAGES = QUANT ? 12 : 0;
   static constexpr int TMEM_COLS = QUANT ? 512 : 2 * MP;
   static constexpr int RAW_OFF = STAGES * STAGE;
   static constexpr int BAR_OFF = RAW_OFF + RAW_STAGES * RW_RAW;
@@ -418,8 +418,9 @@ template <int FMT>
 static int launch_rows_m(int M, const CUtensorMap& tx, const CUtensorMap& tw, const RowsParams& p, int grid, cudaStream_t st) {
   if (M <= 16) return launch_rows<FMT, 16>(tx, tw, p, grid, st);
   if (M <= 32) return launch_rows<FMT, 32>(tx, tw, p, grid, st);
-  if (M <= 64) return launch_rows<FMT, 64>(tx, tw, p, grid, st);
-  return launch_rows<FMT, 128>(tx, tw, p, grid, st);
+  if constexpr (FMT >= 0) return TFB_NOT_TAKEN;      // packed weights: the converters set the pace, more rows only lengthen the drain
+  else if (M <= 64) return launch_rows<FMT, 64>(tx, tw, p, grid, st);
+  else return launch_rows<FMT, 128>(tx, tw, p, grid, st);
 }
 
 int gemm_rows(const void* x, long long ldx, const void* W, long long ldw, const void* codes, const void* scales, int fmt, int group, void* C,

@@ -259,8 +259,7 @@ class InferenceEngine:
         pw = self.packed.get(f"layers.{li}.{name}")
         if pw is None:
             return F.linear(x, w.data, bias, residual)
-        y = self._wq.gemm_wq(x, pw, bias)
-        return y if residual is None else y + residual
+        return self._wq.gemm_wq(x, pw, bias, residual=residual, w_static=True)
 
     def _ffn(self, li, w, f, base):
         """Feed-forward half of a block on normed rows ``f`` with residual ``base``: the dense GLU / MLP, or - for a

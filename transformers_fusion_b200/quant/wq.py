@@ -167,16 +167,47 @@ def dequant_bf16(pw: PackedWeight) -> torch.Tensor:
 _SPLIT_WS = {}
 
 
+ROWS_M = 32       # up to here (decode) the streaming form of gemm_rows.cu: one launch with bias and residual inside.  Measured, us, int8 codes, against
+                  # the split form with its finalize: 28672 x 4096 at 1 / 32 rows 49 / 51 against 57 / 62, 4096 x 14336 28.6 / 30.6 against 29.9 /
+                  # 33.3, 6144 x 4096 16.2 / 17.5 against 16.4 / 19.4; at 64 rows 4096 x 4096 20.3 against 17.3
+
+
 def gemm_wq(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor] = None, splits: int = 0,
-            out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y [M, N] = x [M, K] @ dequant(pw)^T (+ bias).  bf16 in / out.  M <= 16 (decode): fused-dequant kernel with the deep
-    ring and split-K; M < 2048: fused-dequant kernel with 128-row tiles; larger: bf16 image in scratch + bf16 GEMM.
-    ``out`` [M, N] bf16: where the result goes (e.g. the staging buffer of a collective)."""
-    y = _gemm_wq(x, pw, bias, splits, out)
+            out: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None, w_static: bool = False) -> torch.Tensor:
+    """y [M, N] = x [M, K] @ dequant(pw)^T (+ bias) (+ residual).  bf16 in / out.  M <= 32 (decode): streaming kernel; M < 2048:
+    fused-dequant kernel with 128-row tiles; larger: bf16 image in scratch + bf16 GEMM.
+    ``out`` [M, N] bf16: where the result goes (e.g. the staging buffer of a collective).  ``w_static``: the kernel launched just before does not
+    write the packed weight (it may then be fetched ahead of that kernel's end)."""
+    y = None
+    if x.is_cuda and x.shape[0] <= ROWS_M and splits == 0:
+        y = _gemm_rows(x, pw, bias, residual, out, w_static)
+    if y is None:
+        y = _gemm_wq(x, pw, bias, splits, out)
+        if residual is not None:
+            y = y + residual
     if out is not None and y is not out:
         out.copy_(y)
         return out
     return y
+
+
+def _gemm_rows(x, pw, bias, residual, dst, w_static):
+    """The streaming form; None where its operands' layout does not fit it."""
+    M, K = x.shape
+    if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or M < 1:
+        return None
+    if residual is not None and (residual.dtype != torch.bfloat16 or residual.stride(-1) != 1):
+        return None
+    if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != pw.N):
+        return None
+    out = dst if dst is not None and dst.dtype == torch.bfloat16 and dst.stride(-1) == 1 else torch.empty((M, pw.N), dtype=x.dtype, device=x.device)
+    rc = _lib.lib().tfb_gemm_rows_wq(x.data_ptr(), x.stride(0), pw.codes.data_ptr(), pw.scales.data_ptr(), pw.fmt, pw.group, out.data_ptr(),
+                                     out.stride(0), M, pw.N, K, pw.Kp, ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
+                                     int(w_static), _lib.status_word(x.device).data_ptr(), stream())
+    if rc == -1:                     # not taken
+        return None
+    check(rc, "gemm_rows_wq")
+    return out
 
 
 def _gemm_wq(x, pw, bias, splits, dst):

@@ -1,19 +1,23 @@
 // Flash attention backward for sm_100a: exact gradients, probabilities recomputed from the saved
-// log-sum-exp (nothing of size S x S is ever stored).  Two tcgen05 kernels, no atomics; each runs two compute
-// warpgroups that work on the two halves of a 128 x 128 score block, so that the tensor core computes one half while
-// the other half's exponentials and products are in flight, and every scheduler has two compute warps to issue from.
+// log-sum-exp (nothing of size S x S is ever stored).  Two tcgen05 kernels, no atomics.
 //
 //   attn_bwd_dkdv : one CTA per (batch, kv head, 128-key block); loops over the query heads of the group and the
-//                   query blocks that see these keys.  Per step and per half w (64 queries):
-//                     S^T_w = K Q_w^T, dP^T_w = V dO_w^T                       (shared-memory operands, 128 x 64)
-//                     P^T_w = exp(S^T_w - lse), dS^T_w = P^T_w * (dP^T_w - delta)    (one key row per thread)
-//                     dV += P^T_w dO_w, dK += dS^T_w Q_w     (A operand from TMEM, B MN-major), accumulated in TMEM
-//   attn_bwd_dq   : one CTA per (batch, query head, 128-query block); loops over key blocks, half w = 64 keys:
-//                     S_w = Q K_w^T, dP_w = dO V_w^T, dS_w = P_w * (dP_w - delta), dQ += dS_w K_w
+//                   half blocks (64 queries) that see these keys.  Per half block h:
+//                     S^T_h = K Q_h^T, dP^T_h = V dO_h^T                       (shared-memory operands, 128 x 64)
+//                     P^T_h = exp(S^T_h - lse), dS^T_h = P^T_h * (dP^T_h - delta)    (one key row per thread)
+//                     dV += P^T_h dO_h, dK += dS^T_h Q_h     (A operand from TMEM, B MN-major), accumulated in TMEM
+//   attn_bwd_dq   : one CTA per (batch, query head, 128-query block); loops over half blocks of 64 keys:
+//                     S_h = Q K_h^T, dP_h = dO V_h^T, dS_h = P_h * (dP_h - delta), dQ += dS_h K_h
 //   attn_delta    : delta[b,h,s] = sum_d dO * O
+// Two compute warpgroups take the half blocks in turn.  Scores live in a ring of tensor-memory slots (128 columns: S / P in the
+// first 64, dP / dS in the others): with three slots the scores of the next two half blocks are there when a warpgroup is done, and the
+// round trip - P and dS announced, products issued, next scores computed - is off its path; the tensor core runs products
+// and scores in issue order, so a slot may be refilled right behind the products that read it.  dK / dV at heads of 128 fill
+// 256 columns themselves and leave room for two slots.  The operand tiles of the loop come in half blocks too, through a ring
+// that runs ahead of the slots.
+//   Before (two slots, one per warpgroup; whole blocks through two stages): 22 - 27 % of the exponential rate at heads of 64, a warpgroup
+// idle for a tensor-core round trip per half block.
 // The softmax scale multiplies dK and dQ once, when they are written out.
-// Tensor memory: half w owns columns [128 w, 128 w + 64) for S / P and [128 w + 64, 128 w + 128) for dP / dS; the
-// accumulators start at column 256.
 //
 // The reference's memory-efficient attention backward is approximate
 // (src/trainer/zero_optimizer_mem.cpp:496-574); its autograd attention op (src/model/autograd_functions.cpp:17-226)
@@ -25,7 +29,7 @@ namespace tfb {
 
 constexpr int AB_THREADS = 320;   // warp 0 TMA, warp 1 MMA, warps 2-5 half 0, warps 6-9 half 1
 constexpr int AB_BOX = 128 * 64 * 2;
-constexpr int AB_HALF = 64 * 128;  // byte offset of row 64 inside a 128-row, 128-byte-pitch box
+constexpr int AB_HBOX = 64 * 64 * 2;   // 64 columns of a half block (64 rows)
 constexpr float LOG2E = 1.4426950408889634f;
 
 __device__ __forceinline__ float bwd_exp2(float x) {
@@ -47,15 +51,18 @@ struct AttnBwdParams {
   int* status;
 };
 
-template <int D>
+template <int D, bool DKDV>
 struct BwdSmem {
   static constexpr int NB = D / 64;
-  static constexpr int TILE = NB * AB_BOX;
-  static constexpr int RES_OFF = 0;              // two resident tiles
-  static constexpr int RING_OFF = 2 * TILE;      // 2 stages x 2 tiles
-  static constexpr int STAT_OFF = RING_OFF + 4 * TILE;  // [2 stages][2 halves][64 lse | 64 delta] floats
-  static constexpr int BAR_OFF = STAT_OFF + 2 * 2 * 128 * 4;
+  static constexpr int TILE = NB * AB_BOX, HALF = NB * AB_HBOX;     // a resident tile, a half block
+  static constexpr int SLOTS = DKDV && D == 128 ? 2 : 3;            // tensor-memory slots
+  static constexpr int ACC_COL = SLOTS * 128;
+  static constexpr int STAGES = D == 64 ? 6 : DKDV ? 4 : 5;         // half blocks (two operands each) in flight
+  static constexpr int RING_OFF = 2 * TILE;                         // behind two resident tiles
+  static constexpr int STAT_OFF = RING_OFF + STAGES * 2 * HALF;     // [2 warpgroups][2 turns][64 -lse | 64 -delta] floats
+  static constexpr int BAR_OFF = STAT_OFF + (DKDV ? 2 * 2 * 128 * 4 : 0);
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static_assert(ACC_COL + (DKDV ? 2 : 1) * D <= 512 && TOTAL <= 232448, "tensor and shared memory");
 };
 
 // 16 output rows x 128 bf16 columns of an accumulator, written by one thread (its row)
@@ -80,8 +87,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
                      const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                      const AttnBwdParams p) {
   tfb::pdl_sync();
-  using L = BwdSmem<D>;
-  constexpr int NB = L::NB;
+  using L = BwdSmem<D, true>;
+  constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
@@ -89,37 +96,37 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
   float* stats = reinterpret_cast<float*>(smem + L::STAT_OFF);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   const uint32_t bar_kv = smem_u32(bars);
-  const uint32_t bar_full = bar_kv + 8;        // [2] Q / dO stage loaded
-  const uint32_t bar_empty = bar_full + 16;    // [2] stage consumed
-  const uint32_t bar_s = bar_empty + 16;       // [2] S^T_w and dP^T_w ready
-  const uint32_t bar_pds = bar_s + 16;         // [2] P^T_w and dS^T_w written (128 arrivals)
-  const uint32_t bar_stat = bar_pds + 16;      // [2] per-step statistics of half w staged (128 arrivals)
-  const uint32_t bar_acc = bar_stat + 16;      // all accumulation done
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  const uint32_t bar_full = bar_kv + 8;             // [ST] Q / dO half block loaded
+  const uint32_t bar_empty = bar_full + ST * 8;     // [ST] consumed
+  const uint32_t bar_s = bar_empty + ST * 8;        // [NS] S^T and dP^T ready
+  const uint32_t bar_pds = bar_s + NS * 8;          // [NS] P^T and dS^T written (128 arrivals)
+  const uint32_t bar_stat = bar_pds + NS * 8;       // [2] statistics of a warpgroup's half block staged (128 arrivals)
+  const uint32_t bar_acc = bar_stat + 16;           // all accumulation done
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 + 2 * ST + 2 * NS + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nqb = (p.S + 127) / 128;
-  const int nkb = nqb;
   // causal: the first key blocks see the most queries; all of them start first, so that no long block is left for the end (4096 tokens,
   // 32 / 8 heads of 128, both gradient kernels: 874 -> 703 us)
   const int jb = int(blockIdx.x) / (p.Hkv * p.B);
   const int rem = int(blockIdx.x) % (p.Hkv * p.B);
   const int hk = rem % p.Hkv, b = rem / p.Hkv;
   const int G = p.Hq / p.Hkv;
-  const int i0 = p.causal ? jb : 0;
-  const int n_i = nqb - i0;
-  const int n_it = G * n_i;
+  const int i0 = p.causal ? 2 * jb : 0;             // first half block of queries
+  const int n_i = (p.S + 63) / 64 - i0;
+  const int n = G * n_i;
 
   if (threadIdx.x == 0) {
     mbar_init(bar_kv, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < ST; ++s) {
       mbar_init(bar_full + s * 8, 1);
       mbar_init(bar_empty + s * 8, 1);
+    }
+    for (int s = 0; s < NS; ++s) {
       mbar_init(bar_s + s * 8, 1);
       mbar_init(bar_pds + s * 8, 128);
-      mbar_init(bar_stat + s * 8, 128);
     }
+    for (int s = 0; s < 2; ++s) mbar_init(bar_stat + s * 8, 128);
     mbar_init(bar_acc, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -132,7 +139,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tDV = tmem_base + 256, tDK = tmem_base + 256 + D;
+  const uint32_t tDV = tmem_base + L::ACC_COL, tDK = tDV + D;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -142,18 +149,20 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
         tma_load_3d(sK + c * AB_BOX, &tk, bar_kv, p.k_col0 + hk * D + c * 64, jb * 128, b);
         tma_load_3d(sV + c * AB_BOX, &tv, bar_kv, p.v_col0 + hk * D + c * 64, jb * 128, b);
       }
-      for (int it = 0; it < n_it; ++it) {
-        const int st = it & 1;
-        const int h = hk * G + it / n_i, i = i0 + it % n_i;
-        if (!mbar_wait(bar_empty + st * 8, ((it >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+      int st = 0, h = hk * G, i = i0;
+      uint32_t ph = 1;
+      for (int hs = 0; hs < n; ++hs) {
+        if (!mbar_wait(bar_empty + st * 8, ph, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
         const uint32_t fb = bar_full + st * 8;
-        mbar_expect_tx(fb, 2 * L::TILE);
-        const uint32_t sQ = sbase + L::RING_OFF + st * 2 * L::TILE, sDO = sQ + L::TILE;
+        mbar_expect_tx(fb, 2 * L::HALF);
+        const uint32_t sQ = sbase + L::RING_OFF + st * 2 * L::HALF, sDO = sQ + L::HALF;
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
-          tma_load_3d(sQ + c * AB_BOX, &tq, fb, p.q_col0 + h * D + c * 64, i * 128, b);
-          tma_load_3d(sDO + c * AB_BOX, &tdo, fb, h * D + c * 64, i * 128, b);
+          tma_load_3d(sQ + c * AB_HBOX, &tq, fb, p.q_col0 + h * D + c * 64, i * 64, b);
+          tma_load_3d(sDO + c * AB_HBOX, &tdo, fb, h * D + c * 64, i * 64, b);
         }
+        if (++i == i0 + n_i) { i = i0; ++h; }
+        if (++st == ST) { st = 0; ph ^= 1; }
       }
       if (*abort_flag) {
         const uint64_t t0 = globaltimer_ns();
@@ -164,51 +173,46 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc(FMT_BF16, FMT_BF16, false, false, 128, 64);
       constexpr uint32_t idesc_acc = umma_idesc(FMT_BF16, FMT_BF16, false, true, 128, D);
-      // scores of half w for the step whose Q / dO tiles sit in stage st
-      auto issue_scores = [&](int w, int st) {
-        const uint32_t sQ = sbase + L::RING_OFF + st * 2 * L::TILE + w * AB_HALF, sDO = sQ + L::TILE;
-        const uint32_t tS = tmem_base + w * 128, tDP = tS + 64;
+      const uint32_t dK = umma_desc_lo(sK, 16), dV = umma_desc_lo(sV, 16);
+      // scores of the half block in stage st into slot sl
+      auto issue_scores = [&](int sl, int st) {
+        const uint32_t sQ = sbase + L::RING_OFF + st * 2 * L::HALF;
+        const uint32_t dQ = umma_desc_lo(sQ, 16), dDO = umma_desc_lo(sQ + L::HALF, 16);
+        const uint32_t tS = tmem_base + sl * 128, tDP = tS + 64;
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * AB_BOX + (k & 3) * 32;
-          umma_f16_ss(tS, umma_smem_desc(sK + off, 16, 1024), umma_smem_desc(sQ + off, 16, 1024), idesc_s, k > 0);
-        }
+        for (int k = 0; k < D / 16; ++k)
+          umma_f16_ss_lo(tS, dK + (((k >> 2) * AB_BOX + (k & 3) * 32) >> 4), dQ + (((k >> 2) * AB_HBOX + (k & 3) * 32) >> 4), idesc_s, k > 0);
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * AB_BOX + (k & 3) * 32;
-          umma_f16_ss(tDP, umma_smem_desc(sV + off, 16, 1024), umma_smem_desc(sDO + off, 16, 1024), idesc_s, k > 0);
-        }
-        umma_commit(bar_s + w * 8);
+        for (int k = 0; k < D / 16; ++k)
+          umma_f16_ss_lo(tDP, dV + (((k >> 2) * AB_BOX + (k & 3) * 32) >> 4), dDO + (((k >> 2) * AB_HBOX + (k & 3) * 32) >> 4), idesc_s, k > 0);
+        umma_commit(bar_s + sl * 8);
       };
-      bool ok = mbar_wait(bar_kv, 0, abort_flag, p.status, ST_TIMEOUT_FULL) &&
-                (n_it == 0 || mbar_wait(bar_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL));
-      if (ok && n_it > 0) {
+      bool ok = mbar_wait(bar_kv, 0, abort_flag, p.status, ST_TIMEOUT_FULL);
+      int nst = 0;                      // stage and turn of the next scores
+      uint32_t nph = 0;
+      auto next_scores = [&](int sl) {
+        if (!mbar_wait(bar_full + nst * 8, nph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; return; }
         tc_fence_after();
-        issue_scores(0, 0);
-        issue_scores(1, 0);
-      }
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int st = it & 1;
-        if (it + 1 < n_it) {
-          if (!mbar_wait(bar_full + ((it + 1) & 1) * 8, ((it + 1) >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) break;
-          tc_fence_after();
-        }
+        issue_scores(sl, nst);
+        if (++nst == ST) { nst = 0; nph ^= 1; }
+      };
+      for (int hs = 0; hs < NS && hs < n && ok; ++hs) next_scores(hs);
+      int sl = 0, st = 0;
+      uint32_t sph = 0;
+      for (int hs = 0; hs < n && ok; ++hs) {
+        if (!mbar_wait(bar_pds + sl * 8, sph, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
+        tc_fence_after();
+        const uint32_t sQ = sbase + L::RING_OFF + st * 2 * L::HALF;
+        const uint32_t dQ = umma_desc_lo(sQ, AB_HBOX), dDO = umma_desc_lo(sQ + L::HALF, AB_HBOX);
+        const uint32_t tS = tmem_base + sl * 128, tDP = tS + 64;
 #pragma unroll
-        for (int w = 0; w < 2; ++w) {
-          if (!ok) continue;
-          if (!mbar_wait(bar_pds + w * 8, it & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; continue; }
-          tc_fence_after();
-          const uint32_t sQ = sbase + L::RING_OFF + st * 2 * L::TILE + w * AB_HALF, sDO = sQ + L::TILE;
-          const uint32_t tS = tmem_base + w * 128, tDP = tS + 64;
+        for (int k = 0; k < 4; ++k) umma_f16_ts_lo(tDV, tS + k * 8, dDO + k * (2048 >> 4), idesc_acc, hs > 0 || k > 0);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f16_ts(tDV, tS + k * 8, umma_smem_desc(sDO + k * 2048, AB_BOX, 1024), idesc_acc, (it > 0 || w > 0 || k > 0));
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f16_ts(tDK, tDP + k * 8, umma_smem_desc(sQ + k * 2048, AB_BOX, 1024), idesc_acc, (it > 0 || w > 0 || k > 0));
-          if (it + 1 < n_it) issue_scores(w, (it + 1) & 1);
-        }
-        if (ok) umma_commit(bar_empty + st * 8);
+        for (int k = 0; k < 4; ++k) umma_f16_ts_lo(tDK, tDP + k * 8, dQ + k * (2048 >> 4), idesc_acc, hs > 0 || k > 0);
+        umma_commit(bar_empty + st * 8);
+        if (hs + NS < n) next_scores(sl);
+        if (++sl == NS) { sl = 0; sph ^= 1; }
+        if (++st == ST) st = 0;
       }
       umma_commit(bar_acc);
     }
@@ -218,64 +222,84 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
     const int r = quad * 32 + lane;
     const int key_idx = jb * 128 + r;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
-    const uint32_t tS = tmem_base + w * 128 + lane_off, tDP = tS + 64;
-    const float sl2 = p.scale * LOG2E;
+    const float2 sl2 = make_float2(p.scale * LOG2E, p.scale * LOG2E);
     bool ok = true;
-    // thread r stages one statistic of this half's 64 queries: r < 64 the pre-scaled log-sum-exp of query r, else the
-    // delta of query r - 64.  Loaded one step ahead so that the global-memory latency hides behind the arithmetic.
-    auto load_stat = [&](int it) -> float {
-      const int h = hk * G + it / n_i, i = i0 + it % n_i;
-      const int qi = i * 128 + w * 64 + (r & 63);
-      const long long o = ((long long)b * p.Hq + h) * p.S + qi;
-      if (r < 64) return qi < p.S ? p.lse[o] * LOG2E : INFINITY;   // +inf => probability 0 for padded queries
-      return qi < p.S ? p.delta[o] : 0.f;
+    // thread r stages one statistic of the half block's 64 queries, negated: r < 64 the pre-scaled log-sum-exp of query r, else the
+    // delta of query r - 64.  Loaded one turn ahead so that the global-memory latency hides behind the arithmetic.
+    auto load_stat = [&](int g, int i) -> float {
+      const int qi = (i0 + i) * 64 + (r & 63);
+      const long long o = ((long long)b * p.Hq + hk * G + g) * p.S + qi;
+      if (r < 64) return qi < p.S ? -p.lse[o] * LOG2E : -INFINITY;   // probability 0 for padded queries
+      return qi < p.S ? -p.delta[o] : 0.f;
     };
-    float nxt = n_it > 0 ? load_stat(0) : 0.f;
-    for (int it = 0; it < n_it; ++it) {
-      const int i = i0 + it % n_i;
-      const uint32_t ph = it & 1;
-      float* s_lse = stats + ((it & 1) * 2 + w) * 128;
+    auto advance = [&](int& g, int& i) {      // two half blocks on
+      i += 2;
+      while (i >= n_i) { i -= n_i; ++g; }
+    };
+    int g = 0, i = w, slot = w;
+    uint32_t turn = 0, sph = 0;
+    while (i >= n_i) { i -= n_i; ++g; }
+    float nxt = w < n ? load_stat(g, i) : 0.f;
+    for (int hs = w; hs < n; hs += 2, turn ^= 1) {
+      const int q0 = (i0 + i) * 64;
+      const uint32_t tS = tmem_base + slot * 128 + lane_off, tDP = tS + 64;
+      const uint32_t bar_ready = bar_s + slot * 8, bar_done = bar_pds + slot * 8, par = sph;
+      slot += 2;
+      if (slot >= NS) { slot -= NS; sph ^= 1; }
+      float* s_lse = stats + (w * 2 + turn) * 128;
       float* s_dl = s_lse + 64;
       s_lse[r] = nxt;
       mbar_arrive(bar_stat + w * 8);
-      if (it + 1 < n_it) nxt = load_stat(it + 1);
-      if (!mbar_wait_warp(bar_stat + w * 8, ph, abort_flag, p.status, ST_TIMEOUT_FLAG)) { ok = false; break; }
-      if (!mbar_wait_warp(bar_s + w * 8, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      advance(g, i);
+      if (hs + 2 < n) nxt = load_stat(g, i);
+      if (!mbar_wait_warp(bar_stat + w * 8, turn, abort_flag, p.status, ST_TIMEOUT_FLAG)) { ok = false; break; }
+      if (!mbar_wait_warp(bar_ready, par, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      const bool diag = p.causal && (i == jb);
+      const bool diag = p.causal && q0 < jb * 128 + 128;
+      uint32_t sv[2][32], dv[2][32];
+      tmem_ld_32x32(tS, sv[0]);
+      tmem_ld_32x32(tDP, dv[0]);
+      tmem_ld_wait_regs(sv[0]);
+      tmem_ld_wait_regs(dv[0]);
+      tmem_ld_32x32(tS + 32, sv[1]);          // in flight behind the arithmetic of the first half
+      tmem_ld_32x32(tDP + 32, dv[1]);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        uint32_t sv[32], dv[32];
-        tmem_ld_32x32(tS + c * 32, sv);
-        tmem_ld_32x32(tDP + c * 32, dv);
-        tmem_ld_wait();
+        if (c == 1) {
+          tmem_ld_wait_regs(sv[1]);
+          tmem_ld_wait_regs(dv[1]);
+        }
         uint32_t pk[16], ds[16];
 #pragma unroll
-        for (int e4 = 0; e4 < 8; ++e4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(s_lse + c * 32 + e4 * 4);   // same address in every lane: broadcast
-          const float4 d4 = *reinterpret_cast<const float4*>(s_dl + c * 32 + e4 * 4);
-          const int q0 = w * 64 + c * 32 + e4 * 4;      // query index inside the 128-query block
-          float p0 = bwd_exp2(fmaf(__uint_as_float(sv[e4 * 4 + 0]), sl2, -l4.x));
-          float p1 = bwd_exp2(fmaf(__uint_as_float(sv[e4 * 4 + 1]), sl2, -l4.y));
-          float p2 = bwd_exp2(fmaf(__uint_as_float(sv[e4 * 4 + 2]), sl2, -l4.z));
-          float p3 = bwd_exp2(fmaf(__uint_as_float(sv[e4 * 4 + 3]), sl2, -l4.w));
+        for (int e = 0; e < 16; e += 2) {
+          const float4 l4 = *reinterpret_cast<const float4*>(s_lse + c * 32 + e * 2);   // same address in every lane: broadcast
+          const float4 d4 = *reinterpret_cast<const float4*>(s_dl + c * 32 + e * 2);
+          float2 a = fma2(make_float2(__uint_as_float(sv[c][2 * e]), __uint_as_float(sv[c][2 * e + 1])), sl2, make_float2(l4.x, l4.y));
+          float2 e2 = fma2(make_float2(__uint_as_float(sv[c][2 * e + 2]), __uint_as_float(sv[c][2 * e + 3])), sl2, make_float2(l4.z, l4.w));
+          a.x = bwd_exp2(a.x);
+          a.y = bwd_exp2(a.y);
+          e2.x = bwd_exp2(e2.x);
+          e2.y = bwd_exp2(e2.y);
           if (diag) {
-            if (q0 < r) p0 = 0.f;
-            if (q0 + 1 < r) p1 = 0.f;
-            if (q0 + 2 < r) p2 = 0.f;
-            if (q0 + 3 < r) p3 = 0.f;
+            const int q = q0 + c * 32 + 2 * e;
+            if (q < key_idx) a.x = 0.f;
+            if (q + 1 < key_idx) a.y = 0.f;
+            if (q + 2 < key_idx) e2.x = 0.f;
+            if (q + 3 < key_idx) e2.y = 0.f;
           }
-          pk[e4 * 2] = pack_bf16(p0, p1);
-          pk[e4 * 2 + 1] = pack_bf16(p2, p3);
-          ds[e4 * 2] = pack_bf16(p0 * (__uint_as_float(dv[e4 * 4 + 0]) - d4.x), p1 * (__uint_as_float(dv[e4 * 4 + 1]) - d4.y));
-          ds[e4 * 2 + 1] = pack_bf16(p2 * (__uint_as_float(dv[e4 * 4 + 2]) - d4.z), p3 * (__uint_as_float(dv[e4 * 4 + 3]) - d4.w));
+          pk[e] = pack_bf16(a.x, a.y);
+          pk[e + 1] = pack_bf16(e2.x, e2.y);
+          a = mul2(a, add2(make_float2(__uint_as_float(dv[c][2 * e]), __uint_as_float(dv[c][2 * e + 1])), make_float2(d4.x, d4.y)));
+          e2 = mul2(e2, add2(make_float2(__uint_as_float(dv[c][2 * e + 2]), __uint_as_float(dv[c][2 * e + 3])), make_float2(d4.z, d4.w)));
+          ds[e] = pack_bf16(a.x, a.y);
+          ds[e + 1] = pack_bf16(e2.x, e2.y);
         }
         tmem_st_32x16(tS + c * 16, pk);
         tmem_st_32x16(tDP + c * 16, ds);
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(bar_pds + w * 8);
+      mbar_arrive(bar_done);
     }
     if (ok && mbar_wait_warp(bar_acc, 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
@@ -290,7 +314,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
       for (int c = 0; c < D / 32; ++c) {
         uint32_t v[32];
         tmem_ld_32x32(tA + c * 32, v);
-        tmem_ld_wait();
+        tmem_ld_wait_regs(v);
         if (valid) store_row32(dst + c * 32, v, sc);
       }
     }
@@ -307,25 +331,35 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
 // dQ
 // ------------------------------------------------------------------------------------------------
 // dS = P * (dP - delta) for one query row and one half block (64 keys): reads S and dP from tensor memory, writes dS
-// (bf16 pairs) over the dP columns.
+// (bf16 pairs) over the dP columns.  nlse2, ndl: negated log-sum-exp (base 2) and delta of the row.
 template <bool MASK>
-__device__ __forceinline__ void dq_half_block(uint32_t tS, uint32_t tDP, float sl2, float lse2, float dl, int k0, int k_lim) {
+__device__ __forceinline__ void dq_half_block(uint32_t tS, uint32_t tDP, float scale2, float nlse2, float ndl, int k0, int k_lim) {
+  uint32_t sv[2][32], dv[2][32];
+  const float2 sl2 = make_float2(scale2, scale2), l2 = make_float2(nlse2, nlse2), d2 = make_float2(ndl, ndl);
+  tmem_ld_32x32(tS, sv[0]);
+  tmem_ld_32x32(tDP, dv[0]);
+  tmem_ld_wait_regs(sv[0]);
+  tmem_ld_wait_regs(dv[0]);
+  tmem_ld_32x32(tS + 32, sv[1]);             // in flight behind the arithmetic of the first half
+  tmem_ld_32x32(tDP + 32, dv[1]);
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    uint32_t s[32], dp[32];
-    tmem_ld_32x32(tS + c * 32, s);
-    tmem_ld_32x32(tDP + c * 32, dp);
-    tmem_ld_wait();
     uint32_t ds[16];
+    if (c == 1) {
+      tmem_ld_wait_regs(sv[1]);
+      tmem_ld_wait_regs(dv[1]);
+    }
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
-      float p0 = bwd_exp2(fmaf(__uint_as_float(s[2 * e]), sl2, -lse2));
-      float p1 = bwd_exp2(fmaf(__uint_as_float(s[2 * e + 1]), sl2, -lse2));
+      float2 a = fma2(make_float2(__uint_as_float(sv[c][2 * e]), __uint_as_float(sv[c][2 * e + 1])), sl2, l2);
+      a.x = bwd_exp2(a.x);
+      a.y = bwd_exp2(a.y);
       if (MASK) {
-        if (k0 + c * 32 + 2 * e > k_lim) p0 = 0.f;
-        if (k0 + c * 32 + 2 * e + 1 > k_lim) p1 = 0.f;
+        if (k0 + c * 32 + 2 * e > k_lim) a.x = 0.f;
+        if (k0 + c * 32 + 2 * e + 1 > k_lim) a.y = 0.f;
       }
-      ds[e] = pack_bf16(p0 * (__uint_as_float(dp[2 * e]) - dl), p1 * (__uint_as_float(dp[2 * e + 1]) - dl));
+      a = mul2(a, add2(make_float2(__uint_as_float(dv[c][2 * e]), __uint_as_float(dv[c][2 * e + 1])), d2));
+      ds[e] = pack_bf16(a.x, a.y);
     }
     tmem_st_32x16(tDP + c * 16, ds);
   }
@@ -337,36 +371,38 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                    const AttnBwdParams p) {
   tfb::pdl_sync();
-  using L = BwdSmem<D>;
-  constexpr int NB = L::NB;
+  using L = BwdSmem<D, false>;
+  constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
   const uint32_t sQ = sbase, sDO = sbase + L::TILE;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   const uint32_t bar_q = smem_u32(bars);
-  const uint32_t bar_full = bar_q + 8;     // [2]
-  const uint32_t bar_empty = bar_full + 16;
-  const uint32_t bar_s = bar_empty + 16;   // [2] S_w and dP_w ready
-  const uint32_t bar_ds = bar_s + 16;      // [2] dS_w written (128 arrivals)
-  const uint32_t bar_acc = bar_ds + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  const uint32_t bar_full = bar_q + 8;             // [ST]
+  const uint32_t bar_empty = bar_full + ST * 8;    // [ST]
+  const uint32_t bar_s = bar_empty + ST * 8;       // [NS] S and dP ready
+  const uint32_t bar_ds = bar_s + NS * 8;          // [NS] dS written (128 arrivals)
+  const uint32_t bar_acc = bar_ds + NS * 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 + 2 * ST + 2 * NS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nqb = (p.S + 127) / 128;
+  const int nqb = (p.S + 127) / 128, nkh = (p.S + 63) / 64;
   const int bh = p.B * p.Hq;
   const int qb = nqb - 1 - int(blockIdx.x) / bh;
   const int rem = int(blockIdx.x) % bh;
   const int b = rem / p.Hq, h = rem % p.Hq;
   const int hk = h / (p.Hq / p.Hkv);
-  const int n_kv = p.causal ? qb + 1 : nqb;
+  const int n = p.causal ? min(2 * qb + 2, nkh) : nkh;
 
   if (threadIdx.x == 0) {
     mbar_init(bar_q, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < ST; ++s) {
       mbar_init(bar_full + s * 8, 1);
       mbar_init(bar_empty + s * 8, 1);
+    }
+    for (int s = 0; s < NS; ++s) {
       mbar_init(bar_s + s * 8, 1);
       mbar_init(bar_ds + s * 8, 128);
     }
@@ -382,7 +418,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tDQ = tmem_base + 256;
+  const uint32_t tDQ = tmem_base + L::ACC_COL;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -392,17 +428,19 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         tma_load_3d(sQ + c * AB_BOX, &tq, bar_q, p.q_col0 + h * D + c * 64, qb * 128, b);
         tma_load_3d(sDO + c * AB_BOX, &tdo, bar_q, h * D + c * 64, qb * 128, b);
       }
-      for (int j = 0; j < n_kv; ++j) {
-        const int st = j & 1;
-        if (!mbar_wait(bar_empty + st * 8, ((j >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+      int st = 0;
+      uint32_t ph = 1;
+      for (int hs = 0; hs < n; ++hs) {
+        if (!mbar_wait(bar_empty + st * 8, ph, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
         const uint32_t fb = bar_full + st * 8;
-        mbar_expect_tx(fb, 2 * L::TILE);
-        const uint32_t sK = sbase + L::RING_OFF + st * 2 * L::TILE, sV = sK + L::TILE;
+        mbar_expect_tx(fb, 2 * L::HALF);
+        const uint32_t sK = sbase + L::RING_OFF + st * 2 * L::HALF, sV = sK + L::HALF;
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
-          tma_load_3d(sK + c * AB_BOX, &tk, fb, p.k_col0 + hk * D + c * 64, j * 128, b);
-          tma_load_3d(sV + c * AB_BOX, &tv, fb, p.v_col0 + hk * D + c * 64, j * 128, b);
+          tma_load_3d(sK + c * AB_HBOX, &tk, fb, p.k_col0 + hk * D + c * 64, hs * 64, b);
+          tma_load_3d(sV + c * AB_HBOX, &tv, fb, p.v_col0 + hk * D + c * 64, hs * 64, b);
         }
+        if (++st == ST) { st = 0; ph ^= 1; }
       }
       if (*abort_flag) {
         const uint64_t t0 = globaltimer_ns();
@@ -413,47 +451,42 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc(FMT_BF16, FMT_BF16, false, false, 128, 64);
       constexpr uint32_t idesc_acc = umma_idesc(FMT_BF16, FMT_BF16, false, true, 128, D);
-      auto issue_scores = [&](int w, int st) {
-        const uint32_t sK = sbase + L::RING_OFF + st * 2 * L::TILE + w * AB_HALF, sV = sK + L::TILE;
-        const uint32_t tS = tmem_base + w * 128, tDP = tS + 64;
+      const uint32_t dQ = umma_desc_lo(sQ, 16), dDO = umma_desc_lo(sDO, 16);
+      auto issue_scores = [&](int sl, int st) {
+        const uint32_t sK = sbase + L::RING_OFF + st * 2 * L::HALF;
+        const uint32_t dK = umma_desc_lo(sK, 16), dV = umma_desc_lo(sK + L::HALF, 16);
+        const uint32_t tS = tmem_base + sl * 128, tDP = tS + 64;
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * AB_BOX + (k & 3) * 32;
-          umma_f16_ss(tS, umma_smem_desc(sQ + off, 16, 1024), umma_smem_desc(sK + off, 16, 1024), idesc_s, k > 0);
-        }
+        for (int k = 0; k < D / 16; ++k)
+          umma_f16_ss_lo(tS, dQ + (((k >> 2) * AB_BOX + (k & 3) * 32) >> 4), dK + (((k >> 2) * AB_HBOX + (k & 3) * 32) >> 4), idesc_s, k > 0);
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * AB_BOX + (k & 3) * 32;
-          umma_f16_ss(tDP, umma_smem_desc(sDO + off, 16, 1024), umma_smem_desc(sV + off, 16, 1024), idesc_s, k > 0);
-        }
-        umma_commit(bar_s + w * 8);
+        for (int k = 0; k < D / 16; ++k)
+          umma_f16_ss_lo(tDP, dDO + (((k >> 2) * AB_BOX + (k & 3) * 32) >> 4), dV + (((k >> 2) * AB_HBOX + (k & 3) * 32) >> 4), idesc_s, k > 0);
+        umma_commit(bar_s + sl * 8);
       };
-      bool ok = mbar_wait(bar_q, 0, abort_flag, p.status, ST_TIMEOUT_FULL) &&
-                (n_kv == 0 || mbar_wait(bar_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL));
-      if (ok && n_kv > 0) {
+      bool ok = mbar_wait(bar_q, 0, abort_flag, p.status, ST_TIMEOUT_FULL);
+      int nst = 0;                      // stage and turn of the next scores
+      uint32_t nph = 0;
+      auto next_scores = [&](int sl) {
+        if (!mbar_wait(bar_full + nst * 8, nph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; return; }
         tc_fence_after();
-        issue_scores(0, 0);
-        issue_scores(1, 0);
-      }
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int st = j & 1;
-        if (j + 1 < n_kv) {
-          if (!mbar_wait(bar_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) break;
-          tc_fence_after();
-        }
+        issue_scores(sl, nst);
+        if (++nst == ST) { nst = 0; nph ^= 1; }
+      };
+      for (int hs = 0; hs < NS && hs < n && ok; ++hs) next_scores(hs);
+      int sl = 0, st = 0;
+      uint32_t sph = 0;
+      for (int hs = 0; hs < n && ok; ++hs) {
+        if (!mbar_wait(bar_ds + sl * 8, sph, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
+        tc_fence_after();
+        const uint32_t dK = umma_desc_lo(sbase + L::RING_OFF + st * 2 * L::HALF, AB_HBOX);
+        const uint32_t tDP = tmem_base + sl * 128 + 64;
 #pragma unroll
-        for (int w = 0; w < 2; ++w) {
-          if (!ok) continue;
-          if (!mbar_wait(bar_ds + w * 8, j & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; continue; }
-          tc_fence_after();
-          const uint32_t sK = sbase + L::RING_OFF + st * 2 * L::TILE + w * AB_HALF;
-          const uint32_t tDP = tmem_base + w * 128 + 64;
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f16_ts(tDQ, tDP + k * 8, umma_smem_desc(sK + k * 2048, AB_BOX, 1024), idesc_acc, (j > 0 || w > 0 || k > 0));
-          if (j + 1 < n_kv) issue_scores(w, (j + 1) & 1);
-        }
-        if (ok) umma_commit(bar_empty + st * 8);
+        for (int k = 0; k < 4; ++k) umma_f16_ts_lo(tDQ, tDP + k * 8, dK + k * (2048 >> 4), idesc_acc, hs > 0 || k > 0);
+        umma_commit(bar_empty + st * 8);
+        if (hs + NS < n) next_scores(sl);
+        if (++sl == NS) { sl = 0; sph ^= 1; }
+        if (++st == ST) st = 0;
       }
       umma_commit(bar_acc);
     }
@@ -463,23 +496,24 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     const int r = quad * 32 + lane;
     const int q_idx = qb * 128 + r;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
-    const uint32_t tS = tmem_base + w * 128 + lane_off, tDP = tS + 64;
     const float sl2 = p.scale * LOG2E;
     const long long so = ((long long)b * p.Hq + h) * p.S + q_idx;
-    const float lse2 = q_idx < p.S ? p.lse[so] * LOG2E : INFINITY;
-    const float dl = q_idx < p.S ? p.delta[so] : 0.f;
+    const float nlse2 = q_idx < p.S ? -p.lse[so] * LOG2E : -INFINITY;
+    const float ndl = q_idx < p.S ? -p.delta[so] : 0.f;
     bool ok = true;
-    for (int j = 0; j < n_kv; ++j) {
-      if (!mbar_wait_warp(bar_s + w * 8, j & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+    for (int hs = w; hs < n; hs += 2) {
+      const int slot = hs % NS;
+      const uint32_t tS = tmem_base + slot * 128 + lane_off, tDP = tS + 64;
+      if (!mbar_wait_warp(bar_s + slot * 8, (hs / NS) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      const int k0 = j * 128 + w * 64;
-      const bool need_mask = (p.causal && j == qb) || (k0 + 64 > p.S);
+      const int k0 = hs * 64;
+      const bool need_mask = (p.causal && k0 + 63 > qb * 128) || (k0 + 64 > p.S);
       const int k_lim = p.causal ? min(q_idx, p.S - 1) : p.S - 1;
-      if (need_mask) dq_half_block<true>(tS, tDP, sl2, lse2, dl, k0, k_lim);
-      else dq_half_block<false>(tS, tDP, sl2, lse2, dl, k0, k_lim);
+      if (need_mask) dq_half_block<true>(tS, tDP, sl2, nlse2, ndl, k0, k_lim);
+      else dq_half_block<false>(tS, tDP, sl2, nlse2, ndl, k0, k_lim);
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(bar_ds + w * 8);
+      mbar_arrive(bar_ds + slot * 8);
     }
     if (ok && mbar_wait_warp(bar_acc, 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
@@ -535,17 +569,19 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
 }
 
 template <int D>
-static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                      const AttnBwdParams& p, cudaStream_t st) {
-  using L = BwdSmem<D>;
+static int launch_bwd(const CUtensorMap (&m)[8], const AttnBwdParams& p, cudaStream_t st) {
+  // boxes of 128 rows (resident tiles) and of 64 (half blocks)
+  const CUtensorMap &tq = m[0], &tk = m[1], &tv = m[2], &tdo = m[3], &q_half = m[4], &k_half = m[5], &v_half = m[6], &do_half = m[7];
+  using L1 = BwdSmem<D, true>;
+  using L2 = BwdSmem<D, false>;
   static DeviceOnce once1, once2;   // kernel attributes are per device: set on the first launch on each one
   auto k1 = attn_bwd_dkdv_kernel<D>;
   auto k2 = attn_bwd_dq_kernel<D>;
-  if (int e = ensure_dyn_smem(once1, k1, L::TOTAL)) return e;
-  if (int e = ensure_dyn_smem(once2, k2, L::TOTAL)) return e;
+  if (int e = ensure_dyn_smem(once1, k1, L1::TOTAL)) return e;
+  if (int e = ensure_dyn_smem(once2, k2, L2::TOTAL)) return e;
   const int nqb = (p.S + 127) / 128;
-  tfb::launch_k(k1, nqb * p.Hkv * p.B, AB_THREADS, L::TOTAL, st, tq, tk, tv, tdo, p);
-  tfb::launch_k(k2, nqb * p.Hq * p.B, AB_THREADS, L::TOTAL, st, tq, tk, tv, tdo, p);
+  tfb::launch_k(k1, nqb * p.Hkv * p.B, AB_THREADS, L1::TOTAL, st, q_half, tk, tv, do_half, p);
+  tfb::launch_k(k2, nqb * p.Hq * p.B, AB_THREADS, L2::TOTAL, st, tq, k_half, v_half, tdo, p);
   return int(cudaGetLastError());
 }
 
@@ -574,12 +610,13 @@ TFB_API int tfb_attn_bwd(const void* q, long long ldq, int q_col0, const void* k
     tfb::launch_k(attn_delta_kernel, blocks, 256, 0, st, static_cast<const __nv_bfloat16*>(o), ldo,
                                               static_cast<const __nv_bfloat16*>(dout), lddo, delta, B, S, Hq, D);
   }
-  CUtensorMap tq, tk, tv, tdo;
-  int rc;
-  if ((rc = make_tmap_3d(&tq, q, 2, ldq, S, B, ldq * 2, ldq * 2 * S, 64, 128, 1))) return rc;
-  if ((rc = make_tmap_3d(&tk, k, 2, ldk, S, B, ldk * 2, ldk * 2 * S, 64, 128, 1))) return rc;
-  if ((rc = make_tmap_3d(&tv, v, 2, ldv, S, B, ldv * 2, ldv * 2 * S, 64, 128, 1))) return rc;
-  if ((rc = make_tmap_3d(&tdo, dout, 2, lddo, S, B, lddo * 2, lddo * 2 * S, 64, 128, 1))) return rc;
+  CUtensorMap maps[8];
+  for (int i = 0; i < 8; ++i) {
+    const void* base[4] = {q, k, v, dout};
+    const long long ld[4] = {ldq, ldk, ldv, lddo};
+    const long long l = ld[i & 3];
+    if (int rc = make_tmap_3d(&maps[i], base[i & 3], 2, l, S, B, l * 2, l * 2 * S, 64, i < 4 ? 128 : 64, 1)) return rc;
+  }
   AttnBwdParams p;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv; p.scale = scale; p.causal = causal;
   p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
@@ -588,5 +625,5 @@ TFB_API int tfb_attn_bwd(const void* q, long long ldq, int q_col0, const void* k
   p.dk = static_cast<__nv_bfloat16*>(dk); p.lddk = lddk; p.dk_col0 = dk_col0;
   p.dv = static_cast<__nv_bfloat16*>(dv); p.lddv = lddv; p.dv_col0 = dv_col0;
   p.status = status;
-  return D == 64 ? launch_bwd<64>(tq, tk, tv, tdo, p, st) : launch_bwd<128>(tq, tk, tv, tdo, p, st);
+  return D == 64 ? launch_bwd<64>(maps, p, st) : launch_bwd<128>(maps, p, st);
 }

@@ -9,14 +9,15 @@
 //   attn_bwd_dq   : one CTA per (batch, query head, 128-query block); loops over half blocks of 64 keys:
 //                     S_h = Q K_h^T, dP_h = dO V_h^T, dS_h = P_h * (dP_h - delta), dQ += dS_h K_h
 //   attn_delta    : delta[b,h,s] = sum_d dO * O
-// Two compute warpgroups take the half blocks in turn.  Scores live in a ring of tensor-memory slots (128 columns: S / P in the
-// first 64, dP / dS in the others): with three slots the scores of the next two half blocks are there when a warpgroup is done, and the
-// round trip - P and dS announced, products issued, next scores computed - is off its path; the tensor core runs products
-// and scores in issue order, so a slot may be refilled right behind the products that read it.  dK / dV at heads of 128 fill
-// 256 columns themselves and leave room for two slots.  The operand tiles of the loop come in half blocks too, through a ring
-// that runs ahead of the slots.
-//   Before (two slots, one per warpgroup; whole blocks through two stages): 22 - 27 % of the exponential rate at heads of 64, a warpgroup
-// idle for a tensor-core round trip per half block.
+// Scores live in a ring of tensor-memory slots (128 columns: S / P in the first 64, dP / dS in the others); the tensor core runs
+// products and scores in issue order, so a slot may be refilled right behind the products that read it.  The operand tiles of the
+// loop come in half blocks too, through a ring that runs ahead of the slots.
+//   Heads of 128: two compute warpgroups take the half blocks in turn, over three slots (dK / dV: two, their accumulators fill 256
+// columns), so that the scores of the next half block are there when a warpgroup is done.
+//   Heads of 64: loops are short (nine half blocks on average at 1024 tokens) and a CTA's start and end cost as much as they do; one
+// warpgroup and one slot in 256 columns, two CTAs per SM, one working while the other starts, waits or writes.
+// Both kernels and attn_delta, us, before (two warpgroups with a slot each, one CTA per SM) -> three slots -> two CTAs per SM: 64 x
+// 1024, 8 heads of 64 804 -> 747 -> 601; 8 x 1024 112 -> 112 -> 100; 4096, 32 / 8 heads of 128 703 -> 650.
 // The softmax scale multiplies dK and dQ once, when they are written out.
 //
 // The reference's memory-efficient attention backward is approximate
@@ -27,7 +28,7 @@
 
 namespace tfb {
 
-constexpr int AB_THREADS = 320;   // warp 0 TMA, warp 1 MMA, warps 2-5 half 0, warps 6-9 half 1
+// warp 0 TMA, warp 1 MMA, warps 2-5 and (heads of 128) 6-9: compute warpgroups
 constexpr int AB_BOX = 128 * 64 * 2;
 constexpr int AB_HBOX = 64 * 64 * 2;   // 64 columns of a half block (64 rows)
 constexpr float LOG2E = 1.4426950408889634f;
@@ -55,14 +56,16 @@ template <int D, bool DKDV>
 struct BwdSmem {
   static constexpr int NB = D / 64;
   static constexpr int TILE = NB * AB_BOX, HALF = NB * AB_HBOX;     // a resident tile, a half block
-  static constexpr int SLOTS = DKDV && D == 128 ? 2 : 3;            // tensor-memory slots
-  static constexpr int ACC_COL = SLOTS * 128;
-  static constexpr int STAGES = D == 64 ? 6 : DKDV ? 4 : 5;         // half blocks (two operands each) in flight
+  static constexpr int WG = D == 64 ? 1 : 2;                        // compute warpgroups
+  static constexpr int THREADS = 64 + 128 * WG;
+  static constexpr int SLOTS = D == 64 ? 1 : DKDV ? 2 : 3;          // tensor-memory slots
+  static constexpr int ACC_COL = SLOTS * 128, TMEM = D == 64 ? 256 : 512;
+  static constexpr int STAGES = D == 64 || DKDV ? 4 : 5;            // half blocks (two operands each) in flight
   static constexpr int RING_OFF = 2 * TILE;                         // behind two resident tiles
-  static constexpr int STAT_OFF = RING_OFF + STAGES * 2 * HALF;     // [2 warpgroups][2 turns][64 -lse | 64 -delta] floats
-  static constexpr int BAR_OFF = STAT_OFF + (DKDV ? 2 * 2 * 128 * 4 : 0);
+  static constexpr int STAT_OFF = RING_OFF + STAGES * 2 * HALF;     // [warpgroups][2 turns][64 -lse | 64 -delta] floats
+  static constexpr int BAR_OFF = STAT_OFF + (DKDV ? WG * 2 * 128 * 4 : 0);
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
-  static_assert(ACC_COL + (DKDV ? 2 : 1) * D <= 512 && TOTAL <= 232448, "tensor and shared memory");
+  static_assert(ACC_COL + (DKDV ? 2 : 1) * D <= TMEM && TOTAL <= (D == 64 ? 115712 : 232448), "tensor and shared memory");
 };
 
 // 16 output rows x 128 bf16 columns of an accumulator, written by one thread (its row)
@@ -82,13 +85,13 @@ __device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (
 // dK / dV
 // ------------------------------------------------------------------------------------------------
 template <int D>
-__global__ void __launch_bounds__(AB_THREADS, 1)
+__global__ void __launch_bounds__(BwdSmem<D, true>::THREADS, D == 64 ? 2 : 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                      const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                      const AttnBwdParams p) {
   tfb::pdl_sync();
   using L = BwdSmem<D, true>;
-  constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES;
+  constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES, WG = L::WG;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
@@ -132,7 +135,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_alloc(smem_u32(tmem_slot), L::TMEM);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -232,26 +235,26 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
       if (r < 64) return qi < p.S ? -p.lse[o] * LOG2E : -INFINITY;   // probability 0 for padded queries
       return qi < p.S ? -p.delta[o] : 0.f;
     };
-    auto advance = [&](int& g, int& i) {      // two half blocks on
-      i += 2;
+    auto advance = [&](int& g, int& i) {      // to this warpgroup's next half block
+      i += WG;
       while (i >= n_i) { i -= n_i; ++g; }
     };
     int g = 0, i = w, slot = w;
     uint32_t turn = 0, sph = 0;
     while (i >= n_i) { i -= n_i; ++g; }
     float nxt = w < n ? load_stat(g, i) : 0.f;
-    for (int hs = w; hs < n; hs += 2, turn ^= 1) {
+    for (int hs = w; hs < n; hs += WG, turn ^= 1) {
       const int q0 = (i0 + i) * 64;
       const uint32_t tS = tmem_base + slot * 128 + lane_off, tDP = tS + 64;
       const uint32_t bar_ready = bar_s + slot * 8, bar_done = bar_pds + slot * 8, par = sph;
-      slot += 2;
+      slot += WG;
       if (slot >= NS) { slot -= NS; sph ^= 1; }
       float* s_lse = stats + (w * 2 + turn) * 128;
       float* s_dl = s_lse + 64;
       s_lse[r] = nxt;
       mbar_arrive(bar_stat + w * 8);
       advance(g, i);
-      if (hs + 2 < n) nxt = load_stat(g, i);
+      if (hs + WG < n) nxt = load_stat(g, i);
       if (!mbar_wait_warp(bar_stat + w * 8, turn, abort_flag, p.status, ST_TIMEOUT_FLAG)) { ok = false; break; }
       if (!mbar_wait_warp(bar_ready, par, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
@@ -305,17 +308,21 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
       tc_fence_after();
       const bool valid = key_idx < p.S;
       const long long row = (long long)b * p.S + (valid ? key_idx : 0);
-      // half 0 writes dV, half 1 writes dK (scaled).  The tensor-memory loads are warp-collective: every lane executes
-      // them, only the stores are predicated.
-      __nv_bfloat16* dst = w == 0 ? p.dv + row * p.lddv + p.dv_col0 + hk * D : p.dk + row * p.lddk + p.dk_col0 + hk * D;
-      const uint32_t tA = (w == 0 ? tDV : tDK) + lane_off;
-      const float sc = w == 0 ? 1.f : p.scale;
+      // warpgroup 0 writes dV, warpgroup 1 (or the only one) dK, scaled.  The tensor-memory loads are warp-collective: every
+      // lane executes them, only the stores are predicated.
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32(tA + c * 32, v);
-        tmem_ld_wait_regs(v);
-        if (valid) store_row32(dst + c * 32, v, sc);
+      for (int k = 0; k < 2; ++k) {
+        if (WG == 2 && k != w) continue;
+        __nv_bfloat16* dst = k == 0 ? p.dv + row * p.lddv + p.dv_col0 + hk * D : p.dk + row * p.lddk + p.dk_col0 + hk * D;
+        const uint32_t tA = (k == 0 ? tDV : tDK) + lane_off;
+        const float sc = k == 0 ? 1.f : p.scale;
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t v[32];
+          tmem_ld_32x32(tA + c * 32, v);
+          tmem_ld_wait_regs(v);
+          if (valid) store_row32(dst + c * 32, v, sc);
+        }
       }
     }
   }
@@ -323,7 +330,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, L::TMEM);
   }
 }
 
@@ -366,13 +373,13 @@ __device__ __forceinline__ void dq_half_block(uint32_t tS, uint32_t tDP, float s
 }
 
 template <int D>
-__global__ void __launch_bounds__(AB_THREADS, 1)
+__global__ void __launch_bounds__(BwdSmem<D, false>::THREADS, D == 64 ? 2 : 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                    const AttnBwdParams p) {
   tfb::pdl_sync();
   using L = BwdSmem<D, false>;
-  constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES;
+  constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES, WG = L::WG;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
@@ -411,7 +418,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_alloc(smem_u32(tmem_slot), L::TMEM);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -501,7 +508,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     const float nlse2 = q_idx < p.S ? -p.lse[so] * LOG2E : -INFINITY;
     const float ndl = q_idx < p.S ? -p.delta[so] : 0.f;
     bool ok = true;
-    for (int hs = w; hs < n; hs += 2) {
+    for (int hs = w; hs < n; hs += WG) {
       const int slot = hs % NS;
       const uint32_t tS = tmem_base + slot * 128 + lane_off, tDP = tS + 64;
       if (!mbar_wait_warp(bar_s + slot * 8, (hs / NS) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
@@ -517,12 +524,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     }
     if (ok && mbar_wait_warp(bar_acc, 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
-      // each half writes D / 2 columns of the row
-      __nv_bfloat16* dqp = p.dq + ((long long)b * p.S + q_idx) * p.lddq + p.dq_col0 + h * D + w * (D / 2);
+      // each warpgroup writes its share of the row's columns
+      __nv_bfloat16* dqp = p.dq + ((long long)b * p.S + q_idx) * p.lddq + p.dq_col0 + h * D + w * (D / WG);
 #pragma unroll
-      for (int c = 0; c < D / 64; ++c) {
+      for (int c = 0; c < D / 32 / WG; ++c) {
         uint32_t v[32];
-        tmem_ld_32x32(tDQ + lane_off + w * (D / 2) + c * 32, v);
+        tmem_ld_32x32(tDQ + lane_off + w * (D / WG) + c * 32, v);
         tmem_ld_wait();
         if (q_idx < p.S) store_row32(dqp + c * 32, v, p.scale);
       }
@@ -532,7 +539,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, L::TMEM);
   }
 }
 
@@ -580,8 +587,8 @@ static int launch_bwd(const CUtensorMap (&m)[8], const AttnBwdParams& p, cudaStr
   if (int e = ensure_dyn_smem(once1, k1, L1::TOTAL)) return e;
   if (int e = ensure_dyn_smem(once2, k2, L2::TOTAL)) return e;
   const int nqb = (p.S + 127) / 128;
-  tfb::launch_k(k1, nqb * p.Hkv * p.B, AB_THREADS, L1::TOTAL, st, q_half, tk, tv, do_half, p);
-  tfb::launch_k(k2, nqb * p.Hq * p.B, AB_THREADS, L2::TOTAL, st, tq, k_half, v_half, tdo, p);
+  tfb::launch_k(k1, nqb * p.Hkv * p.B, L1::THREADS, L1::TOTAL, st, q_half, tk, tv, do_half, p);
+  tfb::launch_k(k2, nqb * p.Hq * p.B, L2::THREADS, L2::TOTAL, st, tq, k_half, v_half, tdo, p);
   return int(cudaGetLastError());
 }
 

@@ -112,3 +112,46 @@ def test_repetition_penalty_and_bf16():
     r = torch.full((1,), 1.5, device="cuda")
     ids = S.sample(logits.bfloat16().cuda(), t, k, p, r, hist.cuda())
     assert int(ids[0]) == 9
+
+
+@pytest.mark.parametrize("mode", ["bf16", "fp8", "q4"])
+@pytest.mark.parametrize("Hq,Hkv,D,T", [(8, 2, 64, 1), (4, 1, 128, 77), (4, 4, 64, 300), (32, 8, 128, 5)])
+def test_rope_append_is_rotation_then_append(mode, Hq, Hkv, D, T):
+    """One pass gives the rows of the rotation kernel and the cache of the append kernel (rows of slot -1 are not cached)."""
+    from transformers_fusion_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, (Hq + 2 * Hkv) * D, device="cuda", generator=g).bfloat16()
+    cos, sin = F.rope_tables(D, 512, 10000.0, device="cuda")
+    pos = torch.randint(0, 512, (T,), device="cuda", generator=g, dtype=torch.int32)
+    slots = torch.randperm(32 * PAGE, device="cuda")[:T]
+    slots[T // 2] = -1 if T > 1 else slots[0]
+    a, b = PagedKVCache(1, 32, Hkv, D, mode, "cuda"), PagedKVCache(1, 32, Hkv, D, mode, "cuda")
+    y, z = x.clone(), x.clone()
+    a.rope_append(0, y, (cos, sin), pos, Hq, slots)
+    F.rope_(z, cos, sin, Hq + Hkv, D, T, positions=pos)
+    torch.cuda.synchronize()
+    # products and sums of fp32 in another order of contraction: a rounding step of bf16 here and there
+    assert (y.float() - z.float()).abs().max().item() <= 2 ** -7 * z.float().abs().max().item()
+    assert torch.equal(y[:, (Hq + Hkv) * D:], x[:, (Hq + Hkv) * D:])
+    b.append(0, y, Hq * D, (Hq + Hkv) * D, slots)
+    torch.cuda.synchronize()
+    for p, q in ((a.k[0], b.k[0]), (a.v[0], b.v[0])):
+        assert torch.equal(p.data, q.data) and (p.scale is None or torch.equal(p.scale, q.scale))
+
+
+@pytest.mark.parametrize("splits", [1, 2, 3, 7, 16])
+def test_paged_decode_merges_its_splits(splits):
+    """The block that arrives last merges: the same bits from call to call, splits that hold no token included."""
+    Hq, Hkv, D, lens = 8, 2, 64, torch.tensor([1, 17, 300, 129], dtype=torch.int32)
+    c = {d: PagedKVCache(1, 80, Hkv, D, "bf16", d) for d in ("cpu", "cuda")}
+    bt = torch.arange(80, dtype=torch.int32).view(4, 20)
+    slots = torch.cat([bt[b].long().repeat_interleave(PAGE)[:n] * PAGE + torch.arange(n) % PAGE for b, n in enumerate(lens.tolist())])
+    src, q = torch.randn(int(lens.sum()), (Hq + 2 * Hkv) * D).bfloat16(), torch.randn(4, Hq * D).bfloat16()
+    for d, cache in c.items():
+        cache.append(0, src.to(d), Hq * D, (Hq + Hkv) * D, slots.to(d))
+    want = c["cpu"].decode(0, q, bt, lens, Hq).float()
+    got = [c["cuda"].decode(0, q.cuda(), bt.cuda(), lens.cuda(), Hq, splits=splits) for _ in range(3)]
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert (got[0].float().cpu() - want).abs().max().item() < 2e-2
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])

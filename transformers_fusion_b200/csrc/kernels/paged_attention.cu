@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <cuda_fp16.h>
 
 #include "tfb_host.h"
@@ -117,6 +118,63 @@ __global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ src, long lon
   }
   store_row<MODE>(kpool, slot, h, Hkv, D, kv, n, lane);
   store_row<MODE>(vpool, slot, h, Hkv, D, vv, n, lane);
+}
+
+// The rotation of the q and k heads and the append in one pass (a decode step or a prompt of the dense decoder): one warp per token and q
+// or kv head; rotate-half pairs sit in lanes 16 apart.  The rotated k is rounded to bf16 in place and it is that value
+// which goes to the pool, as from the separate kernels.
+template <int MODE, int N>
+__global__ void __launch_bounds__(256) kv_rope_append_kernel(__nv_bfloat16* __restrict__ x, long long ld, const float* __restrict__ cos_t,
+                                                             const float* __restrict__ sin_t, const int* __restrict__ positions,
+                                                             const long long* __restrict__ slot_mapping, KvPool kpool, KvPool vpool, int T, int Hq,
+                                                             int Hkv) {
+  tfb::pdl_sync();
+  constexpr int D = N * 32;
+  using Vec = typename std::conditional<N == 2, uint32_t, uint2>::type;
+  const int lane = threadIdx.x & 31;
+  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  if (w >= (long long)T * (Hq + Hkv)) return;
+  const int h = int(w % (Hq + Hkv));
+  const long long t = w / (Hq + Hkv);
+  __nv_bfloat16* p = x + t * ld + (long long)h * D + lane * N;
+  const Vec raw = *reinterpret_cast<const Vec*>(p);
+  const long long at = (long long)positions[t] * (D / 2) + (lane & 15) * N;
+  const bool is_k = h >= Hq;
+  const long long slot = is_k ? slot_mapping[t] : -1;
+  Vec vraw = raw;
+  if (is_k) vraw = *reinterpret_cast<const Vec*>(p + Hkv * D);
+  const uint32_t* u = reinterpret_cast<const uint32_t*>(&raw);
+  const float sign = lane < 16 ? -1.f : 1.f;
+  float v[N];
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    const float2 f = unpack_bf16(u[i]);
+    const float2 g = unpack_bf16(__shfl_xor_sync(0xffffffffu, u[i], 16));
+    v[2 * i] = f.x * cos_t[at + 2 * i] + sign * g.x * sin_t[at + 2 * i];
+    v[2 * i + 1] = f.y * cos_t[at + 2 * i + 1] + sign * g.y * sin_t[at + 2 * i + 1];
+  }
+  Vec out;
+  uint32_t* o = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) o[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+  *reinterpret_cast<Vec*>(p) = out;
+  if (!is_k || slot < 0) return;                     // warp-uniform
+  TFB_BOUNDS(kpool.rows == 0 || slot < kpool.rows, 51, slot, kpool.rows);
+#ifdef TFB_BOUNDS_CHECK
+  if (kpool.rows != 0 && slot >= kpool.rows) return;
+#endif
+  const uint32_t* vu = reinterpret_cast<const uint32_t*>(&vraw);
+  float kf[4], vf[4];
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    const float2 a = unpack_bf16(o[i]), c = unpack_bf16(vu[i]);
+    kf[2 * i] = a.x;
+    kf[2 * i + 1] = a.y;
+    vf[2 * i] = c.x;
+    vf[2 * i + 1] = c.y;
+  }
+  store_row<MODE>(kpool, slot, h - Hq, Hkv, D, kf, N, lane);
+  store_row<MODE>(vpool, slot, h - Hq, Hkv, D, vf, N, lane);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -522,7 +580,7 @@ template <int MODE, int D>
 __global__ void __launch_bounds__(TC_THREADS) paged_decode_mma_kernel(
     const __nv_bfloat16* __restrict__ q, long long ldq, KvPool kpool, KvPool vpool, const int* __restrict__ block_table,
     int max_pages, const int* __restrict__ seq_lens, float* __restrict__ acc_out, float* __restrict__ ml_out, int Hq, int Hkv,
-    int G, int splits, float scale, int* status) {
+    int G, int splits, float scale, __nv_bfloat16* __restrict__ out, long long ldo, int* __restrict__ counts, int* status) {
   tfb::pdl_sync();
   extern __shared__ __align__(128) uint8_t tc_smem[];
   constexpr int ROWB = D * 2 + 16;                 // padded row pitch (see tc_off)
@@ -707,20 +765,9 @@ __global__ void __launch_bounds__(TC_THREADS) paged_decode_mma_kernel(
     dst[1] = o[n][1];
   }
   __syncthreads();
-  for (int i = tid; i < G * D; i += TC_THREADS) {
-    const int g = i / D, d = i % D;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) M = fmaxf(M, red_m[w * 8 + g]);
-    float v = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float mw = red_m[w * 8 + g];
-      if (mw != -INFINITY) v += red_o[(w * 8 + g) * D + d] * exp2f(mw - M);
-    }
-    const long long base = (((long long)b * Hq + hk * G + g) * splits + sp_idx);
-    acc_out[base * D + d] = v;
-  }
+  // maximum and sum over the warps, one lane per head
+  float* head_m = red_o + 4 * 8 * D;                         // [8] (base 2)
+  float* head_l = head_m + 8;                                // [8]
   if (tid < G) {
     const int g = tid;
     float M = -INFINITY, L = 0.f;
@@ -731,22 +778,80 @@ __global__ void __launch_bounds__(TC_THREADS) paged_decode_mma_kernel(
       const float mw = red_m[w * 8 + g];
       if (mw != -INFINITY) L += red_l[w * 8 + g] * exp2f(mw - M);
     }
-    const long long base = (((long long)b * Hq + hk * G + g) * splits + sp_idx);
-    ml_out[base * 2] = M * 0.6931471805599453f;      // back to natural-log units for the combine kernel
-    ml_out[base * 2 + 1] = L;
+    head_m[g] = M;
+    head_l[g] = L;
+    if (splits > 1) {
+      const long long base = (((long long)b * Hq + hk * G + g) * splits + sp_idx);
+      __stcg(reinterpret_cast<float2*>(ml_out) + base, make_float2(M, L));
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < G * D; i += TC_THREADS) {
+    const int g = i / D, d = i % D;
+    const float M = head_m[g];
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float mw = red_m[w * 8 + g];
+      if (mw != -INFINITY) v += red_o[(w * 8 + g) * D + d] * exp2f(mw - M);
+    }
+    if (splits == 1) {
+      const float L = head_l[g];
+      out[(long long)b * ldo + (hk * G + g) * D + d] = __float2bfloat16(L > 0.f ? v / L : 0.f);
+    } else {
+      __stcg(acc_out + (((long long)b * Hq + hk * G + g) * splits + sp_idx) * D + d, v);
+    }
+  }
+  if (splits == 1) return;
+  // the block that arrives last merges the splits of its heads, in their order, and leaves the counter at zero
+  volatile int* last = reinterpret_cast<volatile int*>(head_l + 8);
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    int* c = counts + b * Hkv + hk;
+    *last = atomicAdd(c, 1) == splits - 1;
+    if (*last) *c = 0;
+  }
+  __syncthreads();
+  if (!*last) return;
+  __threadfence();
+  for (int i = tid; i < G * D; i += TC_THREADS) {
+    const int g = i / D, d = i % D;
+    const long long base = ((long long)b * Hq + hk * G + g) * splits;
+    const float2* ml = reinterpret_cast<const float2*>(ml_out) + base;
+    float M = -INFINITY, L = 0.f, v = 0.f;
+    for (int s0 = 0; s0 < splits; s0 += 4) {                 // four splits' loads in flight
+      float2 x[4];
+      float a[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int s = min(s0 + k, splits - 1);
+        x[k] = __ldcg(ml + s);
+        a[k] = __ldcg(acc_out + (base + s) * D + d);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (s0 + k >= splits || x[k].x == -INFINITY) continue;
+        const float m_new = fmaxf(M, x[k].x), f = exp2f(M - m_new), e = exp2f(x[k].x - m_new);
+        L = L * f + x[k].y * e;
+        v = v * f + a[k] * e;
+        M = m_new;
+      }
+    }
+    out[(long long)b * ldo + (hk * G + g) * D + d] = __float2bfloat16(L > 0.f ? v / L : 0.f);
   }
 }
 
 template <int MODE, int D>
 static int launch_decode_mma(dim3 grid, cudaStream_t st, const __nv_bfloat16* q, long long ldq, KvPool k, KvPool v, const int* bt,
                              int max_pages, const int* lens, float* acc, float* ml, int Hq, int Hkv, int G, int splits, float scale,
-                             int* status) {
+                             __nv_bfloat16* o, long long ldo, int* counts, int* status) {
   constexpr int SMEM = (16 + (TC_THREADS / 32) * 2 * TC_CHUNK) * (D * 2 + 16) + 128;   // Q tile, four K/V tile pairs, barriers
-  static_assert(SMEM >= int(sizeof(float)) * (64 + 4 * 8 * D), "the merge buffers reuse the staging area");
+  static_assert(SMEM >= int(sizeof(float)) * (64 + 4 * 8 * D + 17), "the merge buffers reuse the staging area");
   static DeviceOnce once;
   auto kern = paged_decode_mma_kernel<MODE, D>;
   if (int e = ensure_dyn_smem(once, kern, SMEM)) return e;
-  tfb::launch_k_pdl(kern, grid, TC_THREADS, SMEM, st, q, ldq, k, v, bt, max_pages, lens, acc, ml, Hq, Hkv, G, splits, scale, status);
+  tfb::launch_k_pdl(kern, grid, TC_THREADS, SMEM, st, q, ldq, k, v, bt, max_pages, lens, acc, ml, Hq, Hkv, G, splits, scale, o, ldo, counts, status);
   return int(cudaGetLastError());
 }
 
@@ -888,11 +993,35 @@ TFB_API int tfb_kv_append(const void* src, long long ld, int k_col0, int v_col0,
   return int(cudaGetLastError());
 }
 
-// q: [B, ldq] bf16 (query head h at column h*D).  acc_ws: fp32 [B*Hq*splits*D], ml_ws: fp32 [B*Hq*splits*2].
+// x [T, ld]: rows [q heads | k heads | v heads]; q and k are rotated in place by the tables' rows positions[t], k and v go to the slots
+// (negative: not cached).  ld a multiple of 4, x aligned to 8 bytes.
+TFB_API int tfb_kv_rope_append(void* x, long long ld, const float* cos_t, const float* sin_t, const int* positions, const long long* slot_mapping,
+                               void* k_data, void* k_scale, void* v_data, void* v_scale, int T, int Hq, int Hkv, int D, int mode,
+                               long long pool_rows, void* stream) {
+  if ((D != 64 && D != 128) || T <= 0 || Hq <= 0 || Hkv <= 0 || (ld & 3) || (reinterpret_cast<uintptr_t>(x) & 7)) return TFB_ERR_ARG;
+  KvPool kp{k_data, k_scale, pool_rows}, vp{v_data, v_scale, pool_rows};
+  const unsigned blocks = unsigned(((long long)T * (Hq + Hkv) * 32 + 255) / 256);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto s = static_cast<__nv_bfloat16*>(x);
+#define TFB_GO(MODE)                                                                                                                               \
+  do {                                                                                                                                             \
+    if (D == 64) tfb::launch_k_rows(T, kv_rope_append_kernel<MODE, 2>, blocks, 256, 0, st, s, ld, cos_t, sin_t, positions, slot_mapping, kp, vp, T, Hq, Hkv); \
+    else tfb::launch_k_rows(T, kv_rope_append_kernel<MODE, 4>, blocks, 256, 0, st, s, ld, cos_t, sin_t, positions, slot_mapping, kp, vp, T, Hq, Hkv);         \
+  } while (0)
+  if (mode == KV_BF16) TFB_GO(KV_BF16);
+  else if (mode == KV_FP8) TFB_GO(KV_FP8);
+  else if (mode == KV_Q4) TFB_GO(KV_Q4);
+  else return TFB_ERR_ARG;
+#undef TFB_GO
+  return int(cudaGetLastError());
+}
+
+// q: [B, ldq] bf16 (query head h at column h*D).  acc_ws: fp32 [B*Hq*splits*D], ml_ws: fp32 [B*Hq*splits*2] (8-byte aligned), counts: int
+// [B*Hkv], zero before the first call and left at zero by every call.
 // status: the device status word (a bulk copy that does not land within the wait bound is reported there).
 TFB_API int tfb_paged_decode(const void* q, long long ldq, void* k_data, void* k_scale, void* v_data, void* v_scale,
                              const int* block_table, int max_pages, const int* seq_lens, void* o, long long ldo,
-                             float* acc_ws, float* ml_ws, int B, int Hq, int Hkv, int D, int splits, int mode,
+                             float* acc_ws, float* ml_ws, int* counts, int B, int Hq, int Hkv, int D, int splits, int mode,
                              float scale, long long pool_rows, int* status, void* stream) {
   if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv || splits < 1) return TFB_ERR_ARG;
   const int G = Hq / Hkv;
@@ -900,6 +1029,7 @@ TFB_API int tfb_paged_decode(const void* q, long long ldq, void* k_data, void* k
   dim3 grid(B, Hkv, splits);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto Q = static_cast<const __nv_bfloat16*>(q);
+  auto out = static_cast<__nv_bfloat16*>(o);
   int rc;
   // tensor-core kernel by default (up to 8 query heads per kv head, q rows 16-byte aligned); TFB_PAGED_DECODE=simt
   // selects the CUDA-core kernel
@@ -907,9 +1037,9 @@ TFB_API int tfb_paged_decode(const void* q, long long ldq, void* k_data, void* k
   const bool mma_ok = !simt && G <= 8 && (ldq % 8) == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
 #define TFB_GO(MODE)                                                                                                  \
   rc = mma_ok ? ((D == 64) ? launch_decode_mma<MODE, 64>(grid, st, Q, ldq, kp, vp, block_table, max_pages, seq_lens, acc_ws, ml_ws, \
-                                                         Hq, Hkv, G, splits, scale, status)                           \
+                                                         Hq, Hkv, G, splits, scale, out, ldo, counts, status)         \
                            : launch_decode_mma<MODE, 128>(grid, st, Q, ldq, kp, vp, block_table, max_pages, seq_lens, acc_ws,       \
-                                                          ml_ws, Hq, Hkv, G, splits, scale, status))                  \
+                                                          ml_ws, Hq, Hkv, G, splits, scale, out, ldo, counts, status)) \
      : (D == 64) ? launch_decode_g<MODE, 64>(G, grid, st, Q, ldq, kp, vp, block_table, max_pages, seq_lens, acc_ws,   \
                                              ml_ws, Hq, Hkv, splits, scale)                                           \
                  : launch_decode_g<MODE, 128>(G, grid, st, Q, ldq, kp, vp, block_table, max_pages, seq_lens, acc_ws,  \
@@ -919,7 +1049,7 @@ TFB_API int tfb_paged_decode(const void* q, long long ldq, void* k_data, void* k
   else if (mode == KV_Q4) { TFB_GO(KV_Q4); }
   else return TFB_ERR_ARG;
 #undef TFB_GO
-  if (rc) return rc;
+  if (rc || mma_ok) return rc;
   tfb::launch_k_pdl(paged_combine_kernel, dim3(B, Hq), 128, 0, st, acc_ws, ml_ws, static_cast<__nv_bfloat16*>(o), ldo, Hq, D, splits);
   return int(cudaGetLastError());
 }

@@ -338,9 +338,7 @@ class InferenceEngine:
         for li, w in enumerate(m.layers):
             a, _ = _norm_fwd(mc, h, w.attention_norm, getattr(w, "attention_norm_bias", None))
             qkv = self._lin(a, li, "qkv", w.qkv, getattr(w, "qkv_bias", None))
-            if rope is not None:
-                F.rope_(qkv, rope[0], rope[1], Hq + Hkv, D, S, positions=positions)
-            self.cache.append(li, qkv, Hq * D, (Hq + Hkv) * D, slots)
+            self.cache.rope_append(li, qkv, rope, positions, Hq, slots)
             if pos0 == 0:
                 o, _ = F.attn_fwd(qkv, qkv, qkv, 1, S, Hq, Hkv, D, k_col0=Hq * D, v_col0=(Hq + Hkv) * D)
             else:
@@ -421,9 +419,7 @@ class InferenceEngine:
         for li, w in enumerate(m.layers):
             a, _ = _norm_fwd(mc, h, w.attention_norm, getattr(w, "attention_norm_bias", None))
             qkv = self._lin(a, li, "qkv", w.qkv, getattr(w, "qkv_bias", None))
-            if rope is not None:
-                F.rope_(qkv, rope[0], rope[1], Hq + Hkv, D, pack.rows, positions=positions)
-            self.cache.append(li, qkv, Hq * D, (Hq + Hkv) * D, slots)
+            self.cache.rope_append(li, qkv, rope, positions, Hq, slots)
             o = F.attn_fwd_packed(qkv, qkv, qkv, pack, Hq, Hkv, D, k_col0=Hq * D, v_col0=(Hq + Hkv) * D)
             if mc.use_parallel_residual:
                 attn = self._lin(o, li, "o", w.o, getattr(w, "o_bias", None))
@@ -486,9 +482,7 @@ class InferenceEngine:
         for li, w in enumerate(m.layers):
             a, _ = _norm_fwd(mc, h, w.attention_norm, getattr(w, "attention_norm_bias", None))
             qkv = self._lin(a, li, "qkv", w.qkv, getattr(w, "qkv_bias", None))
-            if rope is not None:
-                F.rope_(qkv, rope[0], rope[1], Hq + Hkv, D, 1, positions=positions)
-            self.cache.append(li, qkv, Hq * D, (Hq + Hkv) * D, slots)
+            self.cache.rope_append(li, qkv, rope, positions, Hq, slots)
             o = self.cache.decode(li, qkv[:, :Hq * D], block_table, lens, Hq)
             if mc.use_parallel_residual:
                 attn = self._lin(o, li, "o", w.o, getattr(w, "o_bias", None))

@@ -13,15 +13,16 @@ from typing import List, Optional
 
 import torch
 
-from ..ops import _lib
+from ..ops import _lib, functional as F
 from ..ops._lib import c_f, c_i, c_ll, c_p, check, ptr, stream
 
 PAGE = 16
 MODES = {"bf16": 0, "fp8": 1, "q4": 2}
 
 _lib.register("tfb_kv_append", [c_p, c_ll, c_i, c_i, c_p, c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_ll, c_p])
+_lib.register("tfb_kv_rope_append", [c_p, c_ll, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_ll, c_p])
 _lib.register("tfb_kv_gather", [c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_ll, c_i, c_i, c_i, c_ll, c_p])
-_lib.register("tfb_paged_decode", [c_p, c_ll, c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_ll, c_p, c_p, c_i, c_i, c_i,
+_lib.register("tfb_paged_decode", [c_p, c_ll, c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_ll, c_p, c_p, c_p, c_i, c_i, c_i,
                                    c_i, c_i, c_i, c_f, c_ll, c_p, c_p])
 
 
@@ -164,6 +165,18 @@ class PagedKVCache:
                                        kp.data.data_ptr(), ptr(kp.scale), vp.data.data_ptr(), ptr(vp.scale), T,
                                        self.Hkv, self.D, MODES[self.mode], self.num_pages * PAGE, stream()), "kv_append")
 
+    def rope_append(self, layer, qkv, rope, positions, Hq, slot_mapping):
+        """Rotate the q and k heads of the rows [q | k | v] in place (``rope``: cos and sin tables, or None) and append k and v."""
+        H, D = self.Hkv, self.D
+        if rope is None or not qkv.is_cuda:
+            if rope is not None:
+                F.rope_(qkv, rope[0], rope[1], Hq + H, D, qkv.shape[0], positions=positions)
+            return self.append(layer, qkv, Hq * D, (Hq + H) * D, slot_mapping)
+        kp, vp = self.k[layer], self.v[layer]
+        check(_lib.lib().tfb_kv_rope_append(qkv.data_ptr(), qkv.stride(0), rope[0].data_ptr(), rope[1].data_ptr(), positions.data_ptr(),
+                                            slot_mapping.data_ptr(), kp.data.data_ptr(), ptr(kp.scale), vp.data.data_ptr(), ptr(vp.scale), qkv.shape[0],
+                                            Hq, H, D, MODES[self.mode], self.num_pages * PAGE, stream()), "kv_rope_append")
+
     def gather(self, layer, pages, n):
         """The first ``n`` cached tokens of one sequence (``pages``: its page list, int32 tensor) as contiguous bf16 rows
         (k [n, Hkv*D], v [n, Hkv*D]), dequantised: the keys / values a prompt suffix attends over besides itself."""
@@ -206,14 +219,15 @@ class PagedKVCache:
         key = (B, Hq, splits)
         if key not in self._ws:
             self._ws[key] = (torch.empty(B * Hq * splits * D, dtype=torch.float32, device=q.device),
-                             torch.empty(B * Hq * splits * 2, dtype=torch.float32, device=q.device))
-        acc, ml = self._ws[key]
+                             torch.empty(B * Hq * splits * 2, dtype=torch.float32, device=q.device),
+                             torch.zeros(B * Hkv, dtype=torch.int32, device=q.device))
+        acc, ml, counts = self._ws[key]
         o = torch.empty((B, Hq * D), dtype=q.dtype, device=q.device)
         kp, vp = self.k[layer], self.v[layer]
         check(_lib.lib().tfb_paged_decode(q.data_ptr(), q.stride(0), kp.data.data_ptr(), ptr(kp.scale),
                                           vp.data.data_ptr(), ptr(vp.scale), block_table.data_ptr(),
                                           block_table.shape[1], seq_lens.data_ptr(), o.data_ptr(), o.stride(0),
-                                          acc.data_ptr(), ml.data_ptr(), B, Hq, Hkv, D, splits, MODES[self.mode],
+                                          acc.data_ptr(), ml.data_ptr(), counts.data_ptr(), B, Hq, Hkv, D, splits, MODES[self.mode],
                                           float(scale), self.num_pages * PAGE, _lib.status_word(q.device).data_ptr(),
-                                          stream()), "paged_decode", 2)
+                                          stream()), "paged_decode", 1 if Hq // Hkv <= 8 else 2)
         return o

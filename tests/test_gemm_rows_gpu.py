@@ -57,7 +57,8 @@ def test_few_rows_epilogue(M, N, K):
 
 
 @pytest.mark.parametrize("fmt,group", [("int8", 32), ("int8", 64), ("mxfp8", 32), ("int4", 32), ("fp4", 32), ("ternary", 64)])
-@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (5, 1000, 776), (16, 4096, 4096), (17, 1536, 512), (32, 512, 14336)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (5, 1000, 776), (16, 4096, 4096), (9, 28672, 512), (16, 512, 14336), (17, 1536, 512),
+                                   (32, 512, 14336)])
 def test_packed_rows(M, N, K, fmt, group):
     x, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
     bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
@@ -93,3 +94,22 @@ def test_rows_under_capture_and_on_streams():
     torch.cuda.synchronize()
     for o in outs:
         assert _rel(o, ref.double()) < 3e-3
+
+
+# 1408: skinny blocks of 8 + 8 columns, pairs of half tiles; 1000 and 8200: ragged tiles of 64 and 128 outputs, the up half right behind them;
+# 24: less than a tile; 14336 x 4096: several blocks per tile, several tiles per block
+@pytest.mark.parametrize("F_,K", [(1408, 512), (1000, 776), (8200, 264), (24, 64), (14336, 4096)])
+@pytest.mark.parametrize("M", [1, 16, 40, 64, 65, 128, 131, 600])
+def test_linear_glu(M, F_, K):
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(2 * F_, K, device="cuda") * K ** -0.5).bfloat16()
+    gu = x.double() @ w.double().t()
+    for act, fn in (("swiglu", torch.nn.functional.silu), ("geglu", lambda v: torch.nn.functional.gelu(v, approximate="tanh"))):
+        want = fn(gu[:, :F_]) * gu[:, F_:]
+        y = F.linear_glu(x, w, act)
+        torch.cuda.synchronize()
+        _lib.check_status()
+        e = _rel(y, want)
+        # one rounding to bf16 (2^-9 at most, 2^-9 / sqrt(3) on average); through a rounded product three of them
+        assert y.shape == (M, F_) and e < 4e-3
+        assert e <= 1.05 * _rel(F.glu_fwd(F.gemm(x, w), act), want)
+        assert torch.equal(y, F.linear_glu(x, w, act))

@@ -37,7 +37,8 @@ struct RowsPlan {
   static constexpr int TMEM_COLS = QUANT ? 512 : 2 * MP;
   static constexpr int RAW_OFF = STAGES * STAGE;
   static constexpr int BAR_OFF = RAW_OFF + RAW_STAGES * RW_RAW;
-  static constexpr int SMEM = BAR_OFF + 512 + 1024;
+  static constexpr int EX_OFF = BAR_OFF + 512;      // 16 rows of x by 64 "up" columns on their way to the "gate" lanes
+  static constexpr int SMEM = EX_OFF + (QUANT ? 0 : 4096) + 1024;
   static constexpr int THREADS = QUANT ? 768 : 256;
   static_assert(2 * MP + (QUANT ? 32 * STAGES : 0) <= 512, "tensor memory");
   static_assert(SMEM <= 232448, "shared memory");
@@ -52,6 +53,7 @@ struct RowsParams {
   long long ldr;
   float alpha;
   int act, out_f32, w_static;
+  int glu;                             // > 0: a tile is 64 rows of W and the 64 rows `glu` further on; out = act(first) * second
   const uint8_t* codes;                // packed weights: tile-major codes and scales
   const __nv_bfloat16* scales;
   int group;
@@ -137,7 +139,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
   } else if (warp == 2) {
     if (lane == 0) {
       if (!p.w_static) pdl_wait();
-      int s = 0, kb = kb_first, row = u0 / p.KB * RW_BN;
+      const int rows_w = p.glu ? RW_BN / 2 : RW_BN;
+      int s = 0, kb = kb_first, row = u0 / p.KB * rows_w;
       uint32_t ph = 1;
       if constexpr (QUANT) {
         constexpr uint32_t code_bytes = 128 * wq_row_bytes(QUANT ? FMT : 0);
@@ -156,8 +159,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
         for (int i = 0; i < n; ++i) {
           if (!mbar_wait(bar_empty + s * 8, ph, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { drain(); break; }
           mbar_expect_tx(bar_full + s * 8, RW_W_BYTES);
-          tma_load_2d(base + s * L::STAGE + L::X_BYTES, &tma_w, bar_full + s * 8, kb * RW_BK, row);
-          if (++kb == p.KB) { kb = 0; row += RW_BN; }
+          const uint32_t sw = base + s * L::STAGE + L::X_BYTES;
+          tma_load_2d(sw, &tma_w, bar_full + s * 8, kb * RW_BK, row);
+          if (p.glu) tma_load_2d(sw + RW_W_BYTES / 2, &tma_w, bar_full + s * 8, kb * RW_BK, p.glu + row);
+          if (++kb == p.KB) { kb = 0; row += rows_w; }
           if (++s == S) { s = 0; ph ^= 1; }
         }
       }
@@ -231,8 +236,24 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
   } else if (warp >= 4) {
     // ------------------------------ epilogue: lane = weight row of the tile, columns = rows of x ------------------------------
     const int quad = warp & 3, nl = quad * 32 + lane;
-    // sixteen rows of x from row c on: the residual's loads are in flight together
-    auto finish = [&](const float (&acc)[16], int c, int n, float bias) {
+    float* ex = reinterpret_cast<float*>(smem + L::EX_OFF);
+    // sixteen rows of x from row c on: the residual's loads are in flight together.  All 128 lanes call it.
+    auto finish = [&](const float (&acc)[16], int c, int n, float bias, bool live) {
+      if (!QUANT && p.glu) {
+        if (nl >= 64) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) ex[j * 64 + nl - 64] = acc[j];
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (nl < 64 && live) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < p.M) static_cast<__nv_bfloat16*>(p.C)[(c + j) * p.ldc + n] = __float2bfloat16(apply_act(acc[j], p.act) * ex[j * 64 + nl]);
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        return;
+      }
+      if (!live) return;
       float v[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = fmaf(acc[j], p.alpha, bias);
@@ -261,7 +282,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
     for (int u = u0; u < u1; ++seg) {
       const int t = u / p.KB, kb0 = u - t * p.KB, end = min(u1, (t + 1) * p.KB), ab = seg & 1;
       const bool whole = kb0 == 0 && end == (t + 1) * p.KB;
-      const int n = t * RW_BN + nl;
+      const int n = p.glu ? t * (RW_BN / 2) + (nl & 63) : t * RW_BN + nl;
       const bool live = n < p.N;
       const float bias = p.bias && live ? __bfloat162float(p.bias[n]) : 0.f;
       if (!mbar_wait_sleep_warp(bar_tfull + ab * 8, (seg >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL, 20)) break;
@@ -279,8 +300,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
         if (!whole) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) __stcg(slot + (c / 4 + j) * 128, make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]));
-        } else if (live) {
-          finish(f, c, n, bias);
+        } else {
+          finish(f, c, n, bias, live);
         }
       }
       tc_fence_before();
@@ -298,7 +319,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (*last_flag) {
           __threadfence();
-          if (live) {
+          {
             // only the first block can have the tile in its second slot: every later one starts inside the tile
             const long long first = (int(c0 * U / G) / p.KB == t ? 0 : 1);
             const float4* src0 = reinterpret_cast<const float4*>(p.ws) + nl;
@@ -332,7 +353,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
                   f[4 * j + 2] = v[4 * h + j].z;
                   f[4 * j + 3] = v[4 * h + j].w;
                 }
-                if (c + h * 16 < p.M) finish(f, c + h * 16, n, bias);
+                if (c + h * 16 < p.M) finish(f, c + h * 16, n, bias, live);
               }
             }
           }
@@ -423,19 +444,21 @@ static int launch_rows_m(int M, const CUtensorMap& tx, const CUtensorMap& tw, co
   else return launch_rows<FMT, 128>(tx, tw, p, grid, st);
 }
 
-int gemm_rows(const void* x, long long ldx, const void* W, long long ldw, const void* codes, const void* scales, int fmt, int group, void* C,
-              long long ldc, int M, int N, int K, int Kw, const void* bias, const void* residual, long long ldr, float alpha, int act, int out_f32,
-              int w_static, int* status, void* stream) {
+static int run_rows(const void* x, long long ldx, const void* W, long long ldw, const void* codes, const void* scales, int fmt, int group, void* C,
+                    long long ldc, int M, int N, int K, int Kw, const void* bias, const void* residual, long long ldr, float alpha, int act,
+                    int out_f32, int glu, int w_static, int* status, void* stream) {
   if (M <= 0 || M > RW_MAX_M || N <= 0 || K <= 0) return TFB_NOT_TAKEN;
   RowsParams p = {};
   p.M = M; p.N = N; p.K = K;
   p.KB = ((fmt >= 0 ? Kw : K) + RW_BK - 1) / RW_BK;
-  p.tiles = (N + RW_BN - 1) / RW_BN;
+  const int rows_w = glu ? RW_BN / 2 : RW_BN;      // outputs of a tile
+  p.tiles = (N + rows_w - 1) / rows_w;
+  p.glu = glu;
   if (p.tiles > RW_MAX_TILES || (long long)p.tiles * p.KB > 0x7fffffffll / RW_MAX_CTAS) return TFB_NOT_TAKEN;
   CUtensorMap tx, tw;
   const int mp = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   if (make_tmap_2d(&tx, x, 2, K, M, ldx * 2, RW_BK, mp)) return TFB_NOT_TAKEN;
-  if (fmt < 0 && make_tmap_2d(&tw, W, 2, K, N, ldw * 2, RW_BK, RW_BN)) return TFB_NOT_TAKEN;
+  if (fmt < 0 && make_tmap_2d(&tw, W, 2, K, glu ? 2 * N : N, ldw * 2, RW_BK, rows_w)) return TFB_NOT_TAKEN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   RowsWs w;
   if (!rows_workspace(st, &w)) return TFB_NOT_TAKEN;
@@ -460,6 +483,17 @@ int gemm_rows(const void* x, long long ldx, const void* W, long long ldw, const 
     case 4: return launch_rows_m<4>(M, tx, tx, p, grid, st);
     default: return TFB_NOT_TAKEN;
   }
+}
+
+int gemm_rows(const void* x, long long ldx, const void* W, long long ldw, const void* codes, const void* scales, int fmt, int group, void* C,
+              long long ldc, int M, int N, int K, int Kw, const void* bias, const void* residual, long long ldr, float alpha, int act, int out_f32,
+              int w_static, int* status, void* stream) {
+  return run_rows(x, ldx, W, ldw, codes, scales, fmt, group, C, ldc, M, N, K, Kw, bias, residual, ldr, alpha, act, out_f32, 0, w_static, status, stream);
+}
+
+int gemm_rows_glu(const void* x, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int F, int K, int act, int w_static,
+                  int* status, void* stream) {
+  return run_rows(x, ldx, W, ldw, nullptr, nullptr, -1, 0, C, ldc, M, F, K, K, nullptr, nullptr, 0, 1.f, act, 0, F, w_static, status, stream);
 }
 
 }  // namespace tfb

@@ -7,6 +7,7 @@
 #include "tfb_elem.cuh"
 #include "tfb_host.h"
 #include "tfb_mma.cuh"
+#include "tfb_ptx.cuh"
 
 namespace tfb {
 
@@ -25,6 +26,7 @@ struct SkinnyArgs {
   const __nv_bfloat16* residual;    // [M, ldr] or null, added last
   long long ldr;
   float alpha;
+  int glu;                          // > 0: out = act(x . W[n]^T) * (x . W[glu + n]^T), N of them; a block takes 8 columns of each half
 };
 
 struct Row16 { uint32_t u[8]; };      // 16 consecutive entries of a row
@@ -43,20 +45,22 @@ __global__ void __launch_bounds__(SK_WARPS * 32) skinny_linear_kernel(const Skin
   tfb::pdl_sync();
   __shared__ float red[SK_WARPS][MT * 16][SK_N + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
-  const int n0 = blockIdx.x * SK_N, h = blockIdx.y, m0 = blockIdx.z * MT * 16, M = min(MT * 16, p.M - m0);
+  const int cols = p.glu ? SK_N / 2 : SK_N, n0 = blockIdx.x * cols, h = blockIdx.y, m0 = blockIdx.z * MT * 16, M = min(MT * 16, p.M - m0);
   float acc[MT][2][4];
 #pragma unroll
   for (int m = 0; m < MT; ++m)
 #pragma unroll
     for (int n = 0; n < 2; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f;
   const __nv_bfloat16* w0 = p.w + ((long long)h * p.N + n0 + g) * p.ldw;
+  const long long second = (p.glu ? p.glu : 8) * p.ldw;                     // the other 8 rows of W
+  const bool live0 = n0 + g < p.N, live1 = n0 + (p.glu ? 0 : 8) + g < p.N;
   const __nv_bfloat16* x0 = p.x + (m0 + g) * p.ldx + (long long)h * p.x_head;
 #pragma unroll 2
   for (int k0 = warp * 64; k0 < p.K; k0 += SK_WARPS * 64) {
     const int k = k0 + q * 16;
     Row16 b[2];
 #pragma unroll
-    for (int n = 0; n < 2; ++n) b[n] = load16(w0 + n * 8 * p.ldw, k, p.K, n0 + n * 8 + g < p.N);
+    for (int n = 0; n < 2; ++n) b[n] = load16(w0 + n * second, k, p.K, n ? live1 : live0);
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
       const Row16 a0 = load16(x0 + m * 16 * p.ldx, k, p.K, m * 16 + g < M), a1 = load16(x0 + (m * 16 + 8) * p.ldx, k, p.K, m * 16 + 8 + g < M);
@@ -75,6 +79,20 @@ __global__ void __launch_bounds__(SK_WARPS * 32) skinny_linear_kernel(const Skin
 #pragma unroll
       for (int e = 0; e < 4; ++e) red[warp][m * 16 + g + (e >> 1) * 8][n * 8 + q * 2 + (e & 1)] = acc[m][n][e];
   __syncthreads();
+  if (p.glu) {
+    for (int i = threadIdx.x; i < MT * 16 * 8; i += SK_WARPS * 32) {
+      const int m = i / 8, n = i % 8;
+      if (m >= M || n0 + n >= p.N) continue;
+      float a = 0.f, u = 0.f;
+#pragma unroll
+      for (int w = 0; w < SK_WARPS; ++w) {
+        a += red[w][m][n];
+        u += red[w][m][n + 8];
+      }
+      static_cast<__nv_bfloat16*>(p.out)[(m0 + m) * p.ldo + n0 + n] = __float2bfloat16(apply_act(a, p.act) * u);
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < MT * 16 * SK_N; i += SK_WARPS * 32) {
     const int m = i / SK_N, n = i % SK_N;
     if (m >= M || n0 + n >= p.N) continue;
@@ -108,8 +126,9 @@ static int launch_skinny(const tfb::SkinnyArgs& p, int heads, int rows, void* st
       (reinterpret_cast<uintptr_t>(p.x) & 15) || (reinterpret_cast<uintptr_t>(p.w) & 15))
     return TFB_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (rows == 0) rows = p.M <= 16 || tfb_skinny_work(p.M, p.N * heads, p.K) <= 1500000 ? 16 : 32;
-  const dim3 grid((p.N + SK_N - 1) / SK_N, heads, (p.M + rows - 1) / rows);
+  if (rows == 0) rows = p.M <= 16 || tfb_skinny_work(p.M, (p.glu ? 2ll : 1ll) * p.N * heads, p.K) <= 1500000 ? 16 : 32;
+  const int cols = p.glu ? SK_N / 2 : SK_N;
+  const dim3 grid((p.N + cols - 1) / cols, heads, (p.M + rows - 1) / rows);
   if (rows == 16) launch_k_pdl(skinny_linear_kernel<1>, grid, SK_WARPS * 32, 0, st, p);
   else if (rows == 32) launch_k_pdl(skinny_linear_kernel<2>, grid, SK_WARPS * 32, 0, st, p);
   else if (rows == 64) launch_k_pdl(skinny_linear_kernel<4>, grid, SK_WARPS * 32, 0, st, p);
@@ -127,7 +146,15 @@ int tfb::gemm_skinny(const void* x, long long ldx, const void* W, long long ldw,
   if (M <= 0 || N <= 0 || K <= 0 || K % 8 || ldx % 8 || ldw % 8 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(W) & 15))
     return TFB_NOT_TAKEN;
   return launch_skinny(SkinnyArgs{static_cast<const bf16*>(x), static_cast<const bf16*>(W), ldx, ldw, C, ldc, M, N, K, act, out_f32, 0, 0, nullptr, 0,
-                                  static_cast<const bf16*>(bias), static_cast<const bf16*>(residual), ldr, alpha}, 1, 0, stream);
+                                  static_cast<const bf16*>(bias), static_cast<const bf16*>(residual), ldr, alpha, 0}, 1, 0, stream);
+}
+
+int tfb::gemm_skinny_glu(const void* x, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int F, int K, int act, void* stream) {
+  if (M <= 0 || M > 64 || F <= 0 || K <= 0 || K % 8 || ldx % 8 || ldw % 8 || (reinterpret_cast<uintptr_t>(x) & 15) ||
+      (reinterpret_cast<uintptr_t>(W) & 15) || tfb_skinny_work(M, 2ll * F, K) > 700000)
+    return TFB_NOT_TAKEN;
+  return launch_skinny(SkinnyArgs{static_cast<const bf16*>(x), static_cast<const bf16*>(W), ldx, ldw, C, ldc, M, F, K, act, 0, 0, 0, nullptr, 0, nullptr,
+                                  nullptr, 0, 1.f, F}, 1, 0, stream);
 }
 
 // 1 where the few-row form is the one to take.  Measured against the tcgen05 form (with its split-K finalize): it wins while a warp's share
@@ -141,7 +168,7 @@ TFB_API int tfb_skinny_linear(const void* x, long long ldx, const void* w, long 
                               int out_f32, int rows, const void* bias, void* stream) {
   if (M > 64 || (act != 0 && act != 4)) return TFB_ERR_ARG;
   return launch_skinny(tfb::SkinnyArgs{static_cast<const bf16*>(x), static_cast<const bf16*>(w), ldx, ldw, out, ldo, M, N, K, act, out_f32, 0, 0,
-                                       nullptr, 0, static_cast<const bf16*>(bias), nullptr, 0, 1.f}, 1, rows, stream);
+                                       nullptr, 0, static_cast<const bf16*>(bias), nullptr, 0, 1.f, 0}, 1, rows, stream);
 }
 
 // One product per head: x [M, ldx] (x_head entries between heads), w: heads blocks [N, K] stacked on the rows, out [M, ldo] (N entries per
@@ -149,5 +176,5 @@ TFB_API int tfb_skinny_linear(const void* x, long long ldx, const void* w, long 
 TFB_API int tfb_skinny_linear_heads(const void* x, long long ldx, int x_head, const void* w, long long ldw, void* out, long long ldo, const void* gate,
                                     long long ldg, int M, int heads, int N, int K, int rows, void* stream) {
   return launch_skinny(tfb::SkinnyArgs{static_cast<const bf16*>(x), static_cast<const bf16*>(w), ldx, ldw, out, ldo, M, N, K, 0, 0, x_head, N,
-                                       static_cast<const bf16*>(gate), ldg, nullptr, nullptr, 0, 1.f}, heads, rows, stream);
+                                       static_cast<const bf16*>(gate), ldg, nullptr, nullptr, 0, 1.f, 0}, heads, rows, stream);
 }

@@ -49,6 +49,10 @@ int gemm_rows(const void* x, long long ldx, const void* W, long long ldw, const 
               int w_static, int* status, void* stream);
 int gemm_skinny(const void* x, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int N, int K, const void* bias,
                 const void* residual, long long ldr, float alpha, int act, int out_f32, void* stream);
+// out [M, F] = act(x . W[0..F)^T) * (x . W[F..2F)^T)
+int gemm_rows_glu(const void* x, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int F, int K, int act, int w_static,
+                  int* status, void* stream);
+int gemm_skinny_glu(const void* x, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int F, int K, int act, void* stream);
 
 // Launch of a kernel of this library: same meaning as kernel<<<grid, block, smem, stream>>>(args...), plus the launch
 // attribute that lets the kernel's CTAs be placed while the previous kernel of the stream drains (each kernel starts with

@@ -270,7 +270,10 @@ class InferenceEngine:
             if mc.variant.upper() == "RESIDUAL_MOE":
                 y = y + f
             return base + y
-        gu = self._lin(f, li, "gate_up", w.gate_up, getattr(w, "gate_up_bias", None))
+        bias = getattr(w, "gate_up_bias", None)
+        if mc.gated and bias is None and f"layers.{li}.gate_up" not in self.packed:
+            return self._lin(F.linear_glu(f, w.gate_up.data, mc.act_kernel), li, "down", w.down, getattr(w, "down_bias", None), base)
+        gu = self._lin(f, li, "gate_up", w.gate_up, bias)
         act = F.glu_fwd(gu, mc.act_kernel) if mc.gated else F.act_fwd(gu, mc.act_kernel)
         return self._lin(act, li, "down", w.down, getattr(w, "down_bias", None), base)
 

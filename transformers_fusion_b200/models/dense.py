@@ -164,8 +164,11 @@ def block_forward(cfg: TransformerConfig, w, h_in, B, S, rope, save: bool):
     else:
         h_mid = F.gemm(o, w.o, bias=w.o_bias, residual=h_in)
         f, st2 = _norm_fwd(cfg, h_mid, w.ffn_norm, w.ffn_norm_bias)
-    gu = F.gemm(f, w.gate_up, bias=w.gate_up_bias)
-    act = F.glu_fwd(gu, cfg.act_kernel) if cfg.gated else F.act_fwd(gu, cfg.act_kernel)
+    if cfg.gated and not save and w.gate_up_bias is None:
+        gu, act = None, F.linear_glu(f, w.gate_up.data, cfg.act_kernel)
+    else:
+        gu = F.gemm(f, w.gate_up, bias=w.gate_up_bias)
+        act = F.glu_fwd(gu, cfg.act_kernel) if cfg.gated else F.act_fwd(gu, cfg.act_kernel)
     h_out = F.gemm(act, w.down, bias=w.down_bias, residual=h_mid)
     if cfg.use_parallel_residual:
         h_out = h_out + attn_out if not h_out.is_cuda else _add(h_out, attn_out)

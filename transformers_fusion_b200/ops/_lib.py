@@ -25,6 +25,8 @@ c_f = C.c_float
 _SIGS = {
     "tfb_sm_count": [],
     "tfb_gemm_bf16_static": [c_p, c_ll, c_p, c_ll, c_p, c_ll, c_i, c_i, c_i, c_p, c_p, c_ll, c_i, c_p, c_p],
+    "tfb_skinny_wq": [c_p, c_ll, c_p, c_p, c_i, c_i, c_p, c_ll, c_i, c_i, c_i, c_i, c_p, c_p, c_ll, c_i, c_p],
+    "tfb_gemm_glu": [c_p, c_ll, c_p, c_ll, c_p, c_ll, c_i, c_i, c_i, c_i, c_i, c_p, c_p],
     "tfb_gemm_rows": [c_p, c_ll, c_p, c_ll, c_p, c_ll, c_i, c_i, c_i, c_p, c_p, c_ll, c_f, c_i, c_i, c_i, c_p, c_p],
     "tfb_gemm_rows_wq": [c_p, c_ll, c_p, c_p, c_i, c_i, c_p, c_ll, c_i, c_i, c_i, c_i, c_p, c_p, c_ll, c_i, c_p, c_p],
     "tfb_gemm_bf16": [c_p, c_ll, c_i, c_p, c_ll, c_i, c_p, c_ll, c_i, c_i, c_i, c_p, c_p, c_ll, c_f, c_i, c_i, c_i, c_p, c_p],

@@ -268,6 +268,21 @@ def glu_fwd(x, act="silu", rows=None):
     return out
 
 
+def linear_glu(x, w, act="silu"):
+    """glu_fwd(linear(x, w), act) for w [2F, K] = [gate | up], in one kernel where its shape allows: the product [M, 2F] does not go through memory
+    and is not rounded before the activation.  As for ``linear``, the kernel launched just before must not write w."""
+    (M, K), F2 = x.shape, w.shape[0]
+    if x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and x.stride(-1) == w.stride(-1) == 1 and F2 % 2 == 0 and ACT[act] > 0:
+        assert w.shape[1] == K
+        out = torch.empty((M, F2 // 2), dtype=x.dtype, device=x.device)
+        rc = _lib.lib().tfb_gemm_glu(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), F2 // 2, M, F2 // 2, K, ACT[act], 1,
+                                     _lib.status_word(x.device).data_ptr(), stream())
+        if rc != -1:                # -1: not taken
+            check(rc, "linear_glu")
+            return out
+    return glu_fwd(linear(x, w), act)
+
+
 def glu_bwd(x, dout, act="silu", rows=None):
     M, F2 = x.shape
     Fh = F2 // 2

@@ -167,14 +167,16 @@ def dequant_bf16(pw: PackedWeight) -> torch.Tensor:
 _SPLIT_WS = {}
 
 
-ROWS_M = 32       # up to here (decode) the streaming form of gemm_rows.cu: one launch with bias and residual inside.  Measured, us, int8 codes, against
-                  # the split form with its finalize: 28672 x 4096 at 1 / 32 rows 49 / 51 against 57 / 62, 4096 x 14336 28.6 / 30.6 against 29.9 /
-                  # 33.3, 6144 x 4096 16.2 / 17.5 against 16.4 / 19.4; at 64 rows 4096 x 4096 20.3 against 17.3
+ROWS_M = 32       # up to here (decode) one launch with bias and residual inside: skinny_wq.cu up to 8 rows, and up to 16 while x is short
+SKINNY_K = 8192   # (K <= 8192: every block reads all of x), else the streaming form of gemm_rows.cu.  Measured, us, int8 codes: gemm_rows against the
+                  # split form with its finalize, 28672 x 4096 at 1 / 32 rows 49 / 51 against 57 / 62, 4096 x 14336 28.6 / 30.6 against 29.9 / 33.3; at
+                  # 64 rows 4096 x 4096 20.3 against 17.3.  skinny_wq against gemm_rows at 8 / 16 rows: 28672 x 4096 34 / 46 against 49, 4096 x
+                  # 14336 23 / 32 against 28
 
 
 def gemm_wq(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor] = None, splits: int = 0,
             out: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None, w_static: bool = False) -> torch.Tensor:
-    """y [M, N] = x [M, K] @ dequant(pw)^T (+ bias) (+ residual).  bf16 in / out.  M <= 32 (decode): streaming kernel; M < 2048:
+    """y [M, N] = x [M, K] @ dequant(pw)^T (+ bias) (+ residual).  bf16 in / out.  M <= 32 (decode): one launch (skinny_wq.cu, gemm_rows.cu); M < 2048:
     fused-dequant kernel with 128-row tiles; larger: bf16 image in scratch + bf16 GEMM.
     ``out`` [M, N] bf16: where the result goes (e.g. the staging buffer of a collective).  ``w_static``: the kernel launched just before does not
     write the packed weight (it may then be fetched ahead of that kernel's end)."""
@@ -192,7 +194,7 @@ def gemm_wq(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor] = No
 
 
 def _gemm_rows(x, pw, bias, residual, dst, w_static):
-    """The streaming form; None where its operands' layout does not fit it."""
+    """The one-launch forms; None where the operands' layout does not fit them."""
     M, K = x.shape
     if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or M < 1:
         return None
@@ -201,9 +203,12 @@ def _gemm_rows(x, pw, bias, residual, dst, w_static):
     if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != pw.N):
         return None
     out = dst if dst is not None and dst.dtype == torch.bfloat16 and dst.stride(-1) == 1 else torch.empty((M, pw.N), dtype=x.dtype, device=x.device)
-    rc = _lib.lib().tfb_gemm_rows_wq(x.data_ptr(), x.stride(0), pw.codes.data_ptr(), pw.scales.data_ptr(), pw.fmt, pw.group, out.data_ptr(),
-                                     out.stride(0), M, pw.N, K, pw.Kp, ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
-                                     int(w_static), _lib.status_word(x.device).data_ptr(), stream())
+    args = (x.data_ptr(), x.stride(0), pw.codes.data_ptr(), pw.scales.data_ptr(), pw.fmt, pw.group, out.data_ptr(), out.stride(0), M, pw.N, K, pw.Kp,
+            ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0, int(w_static))
+    if (M <= 8 or (M <= 16 and K <= SKINNY_K)) and K % 8 == 0:
+        rc = _lib.lib().tfb_skinny_wq(*args, stream())
+    else:
+        rc = _lib.lib().tfb_gemm_rows_wq(*args, _lib.status_word(x.device).data_ptr(), stream())
     if rc == -1:                     # not taken
         return None
     check(rc, "gemm_rows_wq")

@@ -113,3 +113,17 @@ def test_linear_glu(M, F_, K):
         assert y.shape == (M, F_) and e < 4e-3
         assert e <= 1.05 * _rel(F.glu_fwd(F.gemm(x, w), act), want)
         assert torch.equal(y, F.linear_glu(x, w, act))
+
+
+@pytest.mark.parametrize("B,S", [(1, 5), (2, 200)])
+def test_scoring_without_gradients_matches_the_training_forward(B, S):
+    """Without a gradient mode the blocks keep nothing and gate in the product; the logits are those of the pass that keeps everything."""
+    from transformers_fusion_b200.models.config import TransformerConfig
+    from transformers_fusion_b200.models.dense import DenseModel
+    cfg = TransformerConfig(vocab_size=512, hidden_size=256, num_layers=2, num_heads=4, num_kv_heads=2, ffn_hidden_size=704, max_seq_len=256)
+    m = DenseModel(cfg, device="cuda", dtype=torch.bfloat16, seed=0)
+    ids = torch.randint(0, 512, (B, S), device="cuda")
+    a = m(ids)
+    with torch.no_grad():
+        b = m(ids)
+    assert a.requires_grad and not b.requires_grad and _rel(b, a.detach().double()) < 1e-2       # a few bf16 roundings per layer

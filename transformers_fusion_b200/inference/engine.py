@@ -634,6 +634,8 @@ class InferenceEngine:
         """Append one token to every sequence and return the logits [len(reqs), V] at it.  ``pending[i]`` >= 0: the token of row
         i is row pending[i] of ``prev_tokens`` (on the device) instead of host_tokens[i]."""
         dev, alloc = self.device, self.cache.allocator
+        if len(reqs) > self._bucket(self.cfg.max_batch):
+            raise ValueError(f"{len(reqs)} sequences do not fit into a batch of {self.cfg.max_batch}")
         for r in reqs:
             if r.pos // PAGE >= len(r.pages):
                 r.pages.append(alloc.alloc())

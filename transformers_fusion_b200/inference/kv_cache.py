@@ -213,9 +213,12 @@ class PagedKVCache:
             return out.to(q.dtype)
         if splits is None:
             max_len = block_table.shape[1] * PAGE
-            # enough CTAs (128 threads each) for about eight per SM: the kernel is latency-bound per CTA (one K row per
-            # thread, then a serial walk over the tile's V rows), so parallelism across CTAs is what hides it
-            splits = max(1, min(16, (8 * 148) // max(1, B * Hkv), max_len // 128))
+            # as many blocks as run at once (three per SM at heads of 128, four at 64), each over 128 tokens at least (its four warps
+            # take 32 at a time); powers of two, so that few splits end in a partly filled round.  Measured, us, for 1 / 2 / 4 / 8 / 16
+            # splits: 64 sequences of 180 tokens, 8 kv heads of 128 18.5 / 28.3 / 38.0 / 65.3 / 110; 8 of 2200 64.8 / 38.5 / 28.3 / 32.5 / 37.2
+            # (fp8 84 / 48 / 33 / 38 / 49); 4 of 2000 82 / 47 / 27 / 24 / 28; 16 of 300, 8 heads of 64 12.9 / 9.8 / 8.2 / 13.3 / 20.8
+            splits = max(1, min(16, (3 if D == 128 else 4) * 148 // max(1, B * Hkv), max_len // 128))
+            splits = 1 << (splits.bit_length() - 1)
         key = (B, Hq, splits)
         if key not in self._ws:
             self._ws[key] = (torch.empty(B * Hq * splits * D, dtype=torch.float32, device=q.device),

@@ -147,8 +147,9 @@ class BlockCtx:
     __slots__ = ("h_in", "st1", "a", "qkv", "o", "lse", "h_mid", "st2", "f", "gu", "act", "B", "S")
 
 
-def block_forward(cfg: TransformerConfig, w, h_in, B, S, rope, save: bool):
-    """One transformer block on the flattened token stream h_in [T, H].  Returns (h_out, ctx)."""
+def block_forward(cfg: TransformerConfig, w, h_in, B, S, rope, save: bool, no_grad: bool = False):
+    """One transformer block on the flattened token stream h_in [T, H].  Returns (h_out, ctx).  ``no_grad``: no backward pass will follow,
+    not even one that runs this block again (which has to see the values that this pass has seen)."""
     Hq, Hkv, D = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
     ctx = BlockCtx() if save else None
     a, st1 = _norm_fwd(cfg, h_in, w.attention_norm, w.attention_norm_bias)
@@ -164,7 +165,7 @@ def block_forward(cfg: TransformerConfig, w, h_in, B, S, rope, save: bool):
     else:
         h_mid = F.gemm(o, w.o, bias=w.o_bias, residual=h_in)
         f, st2 = _norm_fwd(cfg, h_mid, w.ffn_norm, w.ffn_norm_bias)
-    if cfg.gated and not save and w.gate_up_bias is None:
+    if cfg.gated and no_grad and not save and w.gate_up_bias is None:
         gu, act = None, F.linear_glu(f, w.gate_up.data, cfg.act_kernel)
     else:
         gu = F.gemm(f, w.gate_up, bias=w.gate_up_bias)
@@ -223,9 +224,9 @@ class _BlockFn(torch.autograd.Function):
     """Autograd node for a whole block (used when the model is driven by torch autograd)."""
 
     @staticmethod
-    def forward(ctx, h_in, blk, B, S, rope, recompute, *params):
-        need = any(ctx.needs_input_grad)
-        h_out, bctx = block_forward(blk.cfg, blk, h_in, B, S, rope, save=need and not recompute)
+    def forward(ctx, h_in, blk, B, S, rope, recompute, grad, *params):
+        need = grad and any(ctx.needs_input_grad)      # which weights want gradients is true without a gradient mode as well
+        h_out, bctx = block_forward(blk.cfg, blk, h_in, B, S, rope, save=need and not recompute, no_grad=not need)
         ctx.blk, ctx.bctx, ctx.rope, ctx.recompute = blk, bctx, rope, recompute
         if recompute:
             ctx.saved_h, ctx.BS = h_in, (B, S)
@@ -241,7 +242,7 @@ class _BlockFn(torch.autograd.Function):
             _, bctx = block_forward(blk.cfg, blk, ctx.saved_h, ctx.BS[0], ctx.BS[1], ctx.rope, save=True)
         dh_in = block_backward(blk.cfg, blk, bctx, dh_out.contiguous(), ctx.rope)
         ctx.bctx = None
-        return (dh_in, None, None, None, None, None) + (None,) * len(list(blk.parameters()))
+        return (dh_in, None, None, None, None, None, None) + (None,) * len(list(blk.parameters()))
 
 
 # =================================================================================================
@@ -442,7 +443,7 @@ class DenseModel(nn.Module):
         rope = self.rope(ids.device)
         h = _EmbedFn.apply(ids, self, self.tok_embeddings)
         for blk in self.layers:
-            h = _BlockFn.apply(h, blk, B, S, rope, self.activation_checkpointing, *blk.parameters())
+            h = _BlockFn.apply(h, blk, B, S, rope, self.activation_checkpointing, torch.is_grad_enabled(), *blk.parameters())
         return _FinalNormFn.apply(h, self, self.norm)
 
     def forward(self, ids):

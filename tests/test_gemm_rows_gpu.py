@@ -127,3 +127,42 @@ def test_scoring_without_gradients_matches_the_training_forward(B, S):
     with torch.no_grad():
         b = m(ids)
     assert a.requires_grad and not b.requires_grad and _rel(b, a.detach().double()) < 1e-2       # a few bf16 roundings per layer
+
+
+def test_a_block_that_gives_up_leaves_the_counters_clear():
+    """The bounds-check library lets one block's epilogue give up as if its wait had run out: the status word says so, and the products that
+    follow (same and other shapes over the same counters) are right.  In a child process, because the library is chosen at load time."""
+    import os
+    import subprocess
+    import sys
+    code = r'''
+import torch
+from transformers_fusion_b200.ops import _lib, functional as F
+_lib.register("tfb_test_rows_give_up", [_lib.c_i])
+shapes = [(8, 4096, 4096), (3, 6144, 4096), (16, 28672, 512), (40, 8192, 2048)]
+ops = [(torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()) for M, N, K in shapes]
+def product(x, w):
+    out = torch.full((x.shape[0], w.shape[0]), float("nan"), device="cuda")
+    _lib.check(_lib.lib().tfb_gemm_rows(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), x.shape[0], w.shape[0],
+                                        x.shape[1], None, None, 0, 1.0, 0, 1, 0, _lib.status_word().data_ptr(), _lib.stream()), "gemm_rows")
+    return out
+good = [product(x, w) for x, w in ops]
+_lib.check_status()
+for cta in (0, 3, 147):
+    for x, w in ops:
+        _lib.lib().tfb_test_rows_give_up(cta)
+        product(x, w)
+        _lib.lib().tfb_test_rows_give_up(-1)
+        try:
+            _lib.check_status()
+            raise SystemExit("no status")
+        except _lib.KernelError:
+            pass
+        for (a, b), want in zip(ops, good):
+            assert torch.equal(product(a, b), want)
+        _lib.check_status()
+print("ok")
+'''
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=root, env=dict(os.environ, TFB_BOUNDS_CHECK="1"))
+    assert r.returncode == 0 and "ok" in r.stdout, r.stdout[-1500:] + r.stderr[-1500:]

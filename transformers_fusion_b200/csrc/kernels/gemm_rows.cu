@@ -60,7 +60,21 @@ struct RowsParams {
   float* ws;                           // [grid][2][MP][128] partial sums
   int* count;                          // [tiles] arrivals, zero between launches
   int* status;
+#ifdef TFB_BOUNDS_CHECK
+  int give_up;                         // block whose epilogue behaves as if its first wait had run out; -1: none
+#endif
 };
+
+// The vote of the 128 epilogue threads (barrier 1): all of them or none go on.
+__device__ __forceinline__ bool all_of_128(bool ok) {
+  int r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 1, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(int(ok))
+      : "memory");
+  return r != 0;
+}
 
 template <int FMT, int MP>
 __global__ void __launch_bounds__(RowsPlan<FMT, MP>::THREADS, 1)
@@ -278,6 +292,16 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
           if (c + j < p.M) static_cast<__nv_bfloat16*>(p.C)[(c + j) * p.ldc + n] = __float2bfloat16(v[j]);
       }
     };
+    // blocks that share tile t: the ones whose runs hold its first and its last unit, and those in between
+    auto first_of = [&](int t) { return int((((long long)t * p.KB + 1) * G - 1) / U); };
+    auto last_of = [&](int t) { return int(((long long)(t + 1) * p.KB * G - 1) / U); };
+    // one thread counts this block in at a shared tile; true for the block that arrives last, which leaves the counter at zero
+    auto arrive_last = [&](int t) {
+      const int others = last_of(t) - first_of(t);
+      const bool last = atomicAdd(p.count + t, 1) == others;
+      if (last) p.count[t] = 0;
+      return last;
+    };
     int seg = 0;
     for (int u = u0; u < u1; ++seg) {
       const int t = u / p.KB, kb0 = u - t * p.KB, end = min(u1, (t + 1) * p.KB), ab = seg & 1;
@@ -285,7 +309,26 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
       const int n = p.glu ? t * (RW_BN / 2) + (nl & 63) : t * RW_BN + nl;
       const bool live = n < p.N;
       const float bias = p.bias && live ? __bfloat162float(p.bias[n]) : 0.f;
-      if (!mbar_wait_sleep_warp(bar_tfull + ab * 8, (seg >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL, 20)) break;
+      bool ok = mbar_wait_sleep_warp(bar_tfull + ab * 8, (seg >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL, 20);
+#ifdef TFB_BOUNDS_CHECK
+      if (cta == p.give_up) {
+        ok = false;
+        *abort_flag = 1;
+        report(p.status, ST_TIMEOUT_TMEM_FULL);
+      }
+#endif
+      // The four warps meet at barriers below, so they go on or give up together.  A block that gives up (a wait ran out: the status
+      // word says so, its results are wrong) still arrives at every tile that it shares: the counters outlive the launch, and
+      // one left above zero would let a later product add sums that are not there yet.
+      if (!all_of_128(ok)) {
+        for (int v = u; v < u1;) {
+          const int tv = v / p.KB, ve = min(u1, (tv + 1) * p.KB);
+          if (nl == 0 && !(v == tv * p.KB && ve == (tv + 1) * p.KB)) (void)arrive_last(tv);
+          v = ve;
+        }
+        if (nl == 0) drain();
+        break;
+      }
       tc_fence_after();
       // partial sums: [four rows of x][128 weight rows] of four floats
       float4* slot = reinterpret_cast<float4*>(p.ws + ((long long)cta * 2 + (u == u0 ? 0 : 1)) * (MP * 128)) + nl;
@@ -307,15 +350,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
       tc_fence_before();
       mbar_arrive(bar_tempty + ab * 8);
       if (!whole) {
-        // blocks that share the tile: the ones whose runs hold its first and its last unit, and those in between
-        const int c0 = int((((long long)t * p.KB + 1) * G - 1) / U), c1 = int(((long long)(t + 1) * p.KB * G - 1) / U);
+        const int c0 = first_of(t), c1 = last_of(t);
         __threadfence();
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (nl == 0) {
-          const int before = atomicAdd(p.count + t, 1);
-          *last_flag = before == c1 - c0;
-          if (before == c1 - c0) p.count[t] = 0;
-        }
+        if (nl == 0) *last_flag = arrive_last(t);
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (*last_flag) {
           __threadfence();
@@ -425,6 +463,10 @@ static bool rows_workspace(cudaStream_t stream, RowsWs* out) {
   return false;
 }
 
+#ifdef TFB_BOUNDS_CHECK
+static int g_give_up = -1;
+#endif
+
 template <int FMT, int MP>
 static int launch_rows(const CUtensorMap& tx, const CUtensorMap& tw, const RowsParams& p, int grid, cudaStream_t st) {
   using L = RowsPlan<FMT, MP>;
@@ -470,6 +512,9 @@ static int run_rows(const void* x, long long ldx, const void* W, long long ldw, 
   p.scales = static_cast<const __nv_bfloat16*>(scales);
   p.group = group;
   p.ws = w.ws; p.count = w.count; p.status = status;
+#ifdef TFB_BOUNDS_CHECK
+  p.give_up = g_give_up;
+#endif
   // at least four units per block: below that a block's fill, drain and its part in the meeting cost more than the bytes it streams
   const long long units = (long long)p.tiles * p.KB;
   const int sms = std::min(sm_count(), RW_MAX_CTAS);
@@ -497,6 +542,14 @@ int gemm_rows_glu(const void* x, long long ldx, const void* W, long long ldw, vo
 }
 
 }  // namespace tfb
+
+#ifdef TFB_BOUNDS_CHECK
+// Bounds-check build: the epilogue of block `cta` of every product that follows gives up at its first tile, as if its wait had run out.
+TFB_API int tfb_test_rows_give_up(int cta) {
+  tfb::g_give_up = cta;
+  return 0;
+}
+#endif
 
 // out [M, N] = act(alpha * x [M, K] . W [N, K]^T + bias) + residual, M <= 128; out bf16, or fp32 with out_f32.  w_static: the caller promises
 // that the kernel launched just before this one on the stream does not write W.

@@ -75,7 +75,7 @@ def test_packed_rows(M, N, K, fmt, group):
 
 
 def test_rows_under_capture_and_on_streams():
-    """Captured products share one workspace, eager ones have one per stream; more streams than workspaces take the general path."""
+    """Captured and eager products of one stream give the same bits, and those of many streams the same values."""
     x, w = torch.randn(8, 4096, device="cuda").bfloat16(), (torch.randn(6144, 4096, device="cuda") / 64).bfloat16()
     ref = F.gemm(x, w)
     graph = torch.cuda.CUDAGraph()
@@ -94,6 +94,76 @@ def test_rows_under_capture_and_on_streams():
     torch.cuda.synchronize()
     for o in outs:
         assert _rel(o, ref.double()) < 3e-3
+
+
+def _used(what):
+    _lib.register("tfb_rows_workspaces", [_lib.c_i])
+    return _lib.lib().tfb_rows_workspaces(what)
+
+
+def _streaming_operands(seed=0, M=8, N=8192, K=4096):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(M, K, device="cuda", generator=g).bfloat16(), (torch.randn(N, K, device="cuda", generator=g) / 64).bfloat16()
+
+
+def test_graphs_on_two_streams_share_nothing():
+    """Two graphs (and a third with two branches) replayed side by side give the bits of one at a time; their workspaces come back when
+    the graphs are gone."""
+    import gc
+    import time
+    before = _used(1)
+    ops = [_streaming_operands(i) for i in range(4)]
+    want = [F.linear(x, w) for x, w in ops]
+    graphs = []
+    for i in range(2):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = [F.linear(*ops[i]) for _ in range(20)]
+        graphs.append((graph, outs, want[i]))
+    forked, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(forked):
+        side.wait_stream(torch.cuda.current_stream())
+        a = [F.linear(*ops[2]) for _ in range(20)]
+        with torch.cuda.stream(side):
+            b = [F.linear(*ops[3]) for _ in range(20)]
+        torch.cuda.current_stream().wait_stream(side)
+    assert _used(1) == before + 4
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    for _ in range(30):
+        for s, g in zip(streams, [graphs[0][0], graphs[1][0], forked]):
+            with torch.cuda.stream(s):
+                g.replay()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for _, outs, ref in graphs + [(forked, a, want[2]), (forked, b, want[3])]:
+        assert all(torch.equal(o, ref) for o in outs)
+    del graph, graphs, forked, outs, g, a, b, _
+    gc.collect()
+    torch.cuda.synchronize()
+    for _ in range(50):                      # the driver lets go of a graph's objects on a thread of its own
+        if _used(1) <= before:
+            break
+        time.sleep(0.1)
+    assert _used(1) <= before
+
+
+def test_every_stream_streams():
+    """More streams than a process usually has: each takes the streaming form in a workspace of its own, and they may run side by side."""
+    x, w = _streaming_operands(7)
+    want = F.linear(x, w)
+    held = _used(2)
+    streams = [torch.cuda.Stream() for _ in range(12)]
+    outs = []
+    torch.cuda.synchronize()
+    for _ in range(4):
+        for s in streams:
+            with torch.cuda.stream(s):
+                outs.append(F.linear(x, w))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert all(torch.equal(o, want) for o in outs)
+    assert held + 10 <= _used(2) <= held + 12 and _used(3) <= 512      # some of the pool's streams may have had one before
 
 
 # 1408: skinny blocks of 8 + 8 columns, pairs of half tiles; 1000 and 8200: ragged tiles of 64 and 128 outputs, the up half right behind them;

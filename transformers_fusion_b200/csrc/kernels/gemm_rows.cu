@@ -15,7 +15,9 @@
 //
 // warp 0 loads x, warp 1 issues the MMAs, warp 2 loads the weights, warps 4-7 are the epilogue, warps 8-23 convert packed weights.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
+#include <vector>
 
 #include "tfb_host.h"
 #include "tfb_ptx.cuh"
@@ -409,58 +411,115 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
   }
 }
 
-// Partial sums and counters.  Products issued eagerly have a workspace per stream (up to RW_STREAMS of them; a further stream takes the
-// general path), products captured into graphs share one per device: graphs that hold such products are replayed one at a
-// time on a device, as the serving engine does.  Allocated at the first product outside a capture; 20 MB each.
-constexpr int RW_STREAMS = 6;
+// Partial sums and counters: a workspace belongs to one stream, or to one stream of one capture, so that no two products that may run
+// at the same time share any (two graphs on two streams, branches of a graph, threads with streams of their own).  That of a capture is held by
+// the graph (a user object) and free for the next owner when graph and executables are gone; that of a stream stays with it, and passes on
+// only when the pool is at its bound and the stream has been quiet for RW_QUIET products.  Where none is to be had the general path runs.
+// (Two executables made of one graph share its workspace: as for all memory of a graph, they are not to run at the same time.)
+constexpr size_t RW_POOL_BYTES = size_t(512) << 20;
+constexpr int RW_POOL_SLABS = 64;
+constexpr unsigned long long RW_QUIET = 4096;
 struct RowsWs {
   float* ws;
-  int* count;
+  int* count;                         // zero between products
+  size_t bytes;                       // of ws
+  unsigned long long stream, capture; // owner; capture 0: products issued eagerly
+  unsigned long long used;            // number of the last product
+  std::atomic<bool> busy;
 };
-static bool rows_workspace(cudaStream_t stream, RowsWs* out) {
-  struct Entry { cudaStream_t stream; RowsWs w; bool used; };
-  static Entry table[64][RW_STREAMS + 1] = {};           // [0]: captured products
-  static std::mutex mu;
+struct RowsPool {
+  std::mutex mu;
+  std::vector<RowsWs*> slabs[64];     // by device
+  size_t bytes[64] = {};
+  unsigned long long products = 0;
+};
+static RowsPool& rows_pool() {
+  static RowsPool* p = new RowsPool;  // outlives the graphs that a process still holds at its end
+  return *p;
+}
+static void CUDART_CB rows_give_back(void* slab) { static_cast<RowsWs*>(slab)->busy = false; }      // called by the driver: no CUDA call, no lock
+static RowsWs* rows_make(size_t bytes) {
+  const size_t cb = RW_MAX_TILES * sizeof(int);
+  char* q = nullptr;
+  cudaStream_t st = nullptr;
+  const bool ok = cudaMalloc(reinterpret_cast<void**>(&q), bytes + cb) == cudaSuccess && cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
+                  cudaMemsetAsync(q + bytes, 0, cb, st) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess;
+  if (st) (void)cudaStreamDestroy(st);
+  if (!ok) {
+    if (q) (void)cudaFree(q);
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  return new RowsWs{reinterpret_cast<float*>(q), reinterpret_cast<int*>(q + bytes), bytes, 0, 0, 0, false};
+}
+// The workspace of this stream (of its capture) with room for `need` bytes of partial sums, or null.
+static const RowsWs* rows_workspace(cudaStream_t stream, size_t need) {
   int dev = 0;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
+  unsigned long long cap = 0, sid = 0;
+  cudaGraph_t graph = nullptr;
+  // nothing here is ordered with the stream or waits for it: allowed while this or another thread captures
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+  } relaxed;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 ||
+      cudaStreamGetCaptureInfo(stream, &cs, &cap, &graph, nullptr, nullptr) != cudaSuccess || cs == cudaStreamCaptureStatusInvalidated) {
     (void)cudaGetLastError();
-    return false;
+    return nullptr;
   }
-  std::lock_guard<std::mutex> lock(mu);
-  Entry* t = table[dev];
-  if (cs != cudaStreamCaptureStatusNone) {
-    *out = t[0].w;
-    return t[0].used;
-  }
-  auto make = [&](Entry& e, cudaStream_t s) {
-    const size_t wb = size_t(RW_MAX_CTAS) * 2 * RW_MAX_M * 128 * sizeof(float), cb = RW_MAX_TILES * sizeof(int);
-    char* q = nullptr;
-    if (cudaMalloc(reinterpret_cast<void**>(&q), wb + cb) != cudaSuccess || cudaMemset(q + wb, 0, cb) != cudaSuccess ||
-        cudaDeviceSynchronize() != cudaSuccess) {
+  // handles are used again for later streams, ids are not; a capturing stream may not be asked for its id, but keeps its handle
+  if (cs == cudaStreamCaptureStatusActive) {
+    sid = reinterpret_cast<unsigned long long>(stream);
+  } else {
+    cap = 0;
+    if (cudaStreamGetId(stream, &sid) != cudaSuccess) {
       (void)cudaGetLastError();
-      if (q) (void)cudaFree(q);
-      return false;
-    }
-    e.stream = s;
-    e.w.ws = reinterpret_cast<float*>(q);
-    e.w.count = reinterpret_cast<int*>(q + wb);
-    e.used = true;
-    return true;
-  };
-  for (int i = 1; i <= RW_STREAMS; ++i) {
-    if (t[i].used && t[i].stream == stream) {
-      *out = t[i].w;
-      return true;
-    }
-    if (!t[i].used) {
-      if (!t[0].used && !make(t[0], nullptr)) return false;
-      if (!make(t[i], stream)) return false;
-      *out = t[i].w;
-      return true;
+      return nullptr;
     }
   }
-  return false;
+  RowsPool& pool = rows_pool();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  std::vector<RowsWs*>& all = pool.slabs[dev];
+  const unsigned long long now = ++pool.products;
+  RowsWs *best = nullptr, *quiet = nullptr;
+  for (RowsWs* w : all) {
+    if (w->bytes < need) continue;
+    if (w->busy && w->stream == sid && w->capture == cap) {
+      w->used = now;
+      return w;
+    }
+    if (!w->busy && (!best || w->bytes < best->bytes)) best = w;
+    if (w->busy && !w->capture && now - w->used > RW_QUIET && (!quiet || w->used < quiet->used)) quiet = w;
+  }
+  if (!best && int(all.size()) < RW_POOL_SLABS && pool.bytes[dev] + need <= RW_POOL_BYTES) {
+    best = rows_make(need);
+    if (best) {
+      all.push_back(best);
+      pool.bytes[dev] += need;
+    }
+  }
+  if (!best && quiet && !cap) {
+    if (cudaDeviceSynchronize() == cudaSuccess) best = quiet;       // what its old owner has launched is done
+    else (void)cudaGetLastError();
+  }
+  if (best) {
+    best->stream = sid;
+    best->capture = cap;
+    best->used = now;
+    best->busy = true;
+    cudaUserObject_t obj = nullptr;
+    if (cap && cudaUserObjectCreate(&obj, best, rows_give_back, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+      best->busy = false;
+      best = nullptr;
+    } else if (cap && cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+      (void)cudaUserObjectRelease(obj, 1);                           // gives the workspace back
+      best = nullptr;
+    }
+  }
+  if (!best) (void)cudaGetLastError();
+  return best;
 }
 
 #ifdef TFB_BOUNDS_CHECK
@@ -502,8 +561,9 @@ static int run_rows(const void* x, long long ldx, const void* W, long long ldw, 
   if (make_tmap_2d(&tx, x, 2, K, M, ldx * 2, RW_BK, mp)) return TFB_NOT_TAKEN;
   if (fmt < 0 && make_tmap_2d(&tw, W, 2, K, glu ? 2 * N : N, ldw * 2, RW_BK, rows_w)) return TFB_NOT_TAKEN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  RowsWs w;
-  if (!rows_workspace(st, &w)) return TFB_NOT_TAKEN;
+  const int sms = std::min(sm_count(), RW_MAX_CTAS);
+  const RowsWs* w = rows_workspace(st, size_t(sms) * 2 * mp * 128 * sizeof(float));
+  if (!w) return TFB_NOT_TAKEN;
   p.C = C; p.ldc = ldc;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.residual = static_cast<const __nv_bfloat16*>(residual);
@@ -511,13 +571,12 @@ static int run_rows(const void* x, long long ldx, const void* W, long long ldw, 
   p.codes = static_cast<const uint8_t*>(codes);
   p.scales = static_cast<const __nv_bfloat16*>(scales);
   p.group = group;
-  p.ws = w.ws; p.count = w.count; p.status = status;
+  p.ws = w->ws; p.count = w->count; p.status = status;
 #ifdef TFB_BOUNDS_CHECK
   p.give_up = g_give_up;
 #endif
   // at least four units per block: below that a block's fill, drain and its part in the meeting cost more than the bytes it streams
   const long long units = (long long)p.tiles * p.KB;
-  const int sms = std::min(sm_count(), RW_MAX_CTAS);
   const int grid = int(std::max(1ll, std::min<long long>(sms, units / 4)));
   switch (fmt) {
     case -1: return launch_rows_m<-1>(M, tx, tw, p, grid, st);
@@ -542,6 +601,20 @@ int gemm_rows_glu(const void* x, long long ldx, const void* W, long long ldw, vo
 }
 
 }  // namespace tfb
+
+// Workspaces of the current device: 0 all, 1 held by captures and graphs, 2 held by streams, 3 MB allocated.
+TFB_API int tfb_rows_workspaces(int what) {
+  using namespace tfb;
+  int dev = 0, n[3] = {0, 0, 0};
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+  RowsPool& pool = rows_pool();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  for (const RowsWs* w : pool.slabs[dev]) {
+    ++n[0];
+    if (w->busy) ++n[w->capture ? 1 : 2];
+  }
+  return what >= 0 && what < 3 ? n[what] : int(pool.bytes[dev] >> 20);
+}
 
 #ifdef TFB_BOUNDS_CHECK
 // Bounds-check build: the epilogue of block `cta` of every product that follows gives up at its first tile, as if its wait had run out.

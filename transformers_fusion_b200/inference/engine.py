@@ -182,7 +182,7 @@ class _DecodeGraph:
         self.inp[2:].fill_(-1)
         bt = eng._table()[:bucket]                                               # the scheduler's own table: always current
         run = lambda: eng._logits(eng._layers_decode(self.inp[0], self.inp[1].to(torch.int32), bt, self.inp[2], self.inp[3].to(torch.int32)))
-        side = torch.cuda.Stream(device=dev)
+        side = eng._side = eng._side or torch.cuda.Stream(device=dev)            # one for all buckets: workspaces go by stream
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):                  # warm-up outside capture: workspaces, status words, lazy tables
             for _ in range(2):
@@ -229,7 +229,7 @@ class InferenceEngine:
         self.running: List[Request] = []
         self._ids = itertools.count(1)
         self._step = 0
-        self._graphs = {}
+        self._graphs, self._side = {}, None
         self._sample_cache = None
         self._bt_dev, self._bt_rows = None, []      # block table on the device; (request id, pages) of what its rows hold
         self._uploads = None                        # ring of pinned slots: (memory, slot size, events, next slot)

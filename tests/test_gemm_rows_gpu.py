@@ -74,6 +74,33 @@ def test_packed_rows(M, N, K, fmt, group):
     assert _rel(a, want) < 6e-3 and torch.equal(a, b) and torch.equal(a, c) and c is out
 
 
+@pytest.mark.parametrize("M", [1, 8, 20])
+def test_packed_rows_operands_of_other_layouts(M):
+    """What the general form copies or refuses, the one-launch forms do as well: destinations of a wrong shape, on the host, of another
+    type or pitch; biases with a stride or on the host; residuals that broadcast."""
+    N, K = 520, 256
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") / 16).bfloat16()
+    pw = wq.pack_weight(w, "int8", 32)
+    bias = torch.randn(2 * N, device="cuda").bfloat16()[::2]
+    want = wq.gemm_wq(x, pw, bias.contiguous())
+    for b in (bias, bias.cpu()):
+        assert _rel(wq.gemm_wq(x, pw, b), want.double()) < 3e-3
+    wide = torch.zeros(M, N + 8, device="cuda", dtype=torch.bfloat16)
+    for out in (torch.empty(M, N, dtype=torch.bfloat16), torch.empty(M, N, device="cuda"), wide[:, 8:], torch.empty(N, M, device="cuda", dtype=torch.bfloat16).t()):
+        y = wq.gemm_wq(x, pw, bias.contiguous(), out=out)
+        assert y is out and _rel(y.cuda(), want.double()) < 3e-3
+    assert (wide[:, :8] == 0).all()
+    for shape in ((M, N - 8), (M, N + 8), (2, M, N - 1)) + (((M + 1, N),) if M > 1 else ()):      # one row spreads over several
+        with pytest.raises(RuntimeError):
+            wq.gemm_wq(x, pw, out=torch.empty(shape, device="cuda", dtype=torch.bfloat16))
+    res = torch.randn(1, N, device="cuda").bfloat16()
+    assert _rel(wq.gemm_wq(x, pw, residual=res), wq.gemm_wq(x, pw).double() + res.double()) < 3e-3
+    with pytest.raises(RuntimeError):
+        wq.gemm_wq(x, pw, residual=res[:, :-8])
+    torch.cuda.synchronize()
+    _lib.check_status()
+
+
 def test_rows_under_capture_and_on_streams():
     """Captured and eager products of one stream give the same bits, and those of many streams the same values."""
     x, w = torch.randn(8, 4096, device="cuda").bfloat16(), (torch.randn(6144, 4096, device="cuda") / 64).bfloat16()

@@ -194,15 +194,16 @@ def gemm_wq(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor] = No
 
 
 def _gemm_rows(x, pw, bias, residual, dst, w_static):
-    """The one-launch forms; None where the operands' layout does not fit them."""
+    """The one-launch forms; None where the operands' layout does not fit them (the general form copies or refuses them)."""
     M, K = x.shape
     if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or M < 1:
         return None
-    if residual is not None and (residual.dtype != torch.bfloat16 or residual.stride(-1) != 1):
+    plain = lambda t, shape: t.dtype == torch.bfloat16 and t.device == x.device and t.shape == shape and t.stride(-1) == 1
+    if (residual is not None and not plain(residual, (M, pw.N))) or (bias is not None and not plain(bias, (pw.N,))):
         return None
-    if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != pw.N):
-        return None
-    out = dst if dst is not None and dst.dtype == torch.bfloat16 and dst.stride(-1) == 1 else torch.empty((M, pw.N), dtype=x.dtype, device=x.device)
+    # anything else as a destination (another device or type, overlapping rows) is copied into, and that refuses a wrong shape
+    direct = dst is not None and plain(dst, (M, pw.N)) and (M == 1 or dst.stride(0) >= pw.N)
+    out = dst if direct else torch.empty((M, pw.N), dtype=x.dtype, device=x.device)
     args = (x.data_ptr(), x.stride(0), pw.codes.data_ptr(), pw.scales.data_ptr(), pw.fmt, pw.group, out.data_ptr(), out.stride(0), M, pw.N, K, pw.Kp,
             ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0, int(w_static))
     if (M <= 8 or (M <= 16 and K <= SKINNY_K)) and K % 8 == 0:

@@ -257,6 +257,31 @@ def test_feed_prompts_together_match_one_by_one():
         a.feed([(Request([]), [4, 5], [2]), (Request([]), [4, 5], [0])])
 
 
+@pytest.mark.gpu
+def test_upload_ring_behind_a_backlog_and_from_engine_to_engine_gpu():
+    """More uploads than the ring has slots while the device is busy; then the pinned memory passes to an engine that works on
+    another stream, with copies of the first one still queued."""
+    m = _model("cuda", torch.bfloat16)
+    cfg = EngineConfig(max_batch=2, num_pages=8)
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    a = InferenceEngine(m, None, cfg)
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(200_000_000)                   # a tenth of a second of work in front of the copies
+        first = [a._upload([i, i + 1, i + 2]) for i in range(20)]
+        torch.cuda._sleep(200_000_000)
+        first += [a._upload([i, i + 1, i + 2]) for i in range(20, 28)]
+    memory = a._uploads[0][0].data_ptr()
+    del a
+    b = InferenceEngine(m, None, cfg)
+    with torch.cuda.stream(two):
+        second = [b._upload([-i, -i - 1, -i - 2]) for i in range(20)]
+    assert b._uploads[0][0].data_ptr() == memory
+    torch.cuda.synchronize()
+    assert [t.tolist() for t in first] == [[i, i + 1, i + 2] for i in range(28)]
+    assert [t.tolist() for t in second] == [[-i, -i - 1, -i - 2] for i in range(20)]
+
+
 def _moe_model(device="cpu", dtype=torch.float32):
     from transformers_fusion_b200.models.config import MoEConfig
     from transformers_fusion_b200.models.moe import MoEModel

@@ -148,25 +148,31 @@ class PrefixCache:
 
 
 class _TokenBuffers(list):
-    """A claimed pair of pinned buffers; when the engine that holds it goes away the pair is free for the next engine."""
+    """A claimed pair of pinned buffers; when the engine that holds it goes away the pair is free for the next engine.
+    ``events``: part of the buffers -> event behind the last copy from or into it."""
 
 
-_PINNED_TOKENS: Dict[int, list] = {}        # device index -> [(weak reference to the claiming _TokenBuffers, [buf, buf])]
+_PINNED_TOKENS: Dict[int, list] = {}        # device index -> [(weak reference to the claiming _TokenBuffers, [buf, buf], events)]
 
 
 def _pinned_token_buffers(dev, n: int) -> _TokenBuffers:
     """Two pinned int64 buffers of at least n entries for the device -> host copy of a step's sampled ids.  The memory is
     kept for the life of the process and handed from engine to engine instead of being freed: a pinned block pending
-    release makes the host allocator record and query events, and such calls disturb a stream capture in progress."""
+    release makes the host allocator record and query events, and such calls disturb a stream capture in progress.
+    What the engine before has queued from or into them (on any stream) is waited for."""
     pool = _PINNED_TOKENS.setdefault(dev.index if dev.index is not None else torch.cuda.current_device(), [])
-    for i, (owner, bufs) in enumerate(pool):
+    for i, (owner, bufs, events) in enumerate(pool):
         if owner() is None and bufs[0].numel() >= n:
+            for ev in events.values():
+                ev.synchronize()
+            events.clear()
             break
     else:
-        i, bufs = len(pool), [torch.empty(max(n, 64), dtype=torch.int64).pin_memory() for _ in range(2)]
+        i, bufs, events = len(pool), [torch.empty(max(n, 64), dtype=torch.int64).pin_memory() for _ in range(2)], {}
         pool.append(None)
     held = _TokenBuffers(bufs)
-    pool[i] = (weakref.ref(held), bufs)
+    held.events = events
+    pool[i] = (weakref.ref(held), bufs, events)
     return held
 
 
@@ -232,7 +238,7 @@ class InferenceEngine:
         self._graphs, self._side = {}, None
         self._sample_cache = None
         self._bt_dev, self._bt_rows = None, []      # block table on the device; (request id, pages) of what its rows hold
-        self._uploads = None                        # ring of pinned slots: (memory, slot size, events, next slot)
+        self._uploads = None                        # ring of pinned slots: (memory, slot size, next slot)
         self._inflight = None          # (requests, device tokens, pinned host tokens, event) of the decode step in flight
         self._tok_host = None
         self.stats = InferenceStats()
@@ -618,7 +624,7 @@ class InferenceEngine:
                     self._tok_flip = getattr(self, "_tok_flip", 0) ^ 1  # never the buffer the previous step is still read from
                     host = self._tok_host[self._tok_flip][:len(reqs)]
                     host.copy_(toks_dev, non_blocking=True)
-                    ev = torch.cuda.Event()
+                    ev = self._tok_host.events[self._tok_flip] = torch.cuda.Event()
                     ev.record()
                 self._inflight = (reqs, toks_dev, host, ev)
                 if prev is not None:
@@ -784,21 +790,22 @@ class InferenceEngine:
         dev, k = self.device, len(values)
         if dev.type == "cuda" and self._uploads is None:
             size = max(5 * self._bucket(self.cfg.max_batch), 512)
-            self._uploads = [_pinned_token_buffers(dev, 8 * size), size, [None] * 8, 0]
+            self._uploads = [_pinned_token_buffers(dev, 8 * size), size, 0]
         if dev.type != "cuda" or k > self._uploads[1]:
             t = torch.tensor(values, dtype=torch.int64).to(dev)
             return t if out is None else out.copy_(t)
-        memory, size, events, i = self._uploads
-        if events[i] is None:
-            events[i] = torch.cuda.Event()
+        memory, size, i = self._uploads
+        ev = memory.events.get(i)
+        if ev is None:
+            ev = memory.events[i] = torch.cuda.Event()
         else:
-            events[i].synchronize()
+            ev.synchronize()
         slot = memory[0][i * size:i * size + k]
         slot.copy_(torch.tensor(values, dtype=torch.int64))
         out = torch.empty(k, dtype=torch.int64, device=dev) if out is None else out
         out.copy_(slot, non_blocking=True)
-        events[i].record()
-        self._uploads[3] = (i + 1) % 8
+        ev.record()
+        self._uploads[2] = (i + 1) % 8
         return out
 
     def _block_table(self, reqs):

@@ -257,6 +257,21 @@ def test_feed_prompts_together_match_one_by_one():
         a.feed([(Request([]), [4, 5], [2]), (Request([]), [4, 5], [0])])
 
 
+@pytest.mark.parametrize("lens", [[70], [70, 70], [5, 70]])
+def test_prompts_past_the_learned_positions_are_refused_on_the_host(lens):
+    """One or several in a call, through ``feed`` and through the scheduler: the same error, before any index goes to the device."""
+    m = _model(position_type="learned", max_seq_len=64)
+    for run in ("feed", "step"):
+        eng = InferenceEngine(m, None, EngineConfig(max_batch=4, num_pages=64, max_seq_len=128, enable_prefix_cache=False))
+        with pytest.raises(RuntimeError):
+            if run == "feed":
+                eng.feed([(Request([]), list(range(3, 3 + n)), [0]) for n in lens])
+            else:
+                for n in lens:
+                    eng.add_request(list(range(3, 3 + n)), 2)
+                eng.step()
+
+
 @pytest.mark.gpu
 def test_upload_ring_behind_a_backlog_and_from_engine_to_engine_gpu():
     """More uploads than the ring has slots while the device is busy; then the pinned memory passes to an engine that works on

@@ -422,6 +422,8 @@ class InferenceEngine:
         ids, slots, positions = torch.stack([ids, slots, positions]).to(dev)
         h = F.embedding_fwd(ids, m.tok_embeddings.data, None, 0)
         if m.pos_embeddings is not None:
+            if max(lens) > m.pos_embeddings.shape[0]:        # on the host: an index past the table would cost the device's context
+                raise RuntimeError(f"a prompt of {max(lens)} tokens is longer than the model's {m.pos_embeddings.shape[0]} positions")
             h = h + m.pos_embeddings.data[positions]
         rope = m.rope(dev)
         positions = positions.to(torch.int32)

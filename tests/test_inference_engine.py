@@ -257,6 +257,25 @@ def test_feed_prompts_together_match_one_by_one():
         a.feed([(Request([]), [4, 5], [2]), (Request([]), [4, 5], [0])])
 
 
+def test_a_refused_feed_changes_nothing():
+    """Places outside an entry and more single tokens than the batch holds are refused before pages are taken or sequences move on."""
+    m = _model()
+    eng = InferenceEngine(m, None, EngineConfig(max_batch=3, num_pages=64, max_prefill_tokens=16, enable_prefix_cache=False))
+    going = [Request([]) for _ in range(4)]
+    eng.feed([(r, [5, 6, 7], []) for r in going])
+    free, state = list(eng.cache.allocator.free), [(r.pos, list(r.tokens), list(r.pages)) for r in going]
+    late = Request([])
+    for entries, error in (([(Request([]), [4] * 12, [0]), (late, [4] * 12, [12])], IndexError),          # the second group of prompts
+                           ([(Request([]), [4, 5], [-3])], IndexError),
+                           ([(going[0], [8], [0]), (going[1], [8, 9], [2])], IndexError),                 # a portion of a running sequence
+                           ([(Request([]), [4, 5], [1])] + [(r, [8], [0]) for r in going], ValueError)):
+        with pytest.raises(error):
+            eng.feed(entries)
+        assert eng.cache.allocator.free == free and [(r.pos, r.tokens, r.pages) for r in going] == state
+    assert late.pos == 0 and not late.pages
+    assert [x.shape[0] for x in eng.feed([(late, [4] * 12, [11])] + [(r, [8], [0]) for r in going[:3]])] == [1] * 4
+
+
 @pytest.mark.parametrize("lens", [[70], [70, 70], [5, 70]])
 def test_prompts_past_the_learned_positions_are_refused_on_the_host(lens):
     """One or several in a call, through ``feed`` and through the scheduler: the same error, before any index goes to the device."""

@@ -638,12 +638,15 @@ class InferenceEngine:
             self._collect(prev, finished)
         return finished
 
+    def _check_batch(self, n: int):
+        if n > self.cfg.max_batch:
+            raise ValueError(f"{n} sequences do not fit into a batch of {self.cfg.max_batch}")
+
     def _decode_logits(self, reqs: List[Request], host_tokens, pending=None, prev_tokens=None):
         """Append one token to every sequence and return the logits [len(reqs), V] at it.  ``pending[i]`` >= 0: the token of row
         i is row pending[i] of ``prev_tokens`` (on the device) instead of host_tokens[i]."""
         dev, alloc = self.device, self.cache.allocator
-        if len(reqs) > self._bucket(self.cfg.max_batch):
-            raise ValueError(f"{len(reqs)} sequences do not fit into a batch of {self.cfg.max_batch}")
+        self._check_batch(len(reqs))
         for r in reqs:
             if r.pos // PAGE >= len(r.pages):
                 r.pages.append(alloc.alloc())
@@ -681,6 +684,11 @@ class InferenceEngine:
         for r, t, _ in entries:
             if r.pos + len(t) > self.max_len:
                 raise ValueError(f"a sequence of {r.pos + len(t)} tokens does not fit into {self.max_len}")
+        # what is refused is refused here, before a page is taken or a sequence moves on
+        for r, t, w in entries:
+            if not self.stack and (r.pos == 0 or len(t) > 1) and any(not -len(t) <= x < len(t) for x in w):
+                raise IndexError(f"a place outside the {len(t)} tokens of its entry")
+        self._check_batch(sum(r.pos > 0 and len(t) == 1 for r, t, _ in entries))
         fresh = [i for i, (r, _, _) in enumerate(entries) if r.pos == 0]
         for i in fresh:
             r, t, _ = entries[i]
@@ -708,8 +716,6 @@ class InferenceEngine:
                 at, want = 0, []
                 for i in grp:
                     n = len(entries[i][1])
-                    if any(not -n <= w < n for w in entries[i][2]):
-                        raise IndexError(f"a place outside the {n} tokens of its entry")
                     want.append([at + w % n for w in entries[i][2]])
                     at += n
                 if any(want):

@@ -82,6 +82,19 @@ def test_col_sum(T, N):
     assert ((out.double() - 1 - x.double().sum(0)).abs() <= 1e-5 * (1 + x.double().abs().sum(0))).all()
 
 
+@pytest.mark.gpu
+def test_col_sum_repeats_itself_and_takes_no_rows():
+    for T, N in ((512, 768), (513, 1024), (513, 1032), (700, 4104), (4662, 3072)):        # either side of each form's limits
+        x = torch.randn(T, N + 8, device="cuda").bfloat16()[:, :N]
+        sums = [F.col_sum_(x, torch.zeros(N, device="cuda")) for _ in range(20)]
+        assert all(torch.equal(s, sums[0]) for s in sums)
+        assert ((sums[0].double() - x.double().sum(0)).abs() <= 1e-5 * (1 + x.double().abs().sum(0))).all()
+    out = torch.ones(3072, device="cuda")
+    assert torch.equal(F.col_sum_(x[:0], out), torch.ones_like(out))
+    with pytest.raises(RuntimeError):
+        F.col_sum_(x, torch.zeros(3064, device="cuda"))
+
+
 def test_rope_roundtrip_and_ref():
     T, S, nh, D = 256, 128, 10, 64
     ld = 12 * D

@@ -274,24 +274,30 @@ __global__ void __launch_bounds__(256) norm_bwd_kernel(const __nv_bfloat16* __re
   }
 }
 
-// out[n] += sum over rows of x[m, n]: the gradient of a bias.  Bound by reading x once: a warp covers 256 columns of a row with
-// 16-byte loads, four rows in flight, the block's eight warps and the blocks along y share the rows.
-__global__ void __launch_bounds__(256) col_sum_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, float* __restrict__ out, int rows, int N) {
+// out[n] += sum over rows of x[m, n]: the gradient of a bias.  Bound by reading x once: a block takes 64 columns (eight threads a row,
+// 32 rows at a time, FLIGHT of them in flight per thread), a cluster of BLOCKS shares the rows.  The sums meet in a fixed order - lanes,
+// warps, blocks over distributed shared memory - so that the same input gives the same bits; blocks that meet in atomics are 10 - 40 %
+// faster and do not (us, atomics -> this: 131 x 768 1.8 -> 2.2, 4662 x 768 3.0 -> 4.1, 4662 x 3072 6.5 -> 8.3, 65536 x 3072 59 -> 61; fp32 copy and
+// torch's sum 9.1, 25.7, 61, 667).
+constexpr int CS_ROWS = 32;
+template <int BLOCKS, int FLIGHT>
+__global__ void __cluster_dims__(1, BLOCKS, 1) __launch_bounds__(256) col_sum_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
+                                                                                    float* __restrict__ out, int rows, int N) {
   tfb::pdl_sync();
-  __shared__ float red[8][256];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int col = (blockIdx.x * 32 + lane) * 8;
-  const int step = gridDim.y * 8;
+  __shared__ float red[8][64], part[64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = (threadIdx.x & 7) * 8;
+  const int col = blockIdx.x * 64 + c0;
+  constexpr int STEP = BLOCKS * CS_ROWS;
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (col < N) {
-    for (int row = blockIdx.y * 8 + warp; row < rows; row += 4 * step) {
-      uint4 v[4];
+    for (int row = blockIdx.y * CS_ROWS + int(threadIdx.x >> 3); row < rows; row += FLIGHT * STEP) {
+      uint4 v[FLIGHT];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (row + u * step < rows) v[u] = *reinterpret_cast<const uint4*>(x + (long long)(row + u * step) * ldx + col);
+      for (int u = 0; u < FLIGHT; ++u)
+        if (row + u * STEP < rows) v[u] = *reinterpret_cast<const uint4*>(x + (long long)(row + u * STEP) * ldx + col);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (row + u * step >= rows) break;
+      for (int u = 0; u < FLIGHT; ++u) {
+        if (row + u * STEP >= rows) break;
         float f[8];
         cvt8(v[u], f);
 #pragma unroll
@@ -300,15 +306,37 @@ __global__ void __launch_bounds__(256) col_sum_kernel(const __nv_bfloat16* __res
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) red[warp][lane * 8 + i] = acc[i];
+  for (int i = 0; i < 8; ++i) {
+    acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 8);
+    acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
+  }
+  if (lane < 8) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) red[warp][c0 + i] = acc[i];
+  }
   __syncthreads();
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c < N) {
+  if (threadIdx.x < 64) {
     float v = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) v += red[k][threadIdx.x];
-    atomicAdd(out + c, v);
+    if (BLOCKS == 1) {
+      if (blockIdx.x * 64 + int(threadIdx.x) < N) out[blockIdx.x * 64 + threadIdx.x] += v;
+    } else {
+      part[threadIdx.x] = v;
+    }
   }
+  if (BLOCKS == 1) return;
+  cluster_sync();
+  if (blockIdx.y == 0 && threadIdx.x < 64 && blockIdx.x * 64 + int(threadIdx.x) < N) {
+    const uint32_t mine = smem_u32(&part[threadIdx.x]);
+    float v[BLOCKS], sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < BLOCKS; ++k) v[k] = ld_shared_cluster_f32(map_cta(mine, k));
+#pragma unroll
+    for (int k = 0; k < BLOCKS; ++k) sum += v[k];
+    out[blockIdx.x * 64 + threadIdx.x] += sum;
+  }
+  cluster_sync();      // a block's shared memory stays until it has been read
 }
 
 // Wide rows (more than 1024 entries): one CTA per row, so that a 4096-wide row is two 16-byte loads per thread.
@@ -470,9 +498,19 @@ TFB_API int tfb_layernorm_bwd(const void* dy, const void* h, const void* w, cons
 // out [N] fp32 += column sums of x [rows, N] bf16 (row pitch ldx); N and ldx multiples of 8, x aligned to 16 bytes.
 TFB_API int tfb_col_sum(const void* x, long long ldx, float* out, int rows, int N, void* stream) {
   using namespace tfb;
-  if (rows <= 0 || N <= 0 || N % 8 || ldx % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) return TFB_ERR_ARG;
-  const int gx = (N + 255) / 256;
-  const dim3 g(gx, max(1, min((rows + 31) / 32, sm_count() * 4 / gx)));
-  tfb::launch_k(col_sum_kernel, g, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x), ldx, out, rows, N);
+  if (rows < 0 || N <= 0 || N % 8 || ldx % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) return TFB_ERR_ARG;
+  if (rows == 0) return TFB_OK;
+  auto X = static_cast<const __nv_bfloat16*>(x);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int gx = (N + 63) / 64;
+  // one block per 64 columns while its few turns take less time than a cluster's meeting (512 x 768 2.9 us against 2.8, 131 x 768 2.2
+  // against 2.7); clusters of four where their number is large (8192 x 6144 18 us against 21); more in flight where it is small (16384 x 768 8
+  // against 10)
+#define TFB_GO(BLOCKS, FLIGHT) tfb::launch_k(col_sum_kernel<BLOCKS, FLIGHT>, dim3(gx, BLOCKS), 256, 0, st, X, ldx, out, rows, N)
+  if (rows <= 512) TFB_GO(1, 8);
+  else if (gx > 64) TFB_GO(4, 8);
+  else if (gx > 16) TFB_GO(8, 8);
+  else TFB_GO(8, 16);
+#undef TFB_GO
   return int(cudaGetLastError());
 }

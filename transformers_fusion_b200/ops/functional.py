@@ -191,8 +191,8 @@ _lib.register("tfb_col_sum", [_lib.c_p, _lib.c_ll, _lib.c_p, _lib.c_i, _lib.c_i,
 
 def col_sum_(x, out):
     """out [N] fp32 += the column sums of x [M, N] (the gradient of a bias)."""
-    if not x.is_cuda or x.dtype != torch.bfloat16 or out.dtype != torch.float32 or not out.is_contiguous() or x.stride(-1) != 1 or \
-            x.shape[1] % 8 or x.stride(0) % 8 or x.data_ptr() % 16:
+    if not x.is_cuda or x.dtype != torch.bfloat16 or out.dtype != torch.float32 or out.device != x.device or out.shape != x.shape[1:] or \
+            not out.is_contiguous() or x.stride(-1) != 1 or x.shape[0] == 0 or x.shape[1] % 8 or x.stride(0) % 8 or x.data_ptr() % 16:
         return out.add_(x.float().sum(0))
     check(_lib.lib().tfb_col_sum(x.data_ptr(), x.stride(0), out.data_ptr(), x.shape[0], x.shape[1], stream()), "col_sum")
     return out

@@ -86,6 +86,39 @@ def test_corrupt_quant_block_detected(tmp_path):
         codec.QuantReader(tmp_path / "m.quant").read_tensor("a")
 
 
+def test_kernels_hold_their_tensor_memory_before_the_next_one_may_start():
+    """A kernel that releases its successor (``pdl_sync``) and allocates tensor memory afterwards could find it taken by a block of that
+    successor, which waits for this kernel to end."""
+    import re
+    from transformers_fusion_b200.build import CSRC
+    seen = 0
+    for path in sorted((CSRC / "kernels").glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        starts = [m.start() for m in re.finditer(r"__global__", text)] + [len(text)]
+        for a, b in zip(starts, starts[1:]):
+            body = text[a:b]
+            allocs = [m.start() for m in re.finditer(r"\btmem_alloc(?:_pair)?\(", body)]
+            if not allocs:
+                continue
+            # a block that leaves early (the copy blocks of a fused product) has no tensor memory
+            syncs = [m.start() for m in re.finditer(r"\bpdl_sync\(\)", body) if "return;" not in body[m.start():allocs[0]]]
+            assert syncs and min(syncs) > max(allocs), path.name
+            seen += 1
+    assert seen >= 10
+
+
+@pytest.mark.parametrize("value,mode", [(None, 1), ("", 1), ("0", 0), ("1", 2)])
+def test_programmatic_launches_can_be_switched_off(value, mode):
+    import subprocess
+    import sys
+    env = {k: v for k, v in os.environ.items() if k != "TFB_PDL"}
+    if value is not None:
+        env["TFB_PDL"] = value
+    r = subprocess.run([sys.executable, "-c", "from transformers_fusion_b200.ops import _lib; print(_lib.lib().tfb_pdl_mode())"], capture_output=True,
+                       text=True, timeout=300, env=env, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and int(r.stdout) == mode, r.stdout + r.stderr
+
+
 @pytest.mark.gpu
 def test_device_wait_times_out_with_status():
     """A device-side barrier whose peer never arrives: the kernel gives up after its bounded wait and reports it."""

@@ -89,7 +89,6 @@ __global__ void __launch_bounds__(BwdSmem<D, true>::THREADS, D == 64 ? 2 : 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                      const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                      const AttnBwdParams p) {
-  tfb::pdl_sync();
   using L = BwdSmem<D, true>;
   constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES, WG = L::WG;
   extern __shared__ uint8_t smem_raw[];
@@ -142,6 +141,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tfb::pdl_sync();   // after the allocation: a block of the next kernel may be placed from here on, and must not get the columns first
   const uint32_t tDV = tmem_base + L::ACC_COL, tDK = tDV + D;
 
   if (warp == 0) {
@@ -377,7 +377,6 @@ __global__ void __launch_bounds__(BwdSmem<D, false>::THREADS, D == 64 ? 2 : 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                    const AttnBwdParams p) {
-  tfb::pdl_sync();
   using L = BwdSmem<D, false>;
   constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES, WG = L::WG;
   extern __shared__ uint8_t smem_raw[];
@@ -425,6 +424,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tfb::pdl_sync();   // after the allocation: a block of the next kernel may be placed from here on, and must not get the columns first
   const uint32_t tDQ = tmem_base + L::ACC_COL;
 
   if (warp == 0) {

@@ -42,7 +42,6 @@ struct F8Smem {
 
 __global__ void __launch_bounds__(F8_THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, const F8Params p) {
-  tfb::pdl_sync();
   using L = F8Smem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -76,6 +75,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tfb::pdl_sync();   // after the allocation: a block of the next kernel may be placed from here on, and must not get the columns first
   const int num_tiles = p.tiles_m * p.tiles_n;
 
   if (warp == 0) {

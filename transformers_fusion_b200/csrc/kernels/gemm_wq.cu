@@ -68,7 +68,6 @@ struct WqParams {
 
 template <int FMT, int AROWS>
 __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_constant__ CUtensorMap tma_a, const WqParams p) {
-  tfb::pdl_sync();
   using PL = WqPlan<AROWS>;
   constexpr int WQ_STAGES = PL::STAGES, WQ_A_BYTES = PL::A_BYTES, WQ_STAGE = PL::STAGE, WQ_RAW_OFF = PL::RAW_OFF, WQ_BAR_OFF = PL::BAR_OFF;
   extern __shared__ uint8_t smem_raw[];
@@ -113,6 +112,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  tfb::pdl_sync();   // after the allocation: a block of the next kernel may be placed from here on, and must not get the columns first
   const int KB = (p.K + WQ_BK - 1) / WQ_BK;
   const int num_work = p.tiles_m * p.tiles_n * p.splits;
   const int nctas = gridDim.x, cta = blockIdx.x;

@@ -76,12 +76,12 @@ int make_tmap_4d(CUtensorMap* out, const void* base, int elem_bytes, const uint6
   return r == CUDA_SUCCESS ? TFB_OK : TFB_ERR_DRIVER;
 }
 
-int pdl_enabled() {
-  static const int on = [] {
+int pdl_mode() {
+  static const int mode = [] {
     const char* e = getenv("TFB_PDL");
-    return (e && e[0] == '1') ? 1 : 0;
+    return !e || !e[0] ? 1 : e[0] == '1' ? 2 : 0;
   }();
-  return on;
+  return mode;
 }
 
 int sm_count() {
@@ -98,4 +98,5 @@ int sm_count() {
 }  // namespace tfb
 
 TFB_API int tfb_sm_count() { return tfb::sm_count(); }
+TFB_API int tfb_pdl_mode() { return tfb::pdl_mode(); }
 TFB_API int tfb_version() { return 1; }

@@ -35,11 +35,14 @@ int make_tmap_4d(CUtensorMap* out, const void* base, int elem_bytes, const uint6
 
 int sm_count();
 
-// 1 when the environment has TFB_PDL=1 (read once): whether launches allow programmatic stream serialization.  Off by
-// default: measured on B200 under CUDA-graph replay it shortens a batch-1 decode step of the 8B shape by 5 % (1.45 -> 1.38
-// ms for 8 layers) but lengthens the 64-sequence training step of the 50M model by 3 % (31.1 -> 32.0 ms), where early-placed
+// Whether launches allow programmatic stream serialization, from TFB_PDL (read once): unset, kernels of a decode step only (launch_k_pdl, launch_k_rows);
+// 0, none; 1, all.  Not all by default: measured on B200 under CUDA-graph replay it shortens a batch-1 decode step of the 8B shape by 5 % (1.45 ->
+// 1.38 ms for 8 layers) but lengthens the 64-sequence training step of the 50M model by 3 % (31.1 -> 32.0 ms), where early-placed
 // CTAs of the next kernel take shared memory and registers from the tail of the running one.
-int pdl_enabled();
+// What makes it safe: every kernel waits (pdl_sync) before it touches memory that an earlier one wrote, releases the next kernel only after that
+// wait, and has its tensor memory by then - the first thread that releases does so for its block, and a block of the next kernel that took
+// tensor memory ahead of a warp of this one would wait for this kernel while this kernel waits for it.
+int pdl_mode();      // 0 none, 1 decode steps, 2 all
 
 // gemm_rows.cu, skinny_linear.cu: products of few rows.  x [M, K], W [N, K] (or codes and scales of a packed weight, fmt >= 0).
 // Both return 0, a CUDA error, or TFB_NOT_TAKEN where the general path is to run.
@@ -75,13 +78,13 @@ inline void launch_attr(int pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, 
 
 template <class... KArgs, class... Args>
 inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
-  launch_attr(pdl_enabled(), kern, grid, block, smem, stream, std::forward<Args>(args)...);
+  launch_attr(pdl_mode() == 2, kern, grid, block, smem, stream, std::forward<Args>(args)...);
 }
-// The same with programmatic launch always allowed: kernels of a decode step, a few microseconds each, where the gap between
+// The same with programmatic launch unless it is switched off: kernels of a decode step, a few microseconds each, where the gap between
 // two launches and the set-up of the next are a large part of the time.
 template <class... KArgs, class... Args>
 inline void launch_k_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
-  launch_attr(1, kern, grid, block, smem, stream, std::forward<Args>(args)...);
+  launch_attr(pdl_mode() != 0, kern, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 // For kernels that serve decode steps as well as whole batches: programmatic launch up to 256 rows (a decode batch, a short prompt).
@@ -90,7 +93,7 @@ inline void launch_k_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t s
 constexpr long long PDL_ROWS = 256;
 template <class... KArgs, class... Args>
 inline void launch_k_rows(long long rows, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
-  launch_attr(rows <= PDL_ROWS ? 1 : pdl_enabled(), kern, grid, block, smem, stream, std::forward<Args>(args)...);
+  launch_attr(pdl_mode() == 2 || (pdl_mode() == 1 && rows <= PDL_ROWS), kern, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 // One-time set-up per device.  Kernel attributes (cudaFuncSetAttribute) belong to the device that is current when

@@ -141,7 +141,7 @@ def test_rope_append_is_rotation_then_append(mode, Hq, Hkv, D, T):
 
 @pytest.mark.parametrize("splits", [1, 2, 3, 7, 16])
 def test_paged_decode_merges_its_splits(splits):
-    """The block that arrives last merges: the same bits from call to call, splits that hold no token included."""
+    """The same bits from call to call, splits that hold no token included."""
     Hq, Hkv, D, lens = 8, 2, 64, torch.tensor([1, 17, 300, 129], dtype=torch.int32)
     c = {d: PagedKVCache(1, 80, Hkv, D, "bf16", d) for d in ("cpu", "cuda")}
     bt = torch.arange(80, dtype=torch.int32).view(4, 20)
@@ -155,3 +155,31 @@ def test_paged_decode_merges_its_splits(splits):
     _lib.check_status()
     assert (got[0].float().cpu() - want).abs().max().item() < 2e-2
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("mode,tol", [("bf16", 2e-2), ("fp8", 2e-2), ("q4", 2e-2)])
+@pytest.mark.parametrize("B,Hq,Hkv,D,table", [(1, 8, 2, 128, 1300), (5, 12, 12, 64, 1300), (5, 32, 8, 128, 4000), (40, 16, 8, 64, 1300), (40, 32, 8, 128, 1300),
+                                              (40, 32, 8, 128, 9000)])
+def test_paged_decode_cuts_sequences_by_their_own_length(mode, tol, B, Hq, Hkv, D, table):
+    """The rule's splits: as many blocks as run at once, of 128 tokens at least, or for a full device parts of 384 - lengths at the edges of
+    both, next to sequences that take one part only, in tables of the longest sequence's size and of a roomy one."""
+    lens = torch.tensor(([1, 128, 129, 383, 384, 385, 768, 769, 1200] * 5)[-B:], dtype=torch.int32)
+    n = [(int(x) + PAGE - 1) // PAGE for x in lens]
+    cpu, gpu = (PagedKVCache(1, sum(n), Hkv, D, mode, d) for d in ("cpu", "cuda"))
+    bt, at, slots = torch.zeros(B, table // PAGE, dtype=torch.int32), 0, []
+    for b, k in enumerate(n):
+        bt[b, :k] = torch.arange(at, at + k)
+        slots.append(torch.arange(at * PAGE, at * PAGE + int(lens[b])))
+        at += k
+    slots = torch.cat(slots)
+    src, q = torch.randn(slots.numel(), (Hq + 2 * Hkv) * D).bfloat16(), torch.randn(B, Hq * D).bfloat16()
+    gpu.append(0, src.cuda(), Hq * D, (Hq + Hkv) * D, slots.cuda())
+    for mine, theirs in ((cpu.k[0], gpu.k[0]), (cpu.v[0], gpu.v[0])):          # the oracle reads the same pages
+        mine.data.copy_(theirs.data)
+        if mine.scale is not None:
+            mine.scale.copy_(theirs.scale)
+    want = cpu.decode(0, q, bt, lens, Hq).float()
+    got = gpu.decode(0, q.cuda(), bt.cuda(), lens.cuda(), Hq)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert (got.float().cpu() - want).abs().max().item() < tol

@@ -421,26 +421,74 @@ __global__ void __launch_bounds__(DEC_THREADS) paged_decode_kernel(
   }
 }
 
-// o[b, h, :] = sum_s acc_s * exp(m_s - M) / sum_s l_s * exp(m_s - M)
-__global__ void paged_combine_kernel(const float* __restrict__ acc, const float* __restrict__ ml,
-                                     __nv_bfloat16* __restrict__ o, long long ldo, int Hq, int D, int splits) {
+// Parts that a sequence is cut into: `splits` at most, of about `part_tokens` tokens at least.  The lengths are only known on the device; blocks of
+// the parts that a short sequence does not have leave at once.
+__device__ __forceinline__ int parts_of(int len, int splits, int part_tokens) {
+  return min(splits, max(1, (len + part_tokens - 1) / part_tokens));
+}
+
+// o[b, h, :] = sum_s acc_s * exp(m_s - M) / sum_s l_s * exp(m_s - M).  One warp per sequence and head, the partial results of sixteen splits
+// in flight together, lane s holding the maximum and the sum of split s.
+template <int D>
+__global__ void __launch_bounds__(128) paged_combine_kernel(const float* __restrict__ acc, const float* __restrict__ ml,
+                                                            __nv_bfloat16* __restrict__ o, long long ldo, const int* __restrict__ seq_lens, int heads,
+                                                            int Hq, int splits, int part_tokens) {
   tfb::pdl_sync();
-  const int b = blockIdx.x, h = blockIdx.y;
-  const long long base = ((long long)b * Hq + h) * splits;
-  float M = -INFINITY;
-  for (int s = 0; s < splits; ++s) M = fmaxf(M, ml[(base + s) * 2]);
-  float L = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const float ms = ml[(base + s) * 2];
-    if (ms != -INFINITY) L += ml[(base + s) * 2 + 1] * __expf(ms - M);
-  }
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float v = 0.f;
-    for (int s = 0; s < splits; ++s) {
-      const float ms = ml[(base + s) * 2];
-      if (ms != -INFINITY) v += acc[(base + s) * D + d] * __expf(ms - M);
+  constexpr int N = D / 32, MS = 16;                         // columns per lane, splits per turn
+  const int lane = threadIdx.x & 31, head = int(blockIdx.x) * 4 + int(threadIdx.x >> 5);
+  if (head >= heads) return;
+  const int parts = part_tokens > 0 ? parts_of(seq_lens[head / Hq], splits, part_tokens) : splits;      // 0: every split has written, one as well
+  if (part_tokens > 0 && parts == 1) return;                 // written by its only part
+  const long long base = (long long)head * splits;
+  float M = -INFINITY, L = 0.f, v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = 0.f;
+  for (int s0 = 0; s0 < parts; s0 += MS) {
+    const bool mine = lane < MS && s0 + lane < parts;
+    const float2 x = mine ? reinterpret_cast<const float2*>(ml)[base + s0 + lane] : make_float2(-INFINITY, 0.f);
+    float a[MS][N];
+#pragma unroll
+    for (int k = 0; k < MS; ++k) {
+      if (s0 + k >= parts) break;
+      const float* src = acc + (base + s0 + k) * D + lane * N;
+      if constexpr (N == 4) {
+        const float4 f = *reinterpret_cast<const float4*>(src);
+        a[k][0] = f.x; a[k][1] = f.y; a[k][2] = f.z; a[k][3] = f.w;
+      } else {
+        const float2 f = *reinterpret_cast<const float2*>(src);
+        a[k][0] = f.x; a[k][1] = f.y;
+      }
     }
-    o[(long long)b * ldo + h * D + d] = __float2bfloat16(L > 0.f ? v / L : 0.f);
+    float m = x.x;
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    m = fmaxf(M, __shfl_sync(0xffffffffu, m, 0));
+    if (m == -INFINITY) continue;
+    const float f = __expf(M - m), w = x.x == -INFINITY ? 0.f : __expf(x.x - m);
+    M = m;
+    L *= f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] *= f;
+#pragma unroll
+    for (int k = 0; k < MS; ++k) {
+      if (s0 + k >= parts) break;
+      const float e = __shfl_sync(0xffffffffu, w, k), l = __shfl_sync(0xffffffffu, x.y, k);
+      if (e == 0.f) continue;                                // a split without tokens
+      L += l * e;
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] += a[k][i] * e;
+    }
+  }
+  const float r = L > 0.f ? 1.f / L : 0.f;
+  __nv_bfloat16* dst = o + (long long)(head / Hq) * ldo + (head % Hq) * D + lane * N;
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    if (((ldo & 1) | (reinterpret_cast<uintptr_t>(o) & 3)) == 0) {
+      *reinterpret_cast<uint32_t*>(dst + i) = pack_bf16(v[i] * r, v[i + 1] * r);
+    } else {
+      dst[i] = __float2bfloat16(v[i] * r);
+      dst[i + 1] = __float2bfloat16(v[i + 1] * r);
+    }
   }
 }
 
@@ -576,11 +624,13 @@ __device__ __forceinline__ void tc_stage(const KvPool& pool, const int* __restri
   }
 }
 
+// Blocks per SM: shared memory allows three (heads of 128) and five (64); the registers of the fp8 form two, and left to itself the
+// compiler gives the 4-bit form 194 and the SM two blocks of it (64 sequences of 64 - 2000 tokens 123 us, with three 95).
 template <int MODE, int D>
-__global__ void __launch_bounds__(TC_THREADS) paged_decode_mma_kernel(
+__global__ void __launch_bounds__(TC_THREADS, D == 64 ? 4 : MODE == KV_FP8 ? 2 : 3) paged_decode_mma_kernel(
     const __nv_bfloat16* __restrict__ q, long long ldq, KvPool kpool, KvPool vpool, const int* __restrict__ block_table,
     int max_pages, const int* __restrict__ seq_lens, float* __restrict__ acc_out, float* __restrict__ ml_out, int Hq, int Hkv,
-    int G, int splits, float scale, __nv_bfloat16* __restrict__ out, long long ldo, int* __restrict__ counts, int* status) {
+    int G, int splits, int part_tokens, float scale, __nv_bfloat16* __restrict__ out, long long ldo, int* status) {
   tfb::pdl_sync();
   extern __shared__ __align__(128) uint8_t tc_smem[];
   constexpr int ROWB = D * 2 + 16;                 // padded row pitch (see tc_off)
@@ -602,7 +652,9 @@ __global__ void __launch_bounds__(TC_THREADS) paged_decode_mma_kernel(
     mbar_fence_init();
   }
   const int len = seq_lens[b];
-  const int per = ((len + splits - 1) / splits + PAGE - 1) / PAGE * PAGE;
+  const int parts = parts_of(len, splits, part_tokens);
+  if (sp_idx >= parts) return;
+  const int per = ((len + parts - 1) / parts + PAGE - 1) / PAGE * PAGE;
   const int t_begin = sp_idx * per, t_end = min(len, t_begin + per);
   const int* bt = block_table + (long long)b * max_pages;
 
@@ -780,9 +832,9 @@ __global__ void __launch_bounds__(TC_THREADS) paged_decode_mma_kernel(
     }
     head_m[g] = M;
     head_l[g] = L;
-    if (splits > 1) {
+    if (parts > 1) {
       const long long base = (((long long)b * Hq + hk * G + g) * splits + sp_idx);
-      __stcg(reinterpret_cast<float2*>(ml_out) + base, make_float2(M, L));
+      reinterpret_cast<float2*>(ml_out)[base] = make_float2(M * 0.6931471805599453f, L);      // natural logarithm, as from the other kernel
     }
   }
   __syncthreads();
@@ -795,63 +847,41 @@ __global__ void __launch_bounds__(TC_THREADS) paged_decode_mma_kernel(
       const float mw = red_m[w * 8 + g];
       if (mw != -INFINITY) v += red_o[(w * 8 + g) * D + d] * exp2f(mw - M);
     }
-    if (splits == 1) {
+    if (parts == 1) {
       const float L = head_l[g];
       out[(long long)b * ldo + (hk * G + g) * D + d] = __float2bfloat16(L > 0.f ? v / L : 0.f);
     } else {
-      __stcg(acc_out + (((long long)b * Hq + hk * G + g) * splits + sp_idx) * D + d, v);
+      acc_out[(((long long)b * Hq + hk * G + g) * splits + sp_idx) * D + d] = v;
     }
-  }
-  if (splits == 1) return;
-  // the block that arrives last merges the splits of its heads, in their order, and leaves the counter at zero
-  volatile int* last = reinterpret_cast<volatile int*>(head_l + 8);
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    int* c = counts + b * Hkv + hk;
-    *last = atomicAdd(c, 1) == splits - 1;
-    if (*last) *c = 0;
-  }
-  __syncthreads();
-  if (!*last) return;
-  __threadfence();
-  for (int i = tid; i < G * D; i += TC_THREADS) {
-    const int g = i / D, d = i % D;
-    const long long base = ((long long)b * Hq + hk * G + g) * splits;
-    const float2* ml = reinterpret_cast<const float2*>(ml_out) + base;
-    float M = -INFINITY, L = 0.f, v = 0.f;
-    for (int s0 = 0; s0 < splits; s0 += 4) {                 // four splits' loads in flight
-      float2 x[4];
-      float a[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int s = min(s0 + k, splits - 1);
-        x[k] = __ldcg(ml + s);
-        a[k] = __ldcg(acc_out + (base + s) * D + d);
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (s0 + k >= splits || x[k].x == -INFINITY) continue;
-        const float m_new = fmaxf(M, x[k].x), f = exp2f(M - m_new), e = exp2f(x[k].x - m_new);
-        L = L * f + x[k].y * e;
-        v = v * f + a[k] * e;
-        M = m_new;
-      }
-    }
-    out[(long long)b * ldo + (hk * G + g) * D + d] = __float2bfloat16(L > 0.f ? v / L : 0.f);
   }
 }
 
 template <int MODE, int D>
+constexpr int DECODE_SMEM = (16 + (TC_THREADS / 32) * 2 * TC_CHUNK) * (D * 2 + 16) + 128;   // Q tile, four K/V tile pairs, barriers
+
+template <int MODE, int D>
+static int decode_mma_resident() {
+  static DeviceOnce once;
+  auto kern = paged_decode_mma_kernel<MODE, D>;
+  int n = 0;
+  if (ensure_dyn_smem(once, kern, DECODE_SMEM<MODE, D>) || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, TC_THREADS, DECODE_SMEM<MODE, D>) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+template <int MODE, int D>
 static int launch_decode_mma(dim3 grid, cudaStream_t st, const __nv_bfloat16* q, long long ldq, KvPool k, KvPool v, const int* bt,
-                             int max_pages, const int* lens, float* acc, float* ml, int Hq, int Hkv, int G, int splits, float scale,
-                             __nv_bfloat16* o, long long ldo, int* counts, int* status) {
-  constexpr int SMEM = (16 + (TC_THREADS / 32) * 2 * TC_CHUNK) * (D * 2 + 16) + 128;   // Q tile, four K/V tile pairs, barriers
-  static_assert(SMEM >= int(sizeof(float)) * (64 + 4 * 8 * D + 17), "the merge buffers reuse the staging area");
+                             int max_pages, const int* lens, float* acc, float* ml, int Hq, int Hkv, int G, int splits, int part_tokens,
+                             float scale, __nv_bfloat16* o, long long ldo, int* status) {
+  constexpr int SMEM = DECODE_SMEM<MODE, D>;
+  static_assert(SMEM >= int(sizeof(float)) * (64 + 4 * 8 * D + 16), "the merge buffers reuse the staging area");
   static DeviceOnce once;
   auto kern = paged_decode_mma_kernel<MODE, D>;
   if (int e = ensure_dyn_smem(once, kern, SMEM)) return e;
-  tfb::launch_k_pdl(kern, grid, TC_THREADS, SMEM, st, q, ldq, k, v, bt, max_pages, lens, acc, ml, Hq, Hkv, G, splits, scale, o, ldo, counts, status);
+  tfb::launch_k_pdl(kern, grid, TC_THREADS, SMEM, st, q, ldq, k, v, bt, max_pages, lens, acc, ml, Hq, Hkv, G, splits, part_tokens, scale, o, ldo,
+                    status);
   return int(cudaGetLastError());
 }
 
@@ -1016,14 +1046,27 @@ TFB_API int tfb_kv_rope_append(void* x, long long ld, const float* cos_t, const 
   return int(cudaGetLastError());
 }
 
-// q: [B, ldq] bf16 (query head h at column h*D).  acc_ws: fp32 [B*Hq*splits*D], ml_ws: fp32 [B*Hq*splits*2] (8-byte aligned), counts: int
-// [B*Hkv], zero before the first call and left at zero by every call.
+// Blocks of the tensor-core decode kernel that the current device holds at once; < 0: error.
+TFB_API int tfb_paged_decode_blocks(int D, int mode) {
+  int n = 0;
+#define TFB_GO(MODE)                                    \
+  if (mode == MODE && D == 64) n = decode_mma_resident<MODE, 64>(); \
+  if (mode == MODE && D == 128) n = decode_mma_resident<MODE, 128>()
+  TFB_GO(KV_BF16);
+  TFB_GO(KV_FP8);
+  TFB_GO(KV_Q4);
+#undef TFB_GO
+  return n > 0 ? n * tfb::sm_count() : int(TFB_ERR_ARG);
+}
+
+// q: [B, ldq] bf16 (query head h at column h*D).  acc_ws: fp32 [B*Hq*splits*D] (16-byte aligned), ml_ws: fp32 [B*Hq*splits*2] (8-byte aligned).
+// part_tokens > 0: a sequence takes no more than one of the splits per so many tokens (tensor-core kernel).
 // status: the device status word (a bulk copy that does not land within the wait bound is reported there).
 TFB_API int tfb_paged_decode(const void* q, long long ldq, void* k_data, void* k_scale, void* v_data, void* v_scale,
                              const int* block_table, int max_pages, const int* seq_lens, void* o, long long ldo,
-                             float* acc_ws, float* ml_ws, int* counts, int B, int Hq, int Hkv, int D, int splits, int mode,
+                             float* acc_ws, float* ml_ws, int B, int Hq, int Hkv, int D, int splits, int part_tokens, int mode,
                              float scale, long long pool_rows, int* status, void* stream) {
-  if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv || splits < 1) return TFB_ERR_ARG;
+  if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv || splits < 1 || part_tokens < 1) return TFB_ERR_ARG;
   const int G = Hq / Hkv;
   KvPool kp{k_data, k_scale, pool_rows}, vp{v_data, v_scale, pool_rows};
   dim3 grid(B, Hkv, splits);
@@ -1037,9 +1080,9 @@ TFB_API int tfb_paged_decode(const void* q, long long ldq, void* k_data, void* k
   const bool mma_ok = !simt && G <= 8 && (ldq % 8) == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
 #define TFB_GO(MODE)                                                                                                  \
   rc = mma_ok ? ((D == 64) ? launch_decode_mma<MODE, 64>(grid, st, Q, ldq, kp, vp, block_table, max_pages, seq_lens, acc_ws, ml_ws, \
-                                                         Hq, Hkv, G, splits, scale, out, ldo, counts, status)         \
+                                                         Hq, Hkv, G, splits, part_tokens, scale, out, ldo, status)    \
                            : launch_decode_mma<MODE, 128>(grid, st, Q, ldq, kp, vp, block_table, max_pages, seq_lens, acc_ws,       \
-                                                          ml_ws, Hq, Hkv, G, splits, scale, out, ldo, counts, status)) \
+                                                          ml_ws, Hq, Hkv, G, splits, part_tokens, scale, out, ldo, status)) \
      : (D == 64) ? launch_decode_g<MODE, 64>(G, grid, st, Q, ldq, kp, vp, block_table, max_pages, seq_lens, acc_ws,   \
                                              ml_ws, Hq, Hkv, splits, scale)                                           \
                  : launch_decode_g<MODE, 128>(G, grid, st, Q, ldq, kp, vp, block_table, max_pages, seq_lens, acc_ws,  \
@@ -1049,7 +1092,8 @@ TFB_API int tfb_paged_decode(const void* q, long long ldq, void* k_data, void* k
   else if (mode == KV_Q4) { TFB_GO(KV_Q4); }
   else return TFB_ERR_ARG;
 #undef TFB_GO
-  if (rc || mma_ok) return rc;
-  tfb::launch_k_pdl(paged_combine_kernel, dim3(B, Hq), 128, 0, st, acc_ws, ml_ws, static_cast<__nv_bfloat16*>(o), ldo, Hq, D, splits);
+  if (rc || (mma_ok && splits == 1)) return rc;
+  tfb::launch_k_pdl(D == 64 ? paged_combine_kernel<64> : paged_combine_kernel<128>, dim3((B * Hq + 3) / 4), 128, 0, st, acc_ws, ml_ws, out, ldo, seq_lens,
+                    B * Hq, Hq, splits, mma_ok ? part_tokens : 0);
   return int(cudaGetLastError());
 }

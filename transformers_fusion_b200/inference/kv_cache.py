@@ -22,8 +22,10 @@ MODES = {"bf16": 0, "fp8": 1, "q4": 2}
 _lib.register("tfb_kv_append", [c_p, c_ll, c_i, c_i, c_p, c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_ll, c_p])
 _lib.register("tfb_kv_rope_append", [c_p, c_ll, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_ll, c_p])
 _lib.register("tfb_kv_gather", [c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_ll, c_i, c_i, c_i, c_ll, c_p])
-_lib.register("tfb_paged_decode", [c_p, c_ll, c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_ll, c_p, c_p, c_p, c_i, c_i, c_i,
-                                   c_i, c_i, c_i, c_f, c_ll, c_p, c_p])
+_lib.register("tfb_paged_decode", [c_p, c_ll, c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_ll, c_p, c_p, c_i, c_i, c_i,
+                                   c_i, c_i, c_i, c_i, c_f, c_ll, c_p, c_p])
+_lib.register("tfb_paged_decode_blocks", [c_i, c_i])
+_RESIDENT = {}       # (device, head dim, mode) -> blocks of the decode kernel that run at once
 
 
 class PageAllocator:
@@ -193,6 +195,22 @@ class PagedKVCache:
                                        stream()), "kv_gather")
         return ok, ov
 
+    def _splits(self, B, max_len, device):
+        """(splits, tokens per split at least) of a decode step over a table of ``max_len`` tokens per sequence; how many of the splits a sequence uses
+        goes by its own length, on the device.  While two or more blocks per sequence and kv head run at once: as many as do, of 128 tokens
+        at least (the four warps of a block take 32 at a time).  Otherwise long sequences are cut so that a batch of different lengths does not wait for its
+        longest.  Measured, us, for 1 / 2 / 3 / 4 / 6 / 8 / 16 splits at heads of 128, 8 kv heads: 1 sequence of 230 tokens 8.4 / 6.9 / 7.0 / 7.0 / 7.1 / 7.2 /
+        6.7; 8 of 2200 66 / 37 / 27 / 26 / 21 / 26 / 25; 16 of 600 24 / 19 / 16 / 18 / 19 / 20 / 30; 32 of 400 - 1200 39 / 33 / 30 / 31 / 34 / 36 / 56; 64
+        of 180 19 / 22 / 25 / 30 / 40 / 48 / 77."""
+        key = (device, self.D, self.mode)
+        if key not in _RESIDENT:
+            _RESIDENT[key] = _lib.lib().tfb_paged_decode_blocks(self.D, MODES[self.mode])
+            assert _RESIDENT[key] > 0
+        room = _RESIDENT[key] // max(1, B * self.Hkv)
+        if room >= 2:
+            return min(16, room, (max_len + 127) // 128), 128
+        return max(1, min(8 * 148 // max(1, B * self.Hkv), max_len // 384)), 384
+
     def decode(self, layer, q, block_table, seq_lens, Hq, scale=None, splits=None):
         """q [B, Hq*D] bf16 -> o [B, Hq*D] attending over the first seq_lens[b] cached tokens of each sequence."""
         B = q.shape[0]
@@ -211,26 +229,20 @@ class PagedKVCache:
                 s = torch.einsum("hgd,nhd->hgn", qq, kk) * scale
                 out[b] = torch.einsum("hgn,nhd->hgd", torch.softmax(s, -1), vv).reshape(-1)
             return out.to(q.dtype)
+        part = 1
         if splits is None:
-            max_len = block_table.shape[1] * PAGE
-            # as many blocks as run at once (three per SM at heads of 128, four at 64), each over 128 tokens at least (its four warps
-            # take 32 at a time); powers of two, so that few splits end in a partly filled round.  Measured, us, for 1 / 2 / 4 / 8 / 16
-            # splits: 64 sequences of 180 tokens, 8 kv heads of 128 18.5 / 28.3 / 38.0 / 65.3 / 110; 8 of 2200 64.8 / 38.5 / 28.3 / 32.5 / 37.2
-            # (fp8 84 / 48 / 33 / 38 / 49); 4 of 2000 82 / 47 / 27 / 24 / 28; 16 of 300, 8 heads of 64 12.9 / 9.8 / 8.2 / 13.3 / 20.8
-            splits = max(1, min(16, (3 if D == 128 else 4) * 148 // max(1, B * Hkv), max_len // 128))
-            splits = 1 << (splits.bit_length() - 1)
+            splits, part = self._splits(B, block_table.shape[1] * PAGE, q.device)
         key = (B, Hq, splits)
         if key not in self._ws:
             self._ws[key] = (torch.empty(B * Hq * splits * D, dtype=torch.float32, device=q.device),
-                             torch.empty(B * Hq * splits * 2, dtype=torch.float32, device=q.device),
-                             torch.zeros(B * Hkv, dtype=torch.int32, device=q.device))
-        acc, ml, counts = self._ws[key]
+                             torch.empty(B * Hq * splits * 2, dtype=torch.float32, device=q.device))
+        acc, ml = self._ws[key]
         o = torch.empty((B, Hq * D), dtype=q.dtype, device=q.device)
         kp, vp = self.k[layer], self.v[layer]
         check(_lib.lib().tfb_paged_decode(q.data_ptr(), q.stride(0), kp.data.data_ptr(), ptr(kp.scale),
                                           vp.data.data_ptr(), ptr(vp.scale), block_table.data_ptr(),
                                           block_table.shape[1], seq_lens.data_ptr(), o.data_ptr(), o.stride(0),
-                                          acc.data_ptr(), ml.data_ptr(), counts.data_ptr(), B, Hq, Hkv, D, splits, MODES[self.mode],
+                                          acc.data_ptr(), ml.data_ptr(), B, Hq, Hkv, D, splits, part, MODES[self.mode],
                                           float(scale), self.num_pages * PAGE, _lib.status_word(q.device).data_ptr(),
-                                          stream()), "paged_decode", 1 if Hq // Hkv <= 8 else 2)
+                                          stream()), "paged_decode", 1 if splits == 1 else 2)
         return o

@@ -67,17 +67,6 @@ struct RowsParams {
 #endif
 };
 
-// The vote of the 128 epilogue threads (barrier 1): all of them or none go on.
-__device__ __forceinline__ bool all_of_128(bool ok) {
-  int r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 1, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"(int(ok))
-      : "memory");
-  return r != 0;
-}
-
 template <int FMT, int MP>
 __global__ void __launch_bounds__(RowsPlan<FMT, MP>::THREADS, 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w, const RowsParams p) {
@@ -294,16 +283,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
           if (c + j < p.M) static_cast<__nv_bfloat16*>(p.C)[(c + j) * p.ldc + n] = __float2bfloat16(v[j]);
       }
     };
-    // blocks that share tile t: the ones whose runs hold its first and its last unit, and those in between
-    auto first_of = [&](int t) { return int((((long long)t * p.KB + 1) * G - 1) / U); };
-    auto last_of = [&](int t) { return int(((long long)(t + 1) * p.KB * G - 1) / U); };
-    // one thread counts this block in at a shared tile; true for the block that arrives last, which leaves the counter at zero
-    auto arrive_last = [&](int t) {
-      const int others = last_of(t) - first_of(t);
-      const bool last = atomicAdd(p.count + t, 1) == others;
-      if (last) p.count[t] = 0;
-      return last;
-    };
+    bool gave_up = false;
     int seg = 0;
     for (int u = u0; u < u1; ++seg) {
       const int t = u / p.KB, kb0 = u - t * p.KB, end = min(u1, (t + 1) * p.KB), ab = seg & 1;
@@ -311,26 +291,17 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
       const int n = p.glu ? t * (RW_BN / 2) + (nl & 63) : t * RW_BN + nl;
       const bool live = n < p.N;
       const float bias = p.bias && live ? __bfloat162float(p.bias[n]) : 0.f;
-      bool ok = mbar_wait_sleep_warp(bar_tfull + ab * 8, (seg >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL, 20);
+      // A warp whose wait ran out (the status word says so, the block's results are wrong) goes on with what the accumulator holds: the
+      // other three meet it at the barriers below, and the block has to arrive at every tile that it shares - the counters outlive the
+      // launch, and one left above zero would let a later product add sums that are not there yet.
+      gave_up |= !mbar_wait_sleep_warp(bar_tfull + ab * 8, (seg >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL, 20);
 #ifdef TFB_BOUNDS_CHECK
       if (cta == p.give_up) {
-        ok = false;
+        gave_up = true;
         *abort_flag = 1;
         report(p.status, ST_TIMEOUT_TMEM_FULL);
       }
 #endif
-      // The four warps meet at barriers below, so they go on or give up together.  A block that gives up (a wait ran out: the status
-      // word says so, its results are wrong) still arrives at every tile that it shares: the counters outlive the launch, and
-      // one left above zero would let a later product add sums that are not there yet.
-      if (!all_of_128(ok)) {
-        for (int v = u; v < u1;) {
-          const int tv = v / p.KB, ve = min(u1, (tv + 1) * p.KB);
-          if (nl == 0 && !(v == tv * p.KB && ve == (tv + 1) * p.KB)) (void)arrive_last(tv);
-          v = ve;
-        }
-        if (nl == 0) drain();
-        break;
-      }
       tc_fence_after();
       // partial sums: [four rows of x][128 weight rows] of four floats
       float4* slot = reinterpret_cast<float4*>(p.ws + ((long long)cta * 2 + (u == u0 ? 0 : 1)) * (MP * 128)) + nl;
@@ -352,10 +323,15 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
       tc_fence_before();
       mbar_arrive(bar_tempty + ab * 8);
       if (!whole) {
-        const int c0 = first_of(t), c1 = last_of(t);
+        // blocks that share the tile: the ones whose runs hold its first and its last unit, and those in between
+        const int c0 = int((((long long)t * p.KB + 1) * G - 1) / U), c1 = int(((long long)(t + 1) * p.KB * G - 1) / U);
         __threadfence();
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (nl == 0) *last_flag = arrive_last(t);
+        if (nl == 0) {
+          const int before = atomicAdd(p.count + t, 1);
+          *last_flag = before == c1 - c0;
+          if (before == c1 - c0) p.count[t] = 0;
+        }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (*last_flag) {
           __threadfence();
@@ -402,6 +378,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constan
       }
       u = end;
     }
+    if (gave_up && lane == 0) drain();
   }
   tc_fence_before();
   __syncthreads();
@@ -625,7 +602,8 @@ TFB_API int tfb_test_rows_give_up(int cta) {
 #endif
 
 // out [M, N] = act(alpha * x [M, K] . W [N, K]^T + bias) + residual, M <= 128; out bf16, or fp32 with out_f32.  w_static: the caller promises
-// that the kernel launched just before this one on the stream does not write W.
+// that the kernel launched just before this one on the stream does not write W.  (The models' products come through gemm_bf16.cu, which
+// chooses; this entry takes the streaming form at every size, for tests and measurements.)
 TFB_API int tfb_gemm_rows(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo, int M, int N, int K, const void* bias,
                           const void* residual, long long ldr, float alpha, int act, int out_f32, int w_static, int* status, void* stream) {
   const int rc = tfb::gemm_rows(x, ldx, w, ldw, nullptr, nullptr, -1, 0, out, ldo, M, N, K, K, bias, residual, ldr, alpha, act, out_f32, w_static,

@@ -116,9 +116,12 @@ def test_gemm_tile_edge_sweep(a_mn, b_mn):
 
 
 @pytest.mark.parametrize("am,bm", [(False, False), (False, True), (True, False), (True, True)])
-@pytest.mark.parametrize("M,N,K", [(136, 2816, 512), (256, 256, 64), (304, 1000, 776), (512, 264, 200), (1000, 1536, 1408), (2048, 4096, 4096)])
+@pytest.mark.parametrize("M,N,K", [(136, 2816, 512), (256, 256, 64), (304, 1000, 776), (512, 264, 200), (1000, 1536, 1408), (2048, 4096, 4096),
+                                   (2056, 1544, 840), (2568, 2056, 584), (2568, 2056, 264),      # pairs: one wave, two; the least depth
+                                   (2056, 1544, 768), (2568, 2056, 256), (4616, 1000, 776)])     # just not: too shallow twice, a wave more
 def test_gemm_on_cta_pairs(M, N, K, am, bm):
-    """256 x 256 tiles of CTA pairs: a second half past the last row, ragged columns and depth, split sums, every epilogue."""
+    """256 x 256 tiles of CTA pairs: a second half past the last row, ragged columns and depth, split sums, every epilogue.  (The small shapes run
+    on pairs where they accumulate, and in narrower tiles of single CTAs otherwise.)"""
     a = torch.randn((K, M) if am else (M, K), device="cuda").bfloat16()
     b = (torch.randn((K, N) if bm else (N, K), device="cuda") * K ** -0.5).bfloat16()
     ref = (a.t() if am else a).double() @ (b if bm else b.t()).double()

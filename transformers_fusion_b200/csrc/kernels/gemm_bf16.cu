@@ -1031,6 +1031,45 @@ __global__ void __launch_bounds__(256) splitk_finalize_kernel(float* __restrict_
   }
 }
 
+// Few rows: the product streams the weights once and is bound by how evenly the work items cover the SMs.  The split count whose item
+// count (tiles x splits) fills whole waves best, keeping at least 8 k-blocks per split; the partials are accumulated in fp32 and finished in a
+// second kernel.  `fill`: the share of the waves that the tiles alone fill.
+static int few_row_splits(int M, int N, int K, int sms, double* fill) {
+  using namespace tfb;
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + (N > 128 ? 255 : 127)) / (N > 128 ? 256 : 128));
+  const int total_kb = (K + BK - 1) / BK;
+  int best_s = 1;
+  double best_eff = 0.0, eff1 = double(tiles) / double((tiles + sms - 1) / sms * sms);
+  for (int sp = 1; K >= 16 * BK && sp <= 16 && sp * 8 <= total_kb; ++sp) {
+    const long long items = tiles * sp;
+    const double eff = double(items) / double((items + sms - 1) / sms * sms);
+    if (eff > best_eff + 0.02) { best_eff = eff; best_s = sp; }
+  }
+  if (fill) *fill = eff1;
+  return best_eff < eff1 + 0.1 ? 1 : best_s;          // the workspace pass costs about a tenth of a weight-streaming product
+}
+
+// Products of few rows: whether the streaming form of gemm_rows.cu (tiles of 128 weight rows) is faster than this file's kernels with their
+// split over K.  us, this file / streaming / streaming with the weights fetched ahead (w_static):
+//   - Short K: a block holds many whole tiles, and its time is their drains.  32000 x 512 at 16 / 64 rows 11.1 / 11.8 / 11.8 and 11.3 / 17.0 / 16.2;
+//     50304 x 768 19.3 / 20.4 / 18.4 and 19.9 / 25.1 / 22.8.
+//   - Where this file's tiles fill their waves without a split, one to a block, theirs is one drain: 32000 x 1024 at 8 / 64 rows 16.7 / 18.0 / 16.3
+//     and 16.4 / 21.9 / 20.5, 32000 x 2048 at 64 26.7 / 33.6 / 31.1 (but 32000 x 4096, which it splits, 72 / 54 / 51).
+//   - Many blocks to a tile: they meet in memory, more of it with more rows.  4096 x 4096 at 16 / 64 rows 13.7 / 12.8 / 12.6 and 16.0 / 18.0 / 17.2,
+//     2048 x 8192 at 32 rows 13.9 / 14.9 / 15.2, 6144 x 4096 at 64 18.8 / 19.5 / 18.5, 8192 x 2048 17.8 / 17.1 / 15.9.
+//   - Without the early fetch the longer streams win nothing while this file's kernels fill the machine: 4096 x 14336 at 16 rows 26.1 / 26.4 / 23.9,
+//     8192 x 8192 28.9 / 29.6 / 25.7; from 16384 weight rows on they do not (28672 x 4096 at 16 / 64 / 128 rows 48.6 / 45.4 / 42.1, 63 / 49 / 47
+//     and 86 / 57 / 56).
+static bool rows_pay(int M, int N, int K, long long tiles, int w_static) {
+  const int KB = (K + tfb::BK - 1) / tfb::BK;
+  if (KB < (M <= 16 && w_static ? 12 : 16)) return false;
+  double fill;
+  if ((M > 16 || !w_static) && few_row_splits(M, N, K, tfb::sm_count(), &fill) == 1 && fill >= 0.8) return false;
+  if (M > 64) return tiles >= 128;
+  if (w_static) return M <= 16 || tiles >= 48;
+  return (M <= 16 || tiles >= 64) && (KB <= 64 || tiles >= 128);
+}
+
 static int gemm_impl(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* C,
                      long long ldc, int M, int N, int K, const void* bias, const void* residual, long long ldr,
                      float alpha, int act, int out_mode, int max_ctas, const TfbGemmGroup* grp, int* status,
@@ -1039,13 +1078,8 @@ static int gemm_impl(const void* A, long long lda, int a_mn, const void* B, long
   if (M <= 0 || N <= 0 || K <= 0) return TFB_ERR_ARG;
   if (out_mode != 0 && (bias || residual || act)) return TFB_ERR_ARG;
   if (!grp && !tp && !a_mn && !b_mn && out_mode != 2 && max_ctas <= 0 && M <= 128) {
-    // Few rows: the weights are streamed once.  Above 64 rows only where the tiles of 128 weight rows alone nearly fill the machine
-    // (us, streaming form against this kernel's split form with its finalize: 28672 x 4096 at 128 rows 53.8 against 86.5, 64 rows 46.9
-    // against 62.9, 1 row 44.7 against 43.9; 4096 x 4096 at 128 rows 20.4 against 18.9, 64 rows 15.6 against 15.4, 1 row 12.4
-    // against 13.0; 4096 x 14336 at 128 rows 34.8 against 31.5, 64 rows 29.0 against 28.2, 1 row 26.5 against 24.9).  With the weights
-    // fetched ahead (w_static) the streaming form gains another 1 - 3 us.
     int rc0 = gemm_skinny(A, lda, B, ldb, C, ldc, M, N, K, bias, residual, ldr, alpha, act, out_mode == 1, stream);
-    if (rc0 == TFB_NOT_TAKEN && (M <= 64 || N >= 16384))
+    if (rc0 == TFB_NOT_TAKEN && rows_pay(M, N, K, (N + 127) / 128, w_static))
       rc0 = gemm_rows(A, lda, B, ldb, nullptr, nullptr, -1, 0, C, ldc, M, N, K, K, bias, residual, ldr, alpha, act, out_mode == 1, w_static, status,
                       stream);
     if (rc0 != TFB_NOT_TAKEN) return rc0;
@@ -1054,22 +1088,9 @@ static int gemm_impl(const void* A, long long lda, int a_mn, const void* B, long
   const int E = (gmode != 0) ? grp->num_experts : 1;
   if (gmode == 2 && out_mode == 0) return TFB_ERR_ARG;
   if (gmode == 0 && !tp && out_mode != 2 && M <= 256 && K >= 16 * BK) {
-    // Few rows: the product streams the weights once and is bound by how evenly the work items cover the SMs.  Pick the
-    // split count whose item count (tiles x splits) fills whole waves best, keeping at least 8 k-blocks per split;
-    // accumulate the partials in fp32 and finish in a second kernel.
-    const long long tiles_w = (long long)((M + BM - 1) / BM) * ((N + (N > 128 ? 255 : 127)) / (N > 128 ? 256 : 128));
     const long long ldw = (N + 3) / 4 * 4;
     const int all_sms = (max_ctas > 0 && max_ctas < sm_count()) ? max_ctas : sm_count();
-    const int total_kb0 = (K + BK - 1) / BK;
-    int best_s = 1;
-    double best_eff = 0.0, eff1 = 0.0;
-    for (int sp = 1; sp <= 16 && sp * 8 <= total_kb0; ++sp) {
-      const long long items = tiles_w * sp;
-      const double eff = double(items) / double((items + all_sms - 1) / all_sms * all_sms);
-      if (sp == 1) eff1 = eff;
-      if (eff > best_eff + 0.02) { best_eff = eff; best_s = sp; }
-    }
-    if (best_eff < eff1 + 0.1) best_s = 1;             // the workspace pass costs about a tenth of a weight-streaming product
+    const int best_s = few_row_splits(M, N, K, all_sms, nullptr);
     if (best_s > 1 && (long long)M * ldw <= SPLITK_WS_ELEMS) {
       cudaStream_t st0 = static_cast<cudaStream_t>(stream);
       if (float* ws = splitk_workspace(st0)) {
@@ -1097,8 +1118,21 @@ static int gemm_impl(const void* A, long long lda, int a_mn, const void* B, long
     if (narrow_env && BN == 256 && gmode != 2 && out_mode != 2 && t256 < sms && t128 > t256 && t128 <= sms) BN = 128;
   }
   static const int raster_env = [] { const char* e = getenv("TFB_GEMM_RASTER"); return e ? atoi(e) : -1; }();
-  // Tiles of 256 columns of a plain product with more than one tile row run on CTA pairs.
-  const bool want_pair = BN == 256 && gmode == 0 && !tp && M > BM && sms >= 2;
+  // Tiles of 256 columns of a plain product with more than one tile row run on CTA pairs, except
+  //   - where few k-blocks leave the set-up of the cluster in sight: one wave of at most 12 (us, pairs / single CTAs: 777 x 2816 x 512 9.2 / 8.6, 1024 x
+  //     3072 x 768 10.7 / 10.0; 512 x 6144 x 4096 27.5 / 30.4), or at most 4 (4096 x 4096 x 129 accumulated 22.2 / 19.7; 300 instead of 129
+  //     23.2 / 24.6);
+  //   - where their larger tiles take a wave more, and a wave on pairs at 0.85 of the time does not make up for it (4662 x 1000 x 776, 2 waves against
+  //     1, 24.3 / 18.0; 4662 x 3072 x 768, 4 against 3, 22.7 / 21.5; 4662 x 4096 x 14336, 5 against 4, 395 / 369; 777 x 28672 x 4096, 7 against
+  //     6, 160 / 160) - but not for one or two tile rows over long K, bound by the weights that single CTAs read once more (300 x 28672 x
+  //     4096, 4 against 3, 88 / 110).
+  bool want_pair = BN == 256 && gmode == 0 && !tp && M > BM && sms >= 2;
+  if (want_pair) {
+    const int kbs = (K + BK - 1) / BK, pairs = sms / 2;
+    const long long tm2 = (M + 2 * BM - 1) / (2 * BM), tn = (N + BN - 1) / BN, tm1 = (M + BM - 1) / BM;
+    const long long waves2 = (tm2 * tn + pairs - 1) / pairs, waves1 = (tm1 * tn + sms - 1) / sms;
+    if (kbs <= 4 || (waves2 == 1 && kbs <= 12) || (waves2 * 17 > waves1 * 20 && (tm2 > 2 || kbs < 32 || waves1 == 1))) want_pair = false;
+  }
   CUtensorMap ta, tb;
   int rc;
   if (!a_mn) rc = make_tmap_2d(&ta, A, 2, K, M, lda * 2, BK, BM);
@@ -1301,11 +1335,16 @@ TFB_API int tfb_gemm_glu(const void* A, long long lda, const void* B, long long 
   if (M <= BM) {
     int rc = gemm_skinny_glu(A, lda, B, ldb, C, ldc, M, F, K, act, stream);
     // above 32 rows the exchange of the halves in the epilogue costs more than the gating kernel (64 sequences of the 8b widths: 104 against 101 ms a pass)
-    if (rc == TFB_NOT_TAKEN && M <= 32) rc = gemm_rows_glu(A, lda, B, ldb, C, ldc, M, F, K, act, w_static, status, stream);
+    if (rc == TFB_NOT_TAKEN && M <= 32 && rows_pay(M, 2 * F, K, (F + 63) / 64, w_static)) rc = gemm_rows_glu(A, lda, B, ldb, C, ldc, M, F, K, act, w_static, status, stream);
     return rc == TFB_NOT_TAKEN ? int(TFB_ERR_ARG) : rc;
   }
   CUtensorMap ta, tb, tc;
   if ((reinterpret_cast<uintptr_t>(C) & 15) || ldc % 8 || sm_count() < 2) return TFB_ERR_ARG;
+  // Its tiles of 256 x 128 outputs have to fill their waves on pairs: us, product and gating kernel / this: F x K = 1408 x 512 at 300 rows (0.3 waves)
+  // 9.2 / 11.1, 3072 x 768 at 300 (0.65) 10.7 / 12.5, 5632 x 2048 at 300 (1.2) 22.7 / 28.9; 14336 x 4096 at 300 (3.03) 116 / 90, 8192 x 1024 at 129 (0.9)
+  // 16.5 / 15.0.  Up to 256 rows over long K the other path has a pass over its split sums: 5632 x 2048 at 129 (0.6) 30.9 / 19.4.
+  const long long tiles = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((F + BM - 1) / BM), pairs = sm_count() / 2;
+  if (tiles * 4 < (tiles + pairs - 1) / pairs * pairs * 3 && (M > 2 * BM || K < 16 * BK || tiles * 5 < pairs)) return TFB_ERR_ARG;
   if (int rc = make_tmap_2d(&ta, A, 2, K, M, lda * 2, BK, BM)) return rc;
   if (int rc = make_tmap_2d(&tb, B, 2, K, 2ull * F, ldb * 2, BK, BM)) return rc;
   if (int rc = make_tmap_3d(&tc, C, 2, F, M, 1, ldc * 2, (unsigned long long)ldc * 2 * M, 64, 32, 1)) return rc;

@@ -176,7 +176,7 @@ SKINNY_K = 8192   # (K <= 8192: every block reads all of x), else the streaming 
 
 def gemm_wq(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor] = None, splits: int = 0,
             out: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None, w_static: bool = False) -> torch.Tensor:
-    """y [M, N] = x [M, K] @ dequant(pw)^T (+ bias) (+ residual).  bf16 in / out.  M <= 32 (decode): one launch (skinny_wq.cu, gemm_rows.cu); M < 2048:
+    """y [M, N] = x [M, K] @ dequant(pw)^T (+ bias) (+ residual).  bf16 in / out.  M <= 32 (decode): one launch (skinny_wq.cu, gemm_rows.cu) where that is faster (_rows_pay); M < 2048:
     fused-dequant kernel with 128-row tiles; larger: bf16 image in scratch + bf16 GEMM.
     ``out`` [M, N] bf16: where the result goes (e.g. the staging buffer of a collective).  ``w_static``: the kernel launched just before does not
     write the packed weight (it may then be fetched ahead of that kernel's end)."""
@@ -193,6 +193,20 @@ def gemm_wq(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor] = No
     return y
 
 
+def _rows_pay(M, pw):
+    """Whether the one-launch forms are the faster ones; us, split form / one launch, at 32 rows: several blocks meet at each 128-row tile, and that costs
+    more than the finalize where they are many and their share of K is short (4096 x 4096, 4.6 blocks of 14 k-blocks, fp4 / mxfp8 13.6 / 14.3 and 14.1 /
+    14.6; 2048 x 8192, 9 of 14, 13.0 / 15.7; 512 x 1408, 5.5 of 4, 8.4 / 9.2; but 4096 x 14336, 4.6 of 48, 30.1 / 29.1; 6144 x 4096, 3.1 of 21,
+    18.1 / 17.3; 1536 x 512, 2 of 4, 8.4 / 7.0).  From 9 rows on, mxfp8 codes that one block per SM walks alone: 2048 x 8192 at 16 rows 12.7 / 14.1
+    (int8 12.9 / 12.7, int4 12.3 / 11.4)."""
+    sms = _lib.lib().tfb_sm_count()
+    if M <= 16:
+        return M <= 8 or pw.fmt != FORMATS["mxfp8"] or pw.Np >= 16 * sms or pw.Kp <= 4096
+    tiles, kb = pw.Np // 128, pw.Kp // 64
+    share = min(sms, max(1, tiles * kb // 4)) / tiles
+    return share <= 3.2 or kb / share >= 32
+
+
 def _gemm_rows(x, pw, bias, residual, dst, w_static):
     """The one-launch forms; None where the operands' layout does not fit them (the general form copies or refuses them)."""
     M, K = x.shape
@@ -206,6 +220,8 @@ def _gemm_rows(x, pw, bias, residual, dst, w_static):
     out = dst if direct else torch.empty((M, pw.N), dtype=x.dtype, device=x.device)
     args = (x.data_ptr(), x.stride(0), pw.codes.data_ptr(), pw.scales.data_ptr(), pw.fmt, pw.group, out.data_ptr(), out.stride(0), M, pw.N, K, pw.Kp,
             ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0, int(w_static))
+    if not _rows_pay(M, pw):
+        return None
     if (M <= 8 or (M <= 16 and K <= SKINNY_K)) and K % 8 == 0:
         rc = _lib.lib().tfb_skinny_wq(*args, stream())
     else:

@@ -74,6 +74,8 @@ def test_attn_fwd_packed(lens, causal, D):
 @pytest.mark.parametrize("B,S,Hq,Hkv,D,causal", [
     (1, 128, 1, 1, 64, True), (2, 256, 4, 2, 64, True), (1, 1024, 8, 8, 64, True), (2, 200, 4, 1, 64, True),
     (1, 300, 2, 1, 64, False), (1, 512, 4, 2, 128, True), (2, 130, 2, 2, 128, False),
+    (37, 200, 2, 2, 64, True), (25, 200, 3, 3, 64, False),                                 # heads of 64: 148 blocks (one per SM) and more
+    (2, 577, 32, 4, 64, True), (1, 640, 59, 59, 64, True), (1, 600, 60, 60, 64, False),    # dK / dV 40, dQ 320; 295 and 300
 ])
 def test_attn_bwd(B, S, Hq, Hkv, D, causal):
     qkv = _qkv(B, S, Hq, Hkv, D)

@@ -15,9 +15,10 @@
 //   Heads of 128: two compute warpgroups take the half blocks in turn, over three slots (dK / dV: two, their accumulators fill 256
 // columns), so that the scores of the next half block are there when a warpgroup is done.
 //   Heads of 64: loops are short (nine half blocks on average at 1024 tokens) and a CTA's start and end cost as much as they do; one
-// warpgroup and one slot in 256 columns, two CTAs per SM, one working while the other starts, waits or writes.
-// Both kernels and attn_delta, us, before (two warpgroups with a slot each, one CTA per SM) -> three slots -> two CTAs per SM: 64 x
-// 1024, 8 heads of 64 804 -> 747 -> 601; 8 x 1024 112 -> 112 -> 100; 4096, 32 / 8 heads of 128 703 -> 650.
+// warpgroup and one slot in 256 columns, two CTAs per SM, one working while the other starts, waits or writes.  Launches of few CTAs have no
+// second one for an SM and take two warpgroups over three slots (launch_bwd).
+// Both kernels and attn_delta, us, two warpgroups with a slot each, one CTA per SM -> now: 64 x 1024, 8 heads of 64 769 -> 601, of which the ring
+// of slots 747; 8 x 1024 118 -> 100; 4096, 32 / 8 heads of 128 703 -> 645 (the key blocks in head order before: 876).
 // The softmax scale multiplies dK and dQ once, when they are written out.
 //
 // The reference's memory-efficient attention backward is approximate
@@ -52,20 +53,20 @@ struct AttnBwdParams {
   int* status;
 };
 
-template <int D, bool DKDV>
+template <int D, bool DKDV, int WARPGROUPS>
 struct BwdSmem {
   static constexpr int NB = D / 64;
   static constexpr int TILE = NB * AB_BOX, HALF = NB * AB_HBOX;     // a resident tile, a half block
-  static constexpr int WG = D == 64 ? 1 : 2;                        // compute warpgroups
+  static constexpr int WG = WARPGROUPS;                             // compute warpgroups; one: two blocks per SM (heads of 64)
   static constexpr int THREADS = 64 + 128 * WG;
-  static constexpr int SLOTS = D == 64 ? 1 : DKDV ? 2 : 3;          // tensor-memory slots
-  static constexpr int ACC_COL = SLOTS * 128, TMEM = D == 64 ? 256 : 512;
-  static constexpr int STAGES = D == 64 || DKDV ? 4 : 5;            // half blocks (two operands each) in flight
+  static constexpr int SLOTS = WG == 1 ? 1 : D == 128 && DKDV ? 2 : 3;      // tensor-memory slots
+  static constexpr int ACC_COL = SLOTS * 128, TMEM = WG == 1 ? 256 : 512;
+  static constexpr int STAGES = WG == 1 ? 4 : D == 64 ? 6 : DKDV ? 4 : 5;   // half blocks (two operands each) in flight
   static constexpr int RING_OFF = 2 * TILE;                         // behind two resident tiles
   static constexpr int STAT_OFF = RING_OFF + STAGES * 2 * HALF;     // [warpgroups][2 turns][64 -lse | 64 -delta] floats
   static constexpr int BAR_OFF = STAT_OFF + (DKDV ? WG * 2 * 128 * 4 : 0);
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
-  static_assert(ACC_COL + (DKDV ? 2 : 1) * D <= TMEM && TOTAL <= (D == 64 ? 115712 : 232448), "tensor and shared memory");
+  static_assert(ACC_COL + (DKDV ? 2 : 1) * D <= TMEM && TOTAL <= (WG == 1 ? 115712 : 232448), "tensor and shared memory");
 };
 
 // 16 output rows x 128 bf16 columns of an accumulator, written by one thread (its row)
@@ -84,12 +85,12 @@ __device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (
 // ------------------------------------------------------------------------------------------------
 // dK / dV
 // ------------------------------------------------------------------------------------------------
-template <int D>
-__global__ void __launch_bounds__(BwdSmem<D, true>::THREADS, D == 64 ? 2 : 1)
+template <int D, int WARPGROUPS>
+__global__ void __launch_bounds__(BwdSmem<D, true, WARPGROUPS>::THREADS, WARPGROUPS == 1 ? 2 : 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                      const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                      const AttnBwdParams p) {
-  using L = BwdSmem<D, true>;
+  using L = BwdSmem<D, true, WARPGROUPS>;
   constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES, WG = L::WG;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -372,12 +373,12 @@ __device__ __forceinline__ void dq_half_block(uint32_t tS, uint32_t tDP, float s
   }
 }
 
-template <int D>
-__global__ void __launch_bounds__(BwdSmem<D, false>::THREADS, D == 64 ? 2 : 1)
+template <int D, int WARPGROUPS>
+__global__ void __launch_bounds__(BwdSmem<D, false, WARPGROUPS>::THREADS, WARPGROUPS == 1 ? 2 : 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                    const AttnBwdParams p) {
-  using L = BwdSmem<D, false>;
+  using L = BwdSmem<D, false, WARPGROUPS>;
   constexpr int NB = L::NB, NS = L::SLOTS, ST = L::STAGES, WG = L::WG;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -575,21 +576,41 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   }
 }
 
-template <int D>
-static int launch_bwd(const CUtensorMap (&m)[8], const AttnBwdParams& p, cudaStream_t st) {
+template <int D, int WARPGROUPS>
+static int launch_dkdv(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const AttnBwdParams& p, int blocks,
+                       cudaStream_t st) {
+  using L = BwdSmem<D, true, WARPGROUPS>;
+  static DeviceOnce once;   // kernel attributes are per device: set on the first launch on each one
+  auto kern = attn_bwd_dkdv_kernel<D, WARPGROUPS>;
+  if (int e = ensure_dyn_smem(once, kern, L::TOTAL)) return e;
+  tfb::launch_k(kern, blocks, L::THREADS, L::TOTAL, st, tq, tk, tv, tdo, p);
+  return int(cudaGetLastError());
+}
+template <int D, int WARPGROUPS>
+static int launch_dq(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const AttnBwdParams& p, int blocks,
+                     cudaStream_t st) {
+  using L = BwdSmem<D, false, WARPGROUPS>;
+  static DeviceOnce once;
+  auto kern = attn_bwd_dq_kernel<D, WARPGROUPS>;
+  if (int e = ensure_dyn_smem(once, kern, L::TOTAL)) return e;
+  tfb::launch_k(kern, blocks, L::THREADS, L::TOTAL, st, tq, tk, tv, tdo, p);
+  return int(cudaGetLastError());
+}
+
+static int launch_bwd(int D, const CUtensorMap (&m)[8], const AttnBwdParams& p, cudaStream_t st) {
   // boxes of 128 rows (resident tiles) and of 64 (half blocks)
   const CUtensorMap &tq = m[0], &tk = m[1], &tv = m[2], &tdo = m[3], &q_half = m[4], &k_half = m[5], &v_half = m[6], &do_half = m[7];
-  using L1 = BwdSmem<D, true>;
-  using L2 = BwdSmem<D, false>;
-  static DeviceOnce once1, once2;   // kernel attributes are per device: set on the first launch on each one
-  auto k1 = attn_bwd_dkdv_kernel<D>;
-  auto k2 = attn_bwd_dq_kernel<D>;
-  if (int e = ensure_dyn_smem(once1, k1, L1::TOTAL)) return e;
-  if (int e = ensure_dyn_smem(once2, k2, L2::TOTAL)) return e;
-  const int nqb = (p.S + 127) / 128;
-  tfb::launch_k(k1, nqb * p.Hkv * p.B, L1::THREADS, L1::TOTAL, st, q_half, tk, tv, do_half, p);
-  tfb::launch_k(k2, nqb * p.Hq * p.B, L2::THREADS, L2::TOTAL, st, tq, k_half, v_half, tdo, p);
-  return int(cudaGetLastError());
+  const int nqb = (p.S + 127) / 128, b1 = nqb * p.Hkv * p.B, b2 = nqb * p.Hq * p.B;
+  if (D == 128) {
+    if (int e = launch_dkdv<128, 2>(q_half, tk, tv, do_half, p, b1, st)) return e;
+    return launch_dq<128, 2>(tq, k_half, v_half, tdo, p, b2, st);
+  }
+  // Heads of 64: one warpgroup and two blocks per SM only pay where a second block is there to fill the first one's waits.  us, all gradient kernels,
+  // one warpgroup / two: 36 blocks (1 x 300, 12 heads) 24.6 / 20.2, 64 (1 x 2048, 4) 99.6 / 69.9, 128 (16 x 128, 8) 18.2 / 16.7, 192 (3 x 1024, 8) 58.7 /
+  // 42.4, 256 (4 x 1024, 8) 61.0 / 50.6, but 256 short ones (32 x 128, 8) 23.2 / 28.5, 320 (5 x 1024, 8) 62.9 / 65.5, 512 (8 x 1024, 8) 88.6 / 97.2.
+  const int sms = sm_count(), alone = p.S >= 512 ? 2 * sms : sms;
+  if (int e = b1 <= alone ? launch_dkdv<64, 2>(q_half, tk, tv, do_half, p, b1, st) : launch_dkdv<64, 1>(q_half, tk, tv, do_half, p, b1, st)) return e;
+  return b2 <= alone ? launch_dq<64, 2>(tq, k_half, v_half, tdo, p, b2, st) : launch_dq<64, 1>(tq, k_half, v_half, tdo, p, b2, st);
 }
 
 }  // namespace tfb
@@ -632,5 +653,5 @@ TFB_API int tfb_attn_bwd(const void* q, long long ldq, int q_col0, const void* k
   p.dk = static_cast<__nv_bfloat16*>(dk); p.lddk = lddk; p.dk_col0 = dk_col0;
   p.dv = static_cast<__nv_bfloat16*>(dv); p.lddv = lddv; p.dv_col0 = dv_col0;
   p.status = status;
-  return D == 64 ? launch_bwd<64>(maps, p, st) : launch_bwd<128>(maps, p, st);
+  return launch_bwd(D, maps, p, st);
 }

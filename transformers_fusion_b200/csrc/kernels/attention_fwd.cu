@@ -9,6 +9,8 @@
 // O accumulates in tensor memory relative to a reference maximum that only moves when a row's maximum has grown by more than
 // 2^8 (probabilities are then below 256, which bf16 and the fp32 sums hold as exactly as values below one); a move rescales
 // the accumulator.  The result divides by the sum relative to the same reference.
+// Error of O against float64, of its norm (bf16 rounding of the probabilities and of O): 1.777e-3 at 4 x 1024, heads of 64, 1.793e-3 at 4096, heads of
+// 128; 1.774e-3 and 1.792e-3 with a product per tile, added in registers, and a row's largest probability exactly one.
 //
 // Head size 64: one tile per CTA in 256 columns of tensor memory (scores 0..127, O 128..191, P 192..255), so that two CTAs share an
 // SM and one computes while the other starts or ends; P has columns of its own, so S(j+1) is computed while the

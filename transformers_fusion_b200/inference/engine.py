@@ -50,7 +50,7 @@ class EngineConfig:
     weight_group: int = 32
     cuda_graph: bool = True        # decode steps replay a captured graph per batch-size bucket (CUDA only)
     batch_prefill: bool = True     # prompts admitted in the same step (without a cached prefix) are prefilled together
-    max_prefill_tokens: int = 8192 # padded tokens per prefill batch
+    max_prefill_tokens: int = 8192 # tokens per prefill batch; the scheduler counts each prompt of a batch as long as the longest
     pipeline_decode: object = True # CUDA: a decode step is launched before the previous step's tokens are read on the host
                                    # ("force": the same schedule on any device, for testing the scheduler on CPU)
 
@@ -447,8 +447,9 @@ class InferenceEngine:
         return h[torch.tensor([at + n - 1 for at, n in zip(pack.starts, lens)], dtype=torch.int64, device=dev)]
 
     def _prefill_fresh(self, fresh: List[Request], finished: list):
-        """Groups the newly admitted prompts (sorted by length, so padding stays small) under the padded-token budget and
-        prefills each group in one pass; then samples every sequence's first token."""
+        """Groups the newly admitted prompts, sorted by length, so that the longest one's length times their number stays within the
+        budget (the rows of models that pad; the packed rows of the others are fewer), and prefills each group in one pass; then samples
+        every sequence's first token."""
         fresh = sorted(fresh, key=lambda r: len(r.tokens))
         groups, cur = [], []
         for r in fresh:

@@ -198,8 +198,10 @@ def _rows_pay(M, pw):
     more than the finalize where they are many and their share of K is short (4096 x 4096, 4.6 blocks of 14 k-blocks, fp4 / mxfp8 13.6 / 14.3 and 14.1 /
     14.6; 2048 x 8192, 9 of 14, 13.0 / 15.7; 512 x 1408, 5.5 of 4, 8.4 / 9.2; but 4096 x 14336, 4.6 of 48, 30.1 / 29.1; 6144 x 4096, 3.1 of 21,
     18.1 / 17.3; 1536 x 512, 2 of 4, 8.4 / 7.0).  From 9 rows on, mxfp8 codes that one block per SM walks alone: 2048 x 8192 at 16 rows 12.7 / 14.1
-    (int8 12.9 / 12.7, int4 12.3 / 11.4)."""
+    (int8 12.9 / 12.7, int4 12.3 / 11.4).  Nothing was measured beyond K = 8192, where the one-launch forms stay."""
     sms = _lib.lib().tfb_sm_count()
+    if pw.Kp > SKINNY_K:
+        return True
     if M <= 16:
         return M <= 8 or pw.fmt != FORMATS["mxfp8"] or pw.Np >= 16 * sms or pw.Kp <= 4096
     tiles, kb = pw.Np // 128, pw.Kp // 64
